@@ -665,6 +665,51 @@ __device__ void warp_item(const Scene &S, const ViewConst &V, const HzbDesc *hzb
   warp_flush(ws, wc, V, S.slot_capacity, slot, cut);
 }
 
+// The histogram pass of one warp for the view it works on (HIST): the view's thresholds e_k and band edges high_k,
+// evaluated once instead of in every step of every meshlet's searches, and the triangles entering (0) and leaving (1)
+// the cut per bin, added in shared memory and flushed to the view's histogram when the warp moves to another view.
+// A chunk's meshlets fall into nearly as many bins as there are lanes, so one global atomic per distinct bin and step
+// cost more than the test itself. 8 views of a 4K million-instance world: k_chunks<HIST> 512 -> 233 us (searches
+// started from an estimate of the bin, two probes for most: 222 us, not kept).
+template <bool HIST>
+struct BudgetWork {
+  float e[kBudgetBins], high[kBudgetBins];
+  uint32_t hist[2 * kBudgetBins];
+};
+template <>
+struct BudgetWork<false> {};
+constexpr uint32_t kBudgetFlush = 4096;  // chunks between flushes: 4096 x 1024 meshlets x 128 triangles < 2^32
+
+// first k with pred(k), probed as by budget_bin_high (kBudgetBins when none)
+template <class Pred>
+__device__ __forceinline__ uint32_t first_bin(Pred pred) {
+  uint32_t lo = 0, hi = kBudgetBins;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (pred(mid)) hi = mid;
+    else lo = mid + 1;
+  }
+  return lo;
+}
+
+__device__ __forceinline__ void budget_flush(BudgetWork<true> &w, unsigned long long *hist) {
+  __syncwarp();
+  for (uint32_t i = threadIdx.x & 31; i < 2 * kBudgetBins; i += 32) {
+    const uint32_t v = w.hist[i];
+    if (v) atomicAdd(hist + i, (unsigned long long)v);
+    w.hist[i] = 0;
+  }
+  __syncwarp();
+}
+
+__device__ __forceinline__ void budget_begin(BudgetWork<true> &w, const ViewConst &V, float s) {
+  for (uint32_t k = threadIdx.x & 31; k < kBudgetBins; k += 32) {
+    w.e[k] = budget_e(V, s, k);
+    w.high[k] = budget_high(V, s, k);
+  }
+  __syncwarp();
+}
+
 // Meshlets of one chunk that passed the LOD band (HIST: that enter the cut somewhere in the threshold range),
 // waiting for the rest of their test with all 32 lanes busy: about a third of the tested meshlets pass, and testing
 // them in place would leave most lanes idle.
@@ -697,7 +742,8 @@ __device__ __forceinline__ uint32_t frame_vm(const SpanFrame &F, uint32_t j, flo
 template <bool HIST>
 __device__ __forceinline__ void drain_queue(const Scene &S, const ViewConst &V, const HzbDesc *hzbs, const LodQueue &q,
                                             const SpanFrame &F, uint32_t n, WarpStage &ws, WarpCount &wc, float inv_low,
-                                            float fs, float high0, uint32_t cut, bool occl_on, uint32_t slot) {
+                                            float fs, float high0, uint32_t cut, bool occl_on, uint32_t slot,
+                                            BudgetWork<HIST> &bw) {
   const uint32_t lane = threadIdx.x & 31;
   bool drawn = false;
   uint32_t packed = 0, id = 0, instance = 0, lo = 0, hi = 255;
@@ -730,9 +776,11 @@ __device__ __forceinline__ void drain_queue(const Scene &S, const ViewConst &V, 
     id = __float_as_uint(er.w);
     packed = HIST ? __float_as_uint(er.z) : (__float_as_uint(er.z) | (lo << 8) | (hi << 16));
   }
-  if (HIST) {
-    warp_hist_add(V.hist, drawn, lo, packed);
-    warp_hist_add(V.hist + kBudgetBins, drawn, hi, packed);
+  if constexpr (HIST) {
+    if (drawn) {  // b_own < b_par <= kBudgetBins
+      atomicAdd(&bw.hist[lo], packed);
+      if (hi < kBudgetBins) atomicAdd(&bw.hist[kBudgetBins + hi], packed);
+    }
   } else {
     warp_stage(ws, wc, V, S.slot_capacity, slot, cut, drawn, instance, id, packed);
   }
@@ -1045,7 +1093,7 @@ __global__ void __launch_bounds__(128, 4) k_instances_redo(Scene S0, const Scene
 // meshlets that pass queue up and finish 32 at a time (drain_queue). One draw-list flush per chunk.
 // HIST: the budget histogram of the chunks the budget pass queued.
 template <bool HIST, bool MULTI>
-__global__ void __launch_bounds__(128, MULTI ? 6 : 8) k_chunks(Scene S0, const Scene *__restrict__ scenes,
+__global__ void __launch_bounds__(128, MULTI || HIST ? 6 : 8) k_chunks(Scene S0, const Scene *__restrict__ scenes,
                                                             const ViewConst *__restrict__ views,
                                                             const HzbDesc *__restrict__ hzbs0,
                                                             uint4 *__restrict__ queue, uint32_t *__restrict__ ctl,
@@ -1053,6 +1101,8 @@ __global__ void __launch_bounds__(128, MULTI ? 6 : 8) k_chunks(Scene S0, const S
   __shared__ WarpStage stage[4];
   __shared__ LodQueue queues[4];
   __shared__ SpanFrame frames[4];
+  __shared__ BudgetWork<HIST> budgets[4];
+  BudgetWork<HIST> &bw = budgets[threadIdx.x >> 5];
   WarpStage &ws = stage[threadIdx.x >> 5];
   LodQueue &q = queues[threadIdx.x >> 5];
   SpanFrame &F = frames[threadIdx.x >> 5];
@@ -1060,6 +1110,11 @@ __global__ void __launch_bounds__(128, MULTI ? 6 : 8) k_chunks(Scene S0, const S
   const WorkQueue Q = work_queue(queue, capacity);
   const uint32_t n_chunks = min(uint32_t(*queue_counter(ctl) >> 32), Q.chunk_cap);
   const uint32_t lane = threadIdx.x & 31;
+  uint32_t hist_view = ~0u, hist_chunks = 0;  // HIST: the view the warp's histogram belongs to
+  if constexpr (HIST) {
+    for (uint32_t i = lane; i < 2 * kBudgetBins; i += 32) bw.hist[i] = 0;
+    __syncwarp();
+  }
   WarpFeed<1> feed;
   feed.start(ctl + kCtlNextChunk);
   for (uint32_t c = feed.i; c < n_chunks; c = feed.next()) {
@@ -1075,7 +1130,14 @@ __global__ void __launch_bounds__(128, MULTI ? 6 : 8) k_chunks(Scene S0, const S
     const ViewBands b = bands_of(V);
     const float low = cut ? b.low1 : b.low0, high = cut ? b.high1 : b.high0;
     const float inv_low = 1.0f / low;
-    const float sc = HIST ? get_state(V.state, 0) : 0.0f;
+    if constexpr (HIST) {
+      if (ch.x != hist_view || ++hist_chunks == kBudgetFlush) {
+        if (hist_view != ~0u) budget_flush(bw, views[hist_view].hist);
+        if (ch.x != hist_view) budget_begin(bw, V, get_state(V.state, 0));
+        hist_view = ch.x;
+        hist_chunks = 0;
+      }
+    }
     // spans: one lane each, laid end to end from position 0
     uint4 sp = make_uint4(0u, 0u, 0u, 0u);
     if (lane < ns) sp = Q.spans[ch.w + lane];
@@ -1115,8 +1177,9 @@ __global__ void __launch_bounds__(128, MULTI ? 6 : 8) k_chunks(Scene S0, const S
         const float4 ls = __ldg(S.m_lod + m), ps = __ldg(S.m_parent + m);
         const float2 er = __ldg(reinterpret_cast<const float2 *>(S.m_err + m));
         const ProjErr po = proj_parts(V, VM, VM[12], ls, er.x), pp = proj_parts(V, VM, VM[12], ps, er.y);
-        if (HIST) {
-          const uint32_t bo = budget_bin_high(V, sc, po, er.x), bp = budget_bin(V, sc, pp, er.y);
+        if constexpr (HIST) {
+          const uint32_t bo = first_bin([&](uint32_t k) { return err_le(po, er.x, bw.high[k]); });
+          const uint32_t bp = first_bin([&](uint32_t k) { return err_le(pp, er.y, bw.e[k]); });
           pass = bo < bp;
           own = __uint_as_float(bo);
           parent = __uint_as_float(bp);
@@ -1137,7 +1200,8 @@ __global__ void __launch_bounds__(128, MULTI ? 6 : 8) k_chunks(Scene S0, const S
       qn += __popc(mask);
       __syncwarp();
       if (qn >= 32) {
-        drain_queue<HIST>(S, V, hzbs, q, F, 32, ws, wc, inv_low, b.fade_scale, b.high0, cut, occl_on, cell.slot);
+        drain_queue<HIST>(S, V, hzbs, q, F, 32, ws, wc, inv_low, b.fade_scale, b.high0, cut, occl_on, cell.slot,
+                          bw);
         qn -= 32;
         __syncwarp();
         if (lane < qn) {
@@ -1149,10 +1213,14 @@ __global__ void __launch_bounds__(128, MULTI ? 6 : 8) k_chunks(Scene S0, const S
         __syncwarp();
       }
     }
-    if (qn) drain_queue<HIST>(S, V, hzbs, q, F, qn, ws, wc, inv_low, b.fade_scale, b.high0, cut, occl_on, cell.slot);
+    if (qn)
+      drain_queue<HIST>(S, V, hzbs, q, F, qn, ws, wc, inv_low, b.fade_scale, b.high0, cut, occl_on, cell.slot, bw);
     __syncwarp();
     if (!HIST) warp_flush(ws, wc, V, S.slot_capacity, cell.slot, cut);
     __syncwarp();  // the frame and queue are rewritten by the next chunk
+  }
+  if constexpr (HIST) {
+    if (hist_view != ~0u) budget_flush(bw, views[hist_view].hist);
   }
 }
 
