@@ -184,6 +184,13 @@ int ensure_outputs(vgc_context *ctx, uint32_t slots) {
   if ((rc = dev_alloc(ctx, ctx->d_args, (size_t)n * 2 * ctx->slot_capacity * 2 * 5 * 4))) return rc;
   if ((rc = dev_alloc(ctx, ctx->d_dyn, (size_t)n * 8 * 4))) return rc;
   if ((rc = dev_alloc(ctx, ctx->d_hist, (size_t)n * 2 * kBudgetBins * 8))) return rc;
+  if (n > ctx->out_slots) {
+    uint32_t *fresh = nullptr;
+    CUDA_TRY(cudaMallocHost(&fresh, (size_t)n * kStatWords * 4));
+    if (ctx->h_stats) cudaFreeHost(ctx->h_stats);
+    ctx->h_stats = fresh;
+  }
+  std::memset(ctx->h_stats, 0, (size_t)n * kStatWords * 4);
   CUDA_TRY(cudaMemset(ctx->d_counters.ptr, 0, (size_t)n * ctx->counter_words * 4));
   CUDA_TRY(cudaMemset(ctx->d_args.ptr, 0, (size_t)n * 2 * ctx->slot_capacity * 2 * 5 * 4));
   ctx->out_slots = n;
@@ -532,6 +539,7 @@ int view_constants(vgc_context *ctx, const vgc_view &in, uint32_t out_slot, uint
   k.draw_list = (uint4 *)ctx->d_draw.ptr + (size_t)out_slot * 2 * ctx->opts.max_meshlets;
   k.draw_args = (uint32_t *)ctx->d_args.ptr + (size_t)out_slot * 2 * ctx->slot_capacity * 2 * 5;
   k.dyn = (float *)ctx->d_dyn.ptr + (size_t)out_slot * 8;
+  k.host_stats = ctx->h_stats + (size_t)out_slot * kStatWords;
   k.hist = (unsigned long long *)ctx->d_hist.ptr + (size_t)out_slot * 2 * kBudgetBins;
   return VGC_OK;
 }
@@ -674,12 +682,21 @@ int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st,
   const Scene *scenes = s.multi ? s.d_scenes : nullptr;
   const uint32_t select_grid = s.grid_instances ? s.grid_instances : ctx->select_grid;
   const uint32_t chunk_grid = s.grid_chunks ? s.grid_chunks : ctx->chunk_grid;
-  CUDA_TRY(cudaMemcpyAsync(s.d_views, s.h_views, sizeof(ViewConst) * count, cudaMemcpyHostToDevice, st));
-  if (s.multi) CUDA_TRY(cudaMemcpyAsync(s.d_scenes, s.h_scenes, sizeof(Scene) * s.scene_count, cudaMemcpyHostToDevice, st));
-  if (s.hzb_w && ctx->hzb_grid)
-    CUDA_TRY(cudaMemcpyAsync(s.d_plan, s.h_plan, hzb_plan_bytes(count), cudaMemcpyHostToDevice, st));
+  LaunchInputs in;  // read by the first kernel from pinned memory
+  in.views = s.h_views;
+  if (s.multi) {
+    static_assert(sizeof(Scene) % 4 == 0, "copied as words");
+    in.scenes_src = reinterpret_cast<const uint32_t *>(s.h_scenes);
+    in.scenes_dst = reinterpret_cast<uint32_t *>(s.d_scenes);
+    in.scene_words = (uint32_t)(sizeof(Scene) / 4 * s.scene_count);
+  }
+  if (s.hzb_w && ctx->hzb_grid) {
+    in.plan_src = reinterpret_cast<const uint4 *>(s.h_plan);
+    in.plan_dst = reinterpret_cast<uint4 *>(s.d_plan);
+    in.plan_vecs = (uint32_t)(hzb_plan_bytes(count) / 16);
+  }
   CUDA_TRY(timed(ctx, capture, VGC_KERNEL_RESET, st,
-                 [&] { return launch_reset(s.d_views, count, s.d_unit_count, st); }));
+                 [&] { return launch_reset(in, s.d_views, count, s.d_unit_count, st); }));
   // the HZB build (after the reset, which clears the counter word a failed wait of the build reports in) and the
   // cell pass do not depend on each other: the cell pass runs on a second stream beside the build (a parallel branch
   // of the captured graph), submitted after it so that the build's persistent blocks are resident first, and joins
@@ -694,8 +711,10 @@ int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st,
   }
   const cudaStream_t cells_st = s.hzb_w ? s.side : st;
   CUDA_TRY(timed(ctx, capture, VGC_KERNEL_CELLS, cells_st, [&] {
-    return launch_cells(S, scenes, s.d_views, count, s.units_total, s.d_units, s.d_unit_count, cells_st);
+    return launch_cells(S, scenes, s.d_views, count, s.units_total, s.d_units, s.d_unit_count, cells_st,
+                        s.hzb_w != 0 || s.shared);
   }));
+  bool plain = s.hzb_w != 0 || s.shared;  // the next launch follows the join
   if (s.hzb_w) {
     CUDA_TRY(cudaEventRecord(s.join, s.side));
     CUDA_TRY(cudaStreamWaitEvent(st, s.join, 0));
@@ -704,13 +723,15 @@ int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st,
   if (s.any_budget) {  // the triangleBudget search: histogram pass, then the threshold of each budget view
     CUDA_TRY(timed(ctx, capture, VGC_KERNEL_BUDGET, st, [&] {
       cudaError_t e = launch_instances(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, -1,
-                                       select_grid, s.d_overflow, st, s.chunk_shift);
+                                       select_grid, s.d_overflow, st, s.chunk_shift, plain);
+      plain = s.shared;
       if (e == cudaSuccess)
-        e = launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, -1, chunk_grid, st);
+        e = launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, -1, chunk_grid, st,
+                          s.shared);
       if (e == cudaSuccess)
         e = launch_instances_redo(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, -1,
-                                  s.d_overflow, redo_grid, st, s.chunk_shift);
-      if (e == cudaSuccess) e = launch_budget(s.d_views, count, s.d_unit_count, st);
+                                  s.d_overflow, redo_grid, st, s.chunk_shift, s.shared);
+      if (e == cudaSuccess) e = launch_budget(s.d_views, count, s.d_unit_count, st, s.shared);
       return e;
     }));
   }
@@ -718,22 +739,21 @@ int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st,
     const uint32_t shift = round > 0 && kChunkShiftRetry ? kChunkShiftRetry : s.chunk_shift;
     CUDA_TRY(timed(ctx, capture, round == 0 ? VGC_KERNEL_SELECT0 : VGC_KERNEL_SELECT_RETRY, st, [&] {
       return launch_instances(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, round,
-                              select_grid, s.d_overflow, st, shift);
+                              select_grid, s.d_overflow, st, shift, round == 0 ? plain : s.shared);
     }));
     CUDA_TRY(timed(ctx, capture, round == 0 ? VGC_KERNEL_CHUNKS0 : VGC_KERNEL_SELECT_RETRY, st, [&] {
-      return launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, round, chunk_grid, st);
+      return launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, round, chunk_grid, st,
+                           s.shared);
     }));
     // units whose items did not fit the queue (returns at once when there are none)
     CUDA_TRY(timed(ctx, capture, VGC_KERNEL_SELECT_RETRY, st, [&] {
       return launch_instances_redo(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity,
-                                   round, s.d_overflow, redo_grid, st, shift);
+                                   round, s.d_overflow, redo_grid, st, shift, s.shared);
     }));
     CUDA_TRY(timed(ctx, capture, VGC_KERNEL_FINISH, st, [&] {
-      return launch_finish(s.d_views, count, s.d_unit_count, round, st);
+      return launch_finish(s.d_views, count, s.d_unit_count, round, round == 2 ? s.h_ctl : nullptr, st, s.shared);
     }));
   }
-  // control words (peak queue demand) for the next prepare
-  CUDA_TRY(cudaMemcpyAsync(s.h_ctl, s.d_unit_count, 64, cudaMemcpyDeviceToHost, st));
   return VGC_OK;
 }
 
@@ -917,6 +937,7 @@ int vgc_context_destroy(vgc_context *ctx) {
                     &ctx->d_draw, &ctx->d_args, &ctx->d_dyn, &ctx->d_hist, &ctx->d_state, &ctx->d_hzb_desc})
     dev_free(ctx, *b);
   for (auto &h : ctx->hzb) dev_free(ctx, h.data);
+  if (ctx->h_stats) cudaFreeHost(ctx->h_stats);
   for (auto &p : ctx->prof_pending) {
     cudaEventDestroy(p.second.first);
     cudaEventDestroy(p.second.second);
@@ -1406,11 +1427,10 @@ int vgc_read_stats(vgc_context *ctx, uint32_t slot, vgc_stats *s, vgc_stream str
   if (slot >= ctx->out_slots) return fail(VGC_NOT_FOUND, "output slot not allocated");
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   CUDA_TRY(cudaStreamSynchronize(st));
-  CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  uint32_t c[VGC_COUNTER_HEADER];
-  CUDA_TRY(cudaMemcpy(c, (const uint32_t *)ctx->d_counters.ptr + (size_t)slot * ctx->counter_words, sizeof c, cudaMemcpyDeviceToHost));
-  float dyn = 0;
-  CUDA_TRY(cudaMemcpy(&dyn, (const float *)ctx->d_dyn.ptr + (size_t)slot * 8, 4, cudaMemcpyDeviceToHost));
+  if (st != ctx->stream) CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  const uint32_t *c = ctx->h_stats + (size_t)slot * kStatWords;  // mirrored by the cut's last kernel
+  float dyn;
+  std::memcpy(&dyn, c + VGC_COUNTER_HEADER, 4);
   decode_stats(ctx, c, dyn, s);
   return VGC_OK;
 }
@@ -1421,8 +1441,7 @@ int vgc_read_draw_list(vgc_context *ctx, uint32_t slot, uint32_t cut, uint32_t *
   if (slot >= ctx->out_slots) return fail(VGC_NOT_FOUND, "output slot not allocated");
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   CUDA_TRY(cudaStreamSynchronize(st));
-  uint32_t sel = 0;
-  CUDA_TRY(cudaMemcpy(&sel, (const uint32_t *)ctx->d_counters.ptr + (size_t)slot * ctx->counter_words + VGC_COUNTER_CUT0 + cut * 5 + VGC_CUT_SELECTED, 4, cudaMemcpyDeviceToHost));
+  const uint32_t sel = ctx->h_stats[(size_t)slot * kStatWords + VGC_COUNTER_CUT0 + cut * 5 + VGC_CUT_SELECTED];
   const uint32_t n = std::min(sel, ctx->opts.max_meshlets);
   *count = n;
   const uint32_t copy = std::min(n, capacity);
@@ -1452,19 +1471,11 @@ int vgc_expand(vgc_context *ctx, uint32_t slot, uint32_t cut, uint32_t *index_bu
     if (ctx->mesh_host[m].used && ctx->mesh_host[m].triangle_count == 0)
       return fail(VGC_INVALID_ARG, "vgc_expand needs meshlet_triangles for every mesh (slot " + std::to_string(m) + ")");
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-  // the view constants of this slot, rebuilt from the output pointers (only the pointers and sizes are read)
-  ViewConst k{};
+  ExpandView k;  // by value: no scratch is written, so nothing waits for the cut before
   k.max_drawn = ctx->opts.max_meshlets;
-  k.counters = (uint32_t *)ctx->d_counters.ptr + (size_t)slot * ctx->counter_words;
-  k.draw_list = (uint4 *)ctx->d_draw.ptr + (size_t)slot * 2 * ctx->opts.max_meshlets;
-  int rc = ensure_scratch(ctx, ctx->scratch, 1, 32);
-  if (rc) return rc;
-  if (ctx->scratch.pending) CUDA_TRY(cudaEventSynchronize(ctx->scratch.done));
-  ctx->scratch.h_views[0] = k;
-  CUDA_TRY(cudaMemcpyAsync(ctx->scratch.d_views, ctx->scratch.h_views, sizeof(ViewConst), cudaMemcpyHostToDevice, st));
-  CUDA_TRY(launch_expand(scene_of(ctx), ctx->scratch.d_views, cut, index_buffer, capacity, ctx->sm_count * 8, st));
-  CUDA_TRY(cudaEventRecord(ctx->scratch.done, st));
-  ctx->scratch.pending = true;
+  k.counters = (const uint32_t *)ctx->d_counters.ptr + (size_t)slot * ctx->counter_words;
+  k.draw_list = (const uint4 *)ctx->d_draw.ptr + (size_t)slot * 2 * ctx->opts.max_meshlets;
+  CUDA_TRY(launch_expand(scene_of(ctx), k, cut, index_buffer, capacity, ctx->sm_count * 8, st));
   return VGC_OK;
 }
 
@@ -1660,7 +1671,7 @@ extern "C" int vgc_cut_noalloc(vgc_context *ctx, const vgc_view *view, uint32_t 
     const HzbDesc &d = ctx->hzb[view->hzb].desc;
     CUDA_TRY(launch_hzb_views(d_view, 1, d.w[0], d.h[0], d.levels > 7, st));
   }
-  CUDA_TRY(launch_reset(d_view, 1, ctl, st));
+  CUDA_TRY(launch_reset(LaunchInputs(), d_view, 1, ctl, st));
   CUDA_TRY(launch_cells(S, nullptr, d_view, 1, cells, units, ctl, st));
   if (view->triangle_budget > 0) {
     CUDA_TRY(launch_instances(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, -1, ctx->select_grid, overflow,
@@ -1676,7 +1687,7 @@ extern "C" int vgc_cut_noalloc(vgc_context *ctx, const vgc_view *view, uint32_t 
     CUDA_TRY(launch_chunks(S, nullptr, d_view, chunks, ctl, kNoAllocMaxChunks, round, ctx->chunk_grid, st));
     CUDA_TRY(launch_instances_redo(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, round, overflow,
                                    redo_grid, st));
-    CUDA_TRY(launch_finish(d_view, 1, ctl, round, st));
+    CUDA_TRY(launch_finish(d_view, 1, ctl, round, nullptr, st));
   }
   return VGC_OK;
 }

@@ -66,13 +66,14 @@ struct LaunchScratch {
   uint4 *d_chunks = nullptr;      // meshlet work queue (spans and chunks)
   uint32_t chunk_capacity = 0;    // its entries
   uint32_t queue_want = 0;        // entries the last launch sequence asked for (grown to before the next one)
-  uint32_t *h_ctl = nullptr;      // pinned copy of the control words at the end of the last launch sequence
+  uint32_t *h_ctl = nullptr;      // pinned: control words 6 and 7 at the end of the last launch sequence
   uint32_t grid_instances = 0;    // persistent grids of k_instances / k_chunks (0: the context's occupancy defaults)
   uint32_t grid_chunks = 0;
   uint32_t chunk_shift = kChunkShiftDefault;  // 2^chunk_shift meshlets per k_chunks work unit
   uint32_t view_capacity = 0;
   size_t unit_capacity = 0;
   size_t units_total = 0;         // (view, cell) units of the prepared launch (each view: its scene's cells, padded)
+  bool shared = false;            // other launch sequences run beside this one (a server's lanes): plain launches
   bool multi = false;             // the prepared views belong to several contexts (a multi-scene launch)
   Scene *h_scenes = nullptr;      // pinned: the multi-scene launch's scene table (ViewConst::scene indexes it)
   Scene *d_scenes = nullptr;
@@ -127,6 +128,7 @@ struct vgc_context {
   uint32_t out_slot_capacity = 0;  // slot_capacity the output buffers were sized for
   uint32_t counter_words = 0;
   DevBuf d_counters, d_draw, d_args, d_dyn, d_hist;
+  uint32_t *h_stats = nullptr;  // pinned: kStatWords per output slot, written by the slot's last k_finish
   // controller state slots
   DevBuf d_state;
   uint32_t state_slots = 0;

@@ -33,6 +33,7 @@ constexpr uint32_t kFullFadeBits = 255u << 16;
 constexpr uint32_t kLocalVertexBits = 7;   // ceil(log2(MAX_MESHLET_VERTICES = 128))
 constexpr uint32_t kMaxHzbLevels = 16;
 constexpr uint32_t kStateWords = 8;        // S_SCALE 0..1, S_FILL 2..3, S_RETRY 4..5
+constexpr uint32_t kStatWords = 32;        // an output slot's mirror in pinned memory
 constexpr uint32_t kBudgetBins = 256;
 constexpr uint32_t kChunkShiftMin = 8, kChunkShiftDefault = 9, kChunkShiftMax = 10;  // meshlets per chunk: 256..1024
 #ifndef VGC_RETRY_CHUNK_SHIFT
@@ -139,6 +140,7 @@ struct ViewConst {
   const float *hzb_mip0;  // VGC_VIEW_DEPTH_AS_MIP0: the HZB's mip 0 is `depth` (not copied into the slot); else null
   uint32_t *counters;   // VGC_COUNTER_* header, then per (cut, slot, part): count, start
   uint32_t *state;      // kStateWords, carried between frames
+  uint32_t *host_stats; // pinned: the counter header and dyn[0] (kStatWords), written by the last k_finish
   uint4 *draw_list;     // 2 * max_drawn
   uint32_t *draw_args;  // 2 cuts * slot_capacity * 2 parts * 5
   float *dyn;           // [0] error threshold of this frame (errorThreshold or the budget search result),

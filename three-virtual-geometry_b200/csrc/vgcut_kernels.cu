@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <utility>
 
 #include "vgcut_internal.h"
 #include "vgcut_kernels.h"
@@ -26,6 +27,15 @@
 namespace vgc {
 
 #define C_CUT(cut) (VGC_COUNTER_CUT0 + (cut) * 5)
+
+// The launch sequence's kernels are launched with programmatic serialization: the next kernel's blocks may become
+// resident while this one's last blocks still run. Every kernel of the sequence starts with this wait for the whole
+// kernel before it (and, since that one waited too, for all before), so nothing is read early; what is saved is the
+// launch latency between the sequence's dozen short kernels. A plain launch returns at once.
+__device__ __forceinline__ void wait_previous_kernel() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 __device__ __forceinline__ float fmn(float a, float b) { return a < b ? a : b; }
 __device__ __forceinline__ float fmx(float a, float b) { return a > b ? a : b; }
@@ -231,6 +241,7 @@ __global__ void __launch_bounds__(256) k_cells(Scene S0, const Scene *__restrict
                                                const ViewConst *__restrict__ views, uint32_t nviews,
                                                uint32_t total_units, uint2 *__restrict__ units,
                                                uint32_t *__restrict__ unit_count) {
+  wait_previous_kernel();
   const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
   if ((u & ~31u) >= total_units) return;  // whole warp out of range
@@ -1045,6 +1056,7 @@ __global__ void __launch_bounds__(128, MULTI ? 6 : 8) k_instances(Scene S0, cons
                                                    uint32_t capacity, int round, uint32_t chunk_shift,
                                                    uint32_t *__restrict__ overflow) {
   __shared__ Survivor lists[4][kHalfUnit];
+  wait_previous_kernel();
   if (round > 0 && ctl[round] == 0) return;  // no view redoes a cut in this round
   const uint32_t work = ctl[0] * 2;
   WarpFeed<1> feed;
@@ -1068,6 +1080,7 @@ __global__ void __launch_bounds__(128, 4) k_instances_redo(Scene S0, const Scene
                                                             uint32_t chunk_shift, uint32_t *__restrict__ overflow) {
   __shared__ WarpStage stage[4];
   __shared__ Survivor lists[4][kHalfUnit];
+  wait_previous_kernel();
   if (round > 0 && ctl[round] == 0) return;
   if (ctl[kCtlOverflowed] == 0) return;
   const uint32_t words = (ctl[0] * 4 + 31) / 32;
@@ -1106,6 +1119,7 @@ __global__ void __launch_bounds__(128, MULTI || HIST ? 6 : 8) k_chunks(Scene S0,
   WarpStage &ws = stage[threadIdx.x >> 5];
   LodQueue &q = queues[threadIdx.x >> 5];
   SpanFrame &F = frames[threadIdx.x >> 5];
+  wait_previous_kernel();
   if (round > 0 && ctl[round] == 0) return;  // no view redoes a cut in this round
   const WorkQueue Q = work_queue(queue, capacity);
   const uint32_t n_chunks = min(uint32_t(*queue_counter(ctl) >> 32), Q.chunk_cap);
@@ -1230,6 +1244,7 @@ __global__ void __launch_bounds__(128, MULTI || HIST ? 6 : 8) k_chunks(Scene S0,
 // frame's first selection round.
 __global__ void __launch_bounds__(128) k_budget(const ViewConst *__restrict__ views, uint32_t nviews,
                                                 uint32_t *__restrict__ ctl) {
+  wait_previous_kernel();
   if (blockIdx.x == 0 && threadIdx.x == 0) retire_queue(ctl);
   const uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
@@ -1276,10 +1291,18 @@ __device__ __forceinline__ float fill_of(const ViewConst &V, uint32_t cut) {
 }
 
 __global__ void __launch_bounds__(128) k_finish(const ViewConst *__restrict__ views, uint32_t nviews,
-                                                uint32_t *__restrict__ ctl, int round) {
+                                                uint32_t *__restrict__ ctl, int round,
+                                                uint32_t *__restrict__ host_ctl) {
+  wait_previous_kernel();
   const uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
-  if (blockIdx.x == 0 && threadIdx.x == 0) retire_queue(ctl);  // the next round's work queue starts empty
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    retire_queue(ctl);  // the next round's work queue starts empty
+    if (host_ctl) {     // the peak queue demand, for the host's next launch (pinned memory)
+      host_ctl[6] = ctl[6];
+      host_ctl[7] = ctl[7];
+    }
+  }
   if (v >= nviews) return;
   const ViewConst &V = views[v];
   const uint32_t slot_capacity = V.slot_capacity, slots_used = V.slots_used;
@@ -1372,12 +1395,18 @@ __global__ void __launch_bounds__(128) k_finish(const ViewConst *__restrict__ vi
     }
     ctr[VGC_COUNTER_ROUNDS] += 1;
   }
+  if (round == 2 && V.host_stats) {  // the counters and the threshold, mirrored in pinned memory for vgc_read_stats
+    __syncwarp();
+    uint32_t w = 0;
+    if (lane < VGC_COUNTER_HEADER) w = ctr[lane];
+    else if (lane == VGC_COUNTER_HEADER) w = __float_as_uint(V.dyn[0]);
+    V.host_stats[lane] = w;
+  }
 }
 
 // ------------------------------------------------------------------------------------------------ k_expand
-__global__ void __launch_bounds__(256) k_expand(Scene S, const ViewConst *__restrict__ view, uint32_t cut,
-                                                uint32_t *__restrict__ out, uint64_t capacity) {
-  const ViewConst &V = *view;
+__global__ void __launch_bounds__(256) k_expand(Scene S, const ExpandView V, uint32_t cut, uint32_t *__restrict__ out,
+                                                uint64_t capacity) {
   const uint32_t n = min(V.counters[C_CUT(cut) + VGC_CUT_SELECTED], V.max_drawn);
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -1385,7 +1414,8 @@ __global__ void __launch_bounds__(256) k_expand(Scene S, const ViewConst *__rest
     const uint32_t draw_slot = e + cut * V.max_drawn;
     const uint4 d = V.draw_list[draw_slot];
     const uint32_t slot = S.inst_slot[d.x];
-    const uint32_t region = mesh_count(V, S.slot_capacity, cut, slot, part_of(d.w))[1];
+    const uint32_t region =
+        V.counters[VGC_COUNTER_HEADER + (((cut * S.slot_capacity + slot) * 2 + part_of(d.w)) * 2) + 1];
     const uint32_t first_tri = S.m_info[d.y].y / 3;
     const uint32_t base = draw_slot << kLocalVertexBits;
     const uint32_t tris = d.w & 255u;
@@ -1537,6 +1567,7 @@ __global__ void __launch_bounds__(256) k_hzb_tiles_views(const ViewConst *__rest
 
 // Levels `first` and up of each building view's HZB, one block per view (the tile kernels wrote the levels below).
 __global__ void __launch_bounds__(1024) k_hzb_tail_views(const ViewConst *__restrict__ views, uint32_t first) {
+  wait_previous_kernel();
   const ViewConst &V = views[blockIdx.x];
   if (!V.build_hzb) return;
   const HzbDesc &H = *V.hzb_desc;
@@ -1703,6 +1734,7 @@ __global__ void __launch_bounds__(kHzbStreamThreads, VGC_HZB_BLOCKS_PER_SM) k_hz
   __shared__ __align__(8) uint64_t full[kHzbStages], empty[kHzbStages];
   __shared__ uint4 meta[kHzbStages];  // job, ox, oy, tma of the strip in each stage
   __shared__ uint32_t abort;
+  wait_previous_kernel();
   const HzbPlanHead &P = *reinterpret_cast<const HzbPlanHead *>(plan);
   const HzbJob *jobs = reinterpret_cast<const HzbJob *>(plan + sizeof(HzbPlanHead));
   const uint32_t njobs = P.jobs;
@@ -1906,36 +1938,43 @@ __global__ void __launch_bounds__(256) k_select_cut(Scene S, uint32_t slot, uint
 
 // ------------------------------------------------------------------------------------------------ k_reset
 // Zeroes each view's counter block (reset pass, GeometryPool.ts:714-725) and the batch's unit count; reads the
-// output pointers from the view constants, so a captured graph serves any output slots.
-__global__ void __launch_bounds__(256) k_reset(const ViewConst *__restrict__ views, uint32_t nviews,
+// output pointers from the view constants, so a captured graph serves any output slots. The launch's inputs (view
+// constants, HZB plan, scene table) come from pinned host memory by this kernel's own reads: as copies before it they
+// cost 6 us more in a stream and 20 us in a graph (the gap between a copy node and the first kernel).
+__global__ void __launch_bounds__(256) k_reset(const LaunchInputs in, ViewConst *__restrict__ views, uint32_t nviews,
                                                uint32_t *__restrict__ ctl) {
+  __shared__ __align__(16) uint32_t staged[sizeof(ViewConst) / 4];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (blockIdx.x == 0 && threadIdx.x < 16) ctl[threadIdx.x] = 0;
+  const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (uint32_t i = first; i < in.plan_vecs; i += stride) in.plan_dst[i] = in.plan_src[i];
+  for (uint32_t i = first; i < in.scene_words; i += stride) in.scenes_dst[i] = in.scenes_src[i];
+  if (in.plan_vecs) asm volatile("fence.proxy.tensormap::generic.release.gpu;" ::: "memory");
   for (uint32_t v = blockIdx.x; v < nviews; v += gridDim.x) {
-    uint32_t *c = views[v].counters;
-    const uint32_t words = views[v].counter_words;
+    const uint32_t *src = reinterpret_cast<const uint32_t *>((in.views ? in.views : views) + v);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(views + v);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < sizeof(ViewConst) / 4; i += blockDim.x) {
+      const uint32_t w = src[i];
+      staged[i] = w;
+      if (in.views) dst[i] = w;
+    }
+    __syncthreads();
+    const ViewConst &V = *reinterpret_cast<const ViewConst *>(staged);
+    uint32_t *c = V.counters;
+    const uint32_t words = V.counter_words;
     for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) c[i] = 0;
     if (threadIdx.x == 0) {
-      if (views[v].fresh_state) {  // initial controller state: scales 1.0 (fixed point x10000), no fill, no retry
-        uint32_t *st = views[v].state;
+      if (V.fresh_state) {  // initial controller state: scales 1.0 (fixed point x10000), no fill, no retry
+        uint32_t *st = V.state;
         for (uint32_t i = 0; i < kStateWords; i++) st[i] = i < 2 ? 10000u : 0u;
       }
       // budget views: the search's pass uses the band at the top of the threshold range
-      store_bands(views[v], views[v].budget > 0.0f ? views[v].budget_hi : views[v].error_threshold);
+      store_bands(V, V.budget > 0.0f ? V.budget_hi : V.error_threshold);
     }
-    if (views[v].budget > 0.0f)
-      for (uint32_t i = threadIdx.x; i < 2 * kBudgetBins; i += blockDim.x) views[v].hist[i] = 0;
+    if (V.budget > 0.0f)
+      for (uint32_t i = threadIdx.x; i < 2 * kBudgetBins; i += blockDim.x) V.hist[i] = 0;
   }
-}
-
-// Each view's counter header and the threshold its cut used, 32 words per view, for one device-to-host copy.
-__global__ void __launch_bounds__(32) k_gather_stats(const ViewConst *__restrict__ views, uint32_t nviews,
-                                                     uint32_t *__restrict__ out) {
-  const uint32_t v = blockIdx.x, t = threadIdx.x;
-  if (v >= nviews) return;
-  uint32_t w = 0;
-  if (t < VGC_COUNTER_HEADER) w = views[v].counters[t];
-  else if (t == VGC_COUNTER_HEADER) w = __float_as_uint(views[v].dyn[0]);
-  out[v * 32 + t] = w;
 }
 
 // ------------------------------------------------------------------------------------------------ cell update
@@ -2010,26 +2049,37 @@ cudaError_t launch_cells_update(const float4 *inst, const double sphere[4], uint
   return cudaGetLastError();
 }
 
-cudaError_t launch_gather_stats(const ViewConst *views, uint32_t nviews, uint32_t *out, cudaStream_t st) {
-  k_gather_stats<<<nviews, 32, 0, st>>>(views, nviews, out);
-  return cudaGetLastError();
+// A kernel of the launch sequence behind another kernel on the stream (wait_previous_kernel). plain: launched
+// without, because it follows an event of another stream, or because other streams' batches share the device (blocks
+// that wait would keep their places from them).
+template <class... P, class... A>
+static cudaError_t launch_after(bool plain, void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem,
+                                cudaStream_t st, A &&...args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = plain ? 0 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
-cudaError_t launch_reset(const ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st) {
+cudaError_t launch_reset(const LaunchInputs &in, ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st) {
   const uint32_t blocks = nviews < 1024 ? (nviews ? nviews : 1) : 1024;
-  k_reset<<<blocks, 256, 0, st>>>(views, nviews, ctl);
+  k_reset<<<blocks, 256, 0, st>>>(in, views, nviews, ctl);
   return cudaGetLastError();
 }
 
 cudaError_t launch_cells(const Scene &S, const Scene *scenes, const ViewConst *views, uint32_t nviews,
-                         uint32_t total_units, uint2 *units, uint32_t *unit_count, cudaStream_t st) {
+                         uint32_t total_units, uint2 *units, uint32_t *unit_count, cudaStream_t st, bool plain) {
   if (total_units == 0) return cudaSuccess;
   const uint32_t blocks = (total_units + 255) / 256;
-  if (scenes)
-    k_cells<true><<<blocks, 256, 0, st>>>(S, scenes, views, nviews, total_units, units, unit_count);
-  else
-    k_cells<false><<<blocks, 256, 0, st>>>(S, nullptr, views, nviews, total_units, units, unit_count);
-  return cudaGetLastError();
+  if (scenes) return launch_after(plain, k_cells<true>, blocks, 256, 0, st, S, scenes, views, nviews, total_units, units, unit_count);
+  return launch_after(plain, k_cells<false>, blocks, 256, 0, st, S, scenes, views, nviews, total_units, units, unit_count);
 }
 
 cudaError_t configure_select(bool multi, int *instances_per_sm, int *chunks_per_sm) {
@@ -2041,84 +2091,76 @@ cudaError_t configure_select(bool multi, int *instances_per_sm, int *chunks_per_
 }
 
 template <bool MULTI>
-static void instances_kernel(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
+static cudaError_t instances_kernel(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
                              uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t grid,
-                             uint32_t chunk_shift, uint32_t *overflow, cudaStream_t st) {
+                             uint32_t chunk_shift, uint32_t *overflow, cudaStream_t st, bool plain) {
   if (round < 0)  // the budget search's pass
-    k_instances<true, MULTI><<<grid, 128, 0, st>>>(S, scenes, views, S.hzbs, units, ctl, queue, capacity, 0,
-                                                   chunk_shift, overflow);
-  else
-    k_instances<false, MULTI><<<grid, 128, 0, st>>>(S, scenes, views, S.hzbs, units, ctl, queue, capacity, round,
-                                                    chunk_shift, overflow);
+    return launch_after(plain, k_instances<true, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, units, ctl, queue,
+                        capacity, 0, chunk_shift, overflow);
+  return launch_after(plain, k_instances<false, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, units, ctl, queue,
+                      capacity, round, chunk_shift, overflow);
 }
 
 cudaError_t launch_instances(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
                              uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t grid,
-                             uint32_t *overflow, cudaStream_t st, uint32_t chunk_shift) {
+                             uint32_t *overflow, cudaStream_t st, uint32_t chunk_shift, bool plain) {
   if (chunk_shift < kChunkShiftFloor || chunk_shift > kChunkShiftMax || !overflow) return cudaErrorInvalidValue;
   if (scenes)
-    instances_kernel<true>(S, scenes, views, units, ctl, queue, capacity, round, grid, chunk_shift, overflow, st);
-  else
-    instances_kernel<false>(S, nullptr, views, units, ctl, queue, capacity, round, grid, chunk_shift, overflow, st);
-  return cudaGetLastError();
+    return instances_kernel<true>(S, scenes, views, units, ctl, queue, capacity, round, grid, chunk_shift, overflow, st,
+                                  plain);
+  return instances_kernel<false>(S, nullptr, views, units, ctl, queue, capacity, round, grid, chunk_shift, overflow, st,
+                                 plain);
 }
 
 template <bool MULTI>
-static void instances_redo_kernel(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
+static cudaError_t instances_redo_kernel(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
                                   uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t chunk_shift,
-                                  uint32_t *overflow, uint32_t grid, cudaStream_t st) {
+                                  uint32_t *overflow, uint32_t grid, cudaStream_t st, bool plain) {
   if (round < 0)
-    k_instances_redo<true, MULTI><<<grid, 128, 0, st>>>(S, scenes, views, S.hzbs, units, ctl, queue, capacity, 0,
-                                                        chunk_shift, overflow);
-  else
-    k_instances_redo<false, MULTI><<<grid, 128, 0, st>>>(S, scenes, views, S.hzbs, units, ctl, queue, capacity,
-                                                         round, chunk_shift, overflow);
+    return launch_after(plain, k_instances_redo<true, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, units, ctl, queue,
+                        capacity, 0, chunk_shift, overflow);
+  return launch_after(plain, k_instances_redo<false, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, units, ctl, queue,
+                      capacity, round, chunk_shift, overflow);
 }
 
 cudaError_t launch_instances_redo(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
                                   uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t *overflow,
-                                  uint32_t grid, cudaStream_t st, uint32_t chunk_shift) {
+                                  uint32_t grid, cudaStream_t st, uint32_t chunk_shift, bool plain) {
   if (chunk_shift < kChunkShiftFloor || chunk_shift > kChunkShiftMax || !overflow || grid == 0)
     return cudaErrorInvalidValue;
   if (scenes)
-    instances_redo_kernel<true>(S, scenes, views, units, ctl, queue, capacity, round, chunk_shift, overflow, grid, st);
-  else
-    instances_redo_kernel<false>(S, nullptr, views, units, ctl, queue, capacity, round, chunk_shift, overflow, grid,
-                                 st);
-  return cudaGetLastError();
+    return instances_redo_kernel<true>(S, scenes, views, units, ctl, queue, capacity, round, chunk_shift, overflow,
+                                       grid, st, plain);
+  return instances_redo_kernel<false>(S, nullptr, views, units, ctl, queue, capacity, round, chunk_shift, overflow,
+                                      grid, st, plain);
 }
 
 template <bool MULTI>
-static void chunks_kernel(const Scene &S, const Scene *scenes, const ViewConst *views, uint4 *queue, uint32_t *ctl,
-                          uint32_t capacity, int round, uint32_t grid, cudaStream_t st) {
+static cudaError_t chunks_kernel(const Scene &S, const Scene *scenes, const ViewConst *views, uint4 *queue, uint32_t *ctl,
+                          uint32_t capacity, int round, uint32_t grid, cudaStream_t st, bool plain) {
   if (round < 0)
-    k_chunks<true, MULTI><<<grid, 128, 0, st>>>(S, scenes, views, S.hzbs, queue, ctl, capacity, 0);
-  else
-    k_chunks<false, MULTI><<<grid, 128, 0, st>>>(S, scenes, views, S.hzbs, queue, ctl, capacity, round);
+    return launch_after(plain, k_chunks<true, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, queue, ctl, capacity, 0);
+  return launch_after(plain, k_chunks<false, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, queue, ctl, capacity, round);
 }
 
 cudaError_t launch_chunks(const Scene &S, const Scene *scenes, const ViewConst *views, uint4 *queue, uint32_t *ctl,
-                          uint32_t capacity, int round, uint32_t grid, cudaStream_t st) {
-  if (scenes)
-    chunks_kernel<true>(S, scenes, views, queue, ctl, capacity, round, grid, st);
-  else
-    chunks_kernel<false>(S, nullptr, views, queue, ctl, capacity, round, grid, st);
-  return cudaGetLastError();
+                          uint32_t capacity, int round, uint32_t grid, cudaStream_t st, bool plain) {
+  if (scenes) return chunks_kernel<true>(S, scenes, views, queue, ctl, capacity, round, grid, st, plain);
+  return chunks_kernel<false>(S, nullptr, views, queue, ctl, capacity, round, grid, st, plain);
 }
 
-cudaError_t launch_budget(const ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st) {
+cudaError_t launch_budget(const ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st, bool plain) {
   const uint32_t blocks = (nviews * 32 + 127) / 128;
-  k_budget<<<blocks, 128, 0, st>>>(views, nviews, ctl);
-  return cudaGetLastError();
+  return launch_after(plain, k_budget, blocks, 128, 0, st, views, nviews, ctl);
 }
 
-cudaError_t launch_finish(const ViewConst *views, uint32_t nviews, uint32_t *ctl, int round, cudaStream_t st) {
+cudaError_t launch_finish(const ViewConst *views, uint32_t nviews, uint32_t *ctl, int round, uint32_t *host_ctl,
+                          cudaStream_t st, bool plain) {
   const uint32_t blocks = (nviews * 32 + 127) / 128;
-  k_finish<<<blocks, 128, 0, st>>>(views, nviews, ctl, round);
-  return cudaGetLastError();
+  return launch_after(plain, k_finish, blocks, 128, 0, st, views, nviews, ctl, round, host_ctl);
 }
 
-cudaError_t launch_expand(const Scene &S, const ViewConst *view, uint32_t cut, uint32_t *out, uint64_t capacity,
+cudaError_t launch_expand(const Scene &S, const ExpandView &view, uint32_t cut, uint32_t *out, uint64_t capacity,
                           uint32_t grid, cudaStream_t st) {
   k_expand<<<grid, 256, 0, st>>>(S, view, cut, out, capacity);
   return cudaGetLastError();
@@ -2161,11 +2203,9 @@ uint32_t hzb_stream_blocks_per_sm() {
 
 cudaError_t launch_hzb_stream(const unsigned char *plan, uint32_t grid, const ViewConst *views, uint32_t nviews,
                               bool tail, cudaStream_t st) {
-  k_hzb_stream<<<grid, kHzbStreamThreads, kHzbStreamSmem, st>>>(plan);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_after(false, k_hzb_stream, grid, kHzbStreamThreads, kHzbStreamSmem, st, plan);
   if (e != cudaSuccess || !tail) return e;
-  k_hzb_tail_views<<<nviews, 1024, 0, st>>>(views, kHzbStripLevels);
-  return cudaGetLastError();
+  return launch_after(false, k_hzb_tail_views, nviews, 1024, 0, st, views, kHzbStripLevels);
 }
 
 cudaError_t launch_select_cut(const Scene &S, uint32_t slot, uint32_t mcount, uint32_t count, const float *vm16,

@@ -10,36 +10,56 @@ namespace vgc {
 // Resident 128-thread blocks per SM of the instance / chunk kernels (their persistent grid size); multi: the
 // variants of a multi-scene launch.
 cudaError_t configure_select(bool multi, int *instances_per_sm, int *chunks_per_sm);
+// What the first kernel of a launch sequence reads from pinned host memory: the view constants (null: `views` on the
+// device already holds them), the HZB plan (16-byte vectors) and a multi-scene launch's scene table (words).
+struct LaunchInputs {
+  const ViewConst *views = nullptr;
+  const uint4 *plan_src = nullptr;
+  uint4 *plan_dst = nullptr;
+  uint32_t plan_vecs = 0, scene_words = 0;
+  const uint32_t *scenes_src = nullptr;
+  uint32_t *scenes_dst = nullptr;
+};
 // ctl: per-batch control words: [0] visible units, [1..2] a view redoes a cut in round 1..2, [3] chunks queued
-cudaError_t launch_reset(const ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st);
+cudaError_t launch_reset(const LaunchInputs &in, ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st);
+// plain: launched without programmatic serialization (launch_after).
 // Scene arguments: a launch over one context passes its Scene and scenes = nullptr; a multi-scene launch passes
 // a device table of Scene records that each view's `scene` indexes (S is then unused).
 cudaError_t launch_cells(const Scene &S, const Scene *scenes, const ViewConst *views, uint32_t nviews,
-                         uint32_t total_units, uint2 *units, uint32_t *unit_count, cudaStream_t st);
+                         uint32_t total_units, uint2 *units, uint32_t *unit_count, cudaStream_t st,
+                         bool plain = false);
 // round < 0: the triangleBudget search's histogram pass (k_instances / k_chunks), then launch_budget picks the
 // threshold of each budget view.
-cudaError_t launch_budget(const ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st);
+cudaError_t launch_budget(const ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st, bool plain = false);
 // chunk_shift: windows of 2^chunk_shift meshlets per chunk (kChunkShiftMin..Max; the default 9 = 512 meshlets).
 // overflow: a bit per warp-unit (4 per unit of `units`), zero between passes: k_instances marks the units whose
 // items did not fit the queue, and launch_instances_redo (after launch_chunks of the same pass) tests their items
 // in place and clears the bits.
 cudaError_t launch_instances(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
                              uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t grid,
-                             uint32_t *overflow, cudaStream_t st, uint32_t chunk_shift = kChunkShiftDefault);
+                             uint32_t *overflow, cudaStream_t st, uint32_t chunk_shift = kChunkShiftDefault,
+                             bool plain = false);
 cudaError_t launch_instances_redo(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
                                   uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t *overflow,
-                                  uint32_t grid, cudaStream_t st, uint32_t chunk_shift = kChunkShiftDefault);
+                                  uint32_t grid, cudaStream_t st, uint32_t chunk_shift = kChunkShiftDefault,
+                                  bool plain = false);
 // The meshlet work queue (spans and chunks) lives in `queue`, `capacity` uint4 entries; ctl[4..5] counts it.
 cudaError_t launch_chunks(const Scene &S, const Scene *scenes, const ViewConst *views, uint4 *queue,
-                          uint32_t *ctl, uint32_t capacity, int round, uint32_t grid, cudaStream_t st);
-// 32 words per view: the VGC_COUNTER_HEADER counter words, then the threshold the cut used (float bits).
-cudaError_t launch_gather_stats(const ViewConst *views, uint32_t nviews, uint32_t *out, cudaStream_t st);
+                          uint32_t *ctl, uint32_t capacity, int round, uint32_t grid, cudaStream_t st,
+                          bool plain = false);
 // computeCell on the device for n cells from c0 of one mesh (bit-identical to the host's computation).
 cudaError_t launch_cells_update(const float4 *inst, const double sphere[4], uint32_t instance_base,
                                 uint32_t instance_count, uint32_t cell_base, uint32_t slot, uint32_t c0, uint32_t n,
                                 CellRec *cells, cudaStream_t st);
-cudaError_t launch_finish(const ViewConst *views, uint32_t nviews, uint32_t *ctl, int round, cudaStream_t st);
-cudaError_t launch_expand(const Scene &S, const ViewConst *view, uint32_t cut, uint32_t *out, uint64_t capacity,
+// host_ctl (round 2, optional, pinned): receives control words 6 and 7, the peak queue demand of the sequence.
+cudaError_t launch_finish(const ViewConst *views, uint32_t nviews, uint32_t *ctl, int round, uint32_t *host_ctl,
+                          cudaStream_t st, bool plain = false);
+struct ExpandView {  // what index expansion reads of an output slot
+  const uint32_t *counters;
+  const uint4 *draw_list;
+  uint32_t max_drawn;
+};
+cudaError_t launch_expand(const Scene &S, const ExpandView &view, uint32_t cut, uint32_t *out, uint64_t capacity,
                           uint32_t grid, cudaStream_t st);
 cudaError_t launch_hzb(const float *depth, const HzbDesc &H, float *out, int copy_mip0, cudaStream_t st);
 // HZB builds of the views whose constants carry build_hzb (grid covers the largest depth image).

@@ -10,7 +10,7 @@
 //    batch takes the requests of the oldest admissible request's scene;
 //  * continuous batching: each of `streams` lanes owns a CUDA stream and launch scratch; a lane that finishes is
 //    refilled from whatever is pending, while the other lanes' batches keep running;
-//  * completion: the lane's stream gathers every view's counters into pinned memory and then runs a host callback,
+//  * completion: each view's last kernel mirrors its counters in pinned memory; the lane's stream then runs a host callback,
 //    which stamps the completion time and wakes the worker; no CUDA call that can wait on a stream is made under
 //    the server lock (the callbacks take it).
 #include <algorithm>
@@ -47,8 +47,6 @@ struct Lane {
   cudaStream_t stream = nullptr;
   LaunchScratch scratch;
   cudaEvent_t start = nullptr, end = nullptr;
-  uint32_t *d_words = nullptr;  // 32 words per view (launch_gather_stats)
-  uint32_t *h_words = nullptr;  // pinned copy
   bool busy = false;
   bool complete = false;  // set by the stream callback
   double done_us = 0;
@@ -180,8 +178,6 @@ int launch_batch(vgc_server *s, Lane &lane, const std::vector<uint32_t> &slots, 
   if (rc) return rc;
   CUDA_TRY(cudaEventRecord(lane.start, lane.stream));
   if ((rc = enqueue(ctx, lane.scratch, n, lane.stream, false))) return rc;
-  CUDA_TRY(launch_gather_stats(lane.scratch.d_views, n, lane.d_words, lane.stream));
-  CUDA_TRY(cudaMemcpyAsync(lane.h_words, lane.d_words, (size_t)n * 32 * 4, cudaMemcpyDeviceToHost, lane.stream));
   CUDA_TRY(cudaEventRecord(lane.end, lane.stream));
   CUDA_TRY(cudaLaunchHostFunc(lane.stream, lane_done, cb));
   return VGC_OK;
@@ -201,7 +197,7 @@ void finish_lane(vgc_server *s, Lane &lane) {
     r.result.done_us = lane.status == VGC_OK ? lane.done_us : now_us();
     r.result.batch_gpu_ms = gpu_ms;
     if (lane.status == VGC_OK) {
-      const uint32_t *w = lane.h_words + i * 32;
+      const uint32_t *w = ctx->h_stats + (size_t)r.result.slot * kStatWords;  // the slot is this request's until released
       float threshold;
       std::memcpy(&threshold, &w[VGC_COUNTER_HEADER], 4);
       decode_stats(ctx, w, threshold, &r.result.stats);
@@ -323,12 +319,11 @@ int vgc_server_create(vgc_context *const *scenes, uint32_t scene_count, const vg
   s->multi_grid[1] = (uint32_t)std::max(1, mc) * largest->sm_count;
   const size_t units = (size_t)o.max_batch * pad32((uint32_t)largest->cells.size());
   for (Lane &lane : s->lanes) {
+    lane.scratch.shared = true;
     int rc = ensure_scratch(largest, lane.scratch, o.max_batch, units);
     if (rc) return cleanup(rc);
     if (cudaStreamCreateWithFlags(&lane.stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreate(&lane.start) != cudaSuccess || cudaEventCreate(&lane.end) != cudaSuccess ||
-        cudaMalloc(&lane.d_words, (size_t)o.max_batch * 32 * 4) != cudaSuccess ||
-        cudaMallocHost(&lane.h_words, (size_t)o.max_batch * 32 * 4) != cudaSuccess)
+        cudaEventCreate(&lane.start) != cudaSuccess || cudaEventCreate(&lane.end) != cudaSuccess)
       return cleanup(fail(VGC_DEVICE_ERROR, "server lane setup failed"));
   }
   s->worker = std::thread(worker_main, s);
@@ -422,8 +417,6 @@ int vgc_server_destroy(vgc_server *s) {
     free_scratch(lane.scratch);
     if (lane.start) cudaEventDestroy(lane.start);
     if (lane.end) cudaEventDestroy(lane.end);
-    if (lane.d_words) cudaFree(lane.d_words);
-    if (lane.h_words) cudaFreeHost(lane.h_words);
     if (lane.stream) cudaStreamDestroy(lane.stream);
   }
   delete s;
