@@ -271,9 +271,9 @@ int ensure_scratch(vgc_context *ctx, LaunchScratch &s, uint32_t views, size_t un
   }
   if (!s.d_unit_count) CUDA_TRY(cudaMalloc(&s.d_unit_count, 64));
   // meshlet work queue: about one span per instance with a level range and cut, one chunk per 512 meshlets of a
-  // warp's items. Sized for 64k entries per view; a warp that cannot reserve tests its items itself, so a full
+  // warp's items (fewer in a launch of few views: pass_shape). Sized for 64k entries per view, 256k at least; a warp that cannot reserve tests its items itself, so a full
   // queue costs time, not correctness.
-  const uint32_t want_chunks = std::max<uint32_t>(std::max<uint32_t>(65536, views * 65536u), s.queue_want);
+  const uint32_t want_chunks = std::max<uint32_t>(std::max<uint32_t>(kQueueMin, views * 65536u), s.queue_want);
   if (want_chunks > s.chunk_capacity) {
     if (s.d_chunks) {
       cudaFree(s.d_chunks);
@@ -720,26 +720,31 @@ int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st,
     CUDA_TRY(cudaStreamWaitEvent(st, s.join, 0));
   }
   const uint32_t redo_grid = (uint32_t)ctx->sm_count * 2;
+  // a batch whose chunk size was picked by the autotuner (or its caller) keeps to it
+  PassLimits lim;
+  lim.chunk_min = s.chunk_tuned ? s.chunk_shift : kChunkShiftFloor;
+  lim.chunk_max = s.chunk_shift;
+  lim.fine_units = select_grid * 4 / 2;  // fewer half-units than warps
   if (s.any_budget) {  // the triangleBudget search: histogram pass, then the threshold of each budget view
     CUDA_TRY(timed(ctx, capture, VGC_KERNEL_BUDGET, st, [&] {
       cudaError_t e = launch_instances(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, -1,
-                                       select_grid, s.d_overflow, st, s.chunk_shift, plain);
+                                       select_grid, s.d_overflow, st, lim, plain);
       plain = s.shared;
       if (e == cudaSuccess)
         e = launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, -1, chunk_grid, st,
                           s.shared);
       if (e == cudaSuccess)
         e = launch_instances_redo(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, -1,
-                                  s.d_overflow, redo_grid, st, s.chunk_shift, s.shared);
+                                  s.d_overflow, redo_grid, st, lim, s.shared);
       if (e == cudaSuccess) e = launch_budget(s.d_views, count, s.d_unit_count, st, s.shared);
       return e;
     }));
   }
   for (int round = 0; round < 3; round++) {
-    const uint32_t shift = round > 0 && kChunkShiftRetry ? kChunkShiftRetry : s.chunk_shift;
+    if (round > 0 && kChunkShiftRetry) lim.chunk_max = kChunkShiftRetry, lim.chunk_min = std::min(lim.chunk_min, kChunkShiftRetry);
     CUDA_TRY(timed(ctx, capture, round == 0 ? VGC_KERNEL_SELECT0 : VGC_KERNEL_SELECT_RETRY, st, [&] {
       return launch_instances(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, round,
-                              select_grid, s.d_overflow, st, shift, round == 0 ? plain : s.shared);
+                              select_grid, s.d_overflow, st, lim, round == 0 ? plain : s.shared);
     }));
     CUDA_TRY(timed(ctx, capture, round == 0 ? VGC_KERNEL_CHUNKS0 : VGC_KERNEL_SELECT_RETRY, st, [&] {
       return launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, round, chunk_grid, st,
@@ -748,7 +753,7 @@ int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st,
     // units whose items did not fit the queue (returns at once when there are none)
     CUDA_TRY(timed(ctx, capture, VGC_KERNEL_SELECT_RETRY, st, [&] {
       return launch_instances_redo(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity,
-                                   round, s.d_overflow, redo_grid, st, shift, s.shared);
+                                   round, s.d_overflow, redo_grid, st, lim, s.shared);
     }));
     CUDA_TRY(timed(ctx, capture, VGC_KERNEL_FINISH, st, [&] {
       return launch_finish(s.d_views, count, s.d_unit_count, round, round == 2 ? s.h_ctl : nullptr, st, s.shared);
@@ -1285,7 +1290,7 @@ int vgc_batch_run(vgc_batch *b, const vgc_view *views, uint32_t count, uint32_t 
       b->graph_hzb_w != b->scratch.hzb_w || b->graph_hzb_h != b->scratch.hzb_h || b->graph_hzb_tail != b->scratch.hzb_tail ||
       b->graph_budget != b->scratch.any_budget || b->graph_queue != b->scratch.d_chunks ||
       b->graph_grids[0] != b->scratch.grid_instances || b->graph_grids[1] != b->scratch.grid_chunks ||
-      b->graph_chunk_shift != b->scratch.chunk_shift) {
+      b->graph_chunk_shift != b->scratch.chunk_shift || b->graph_chunk_tuned != b->scratch.chunk_tuned) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     b->exec = nullptr;
@@ -1312,6 +1317,7 @@ int vgc_batch_run(vgc_batch *b, const vgc_view *views, uint32_t count, uint32_t 
     b->graph_grids[0] = b->scratch.grid_instances;
     b->graph_grids[1] = b->scratch.grid_chunks;
     b->graph_chunk_shift = b->scratch.chunk_shift;
+    b->graph_chunk_tuned = b->scratch.chunk_tuned;
   }
   CUDA_TRY(cudaGraphLaunch(b->exec, st));
   CUDA_TRY(cudaEventRecord(b->scratch.done, st));
@@ -1348,6 +1354,7 @@ int vgc_batch_autotune(vgc_batch *b, const vgc_view *views, uint32_t count, uint
       b->scratch.grid_instances = bi * sms;
       b->scratch.grid_chunks = bc * sms;
       b->scratch.chunk_shift = shift;
+      b->scratch.chunk_tuned = true;
       if ((rc = vgc_batch_run(b, views, count, first_slot, stream))) break;  // capture + warm-up
       std::vector<float> ms;
       for (uint32_t r = 0; r < reps; r++) {  // replays of the captured graph: device time only
@@ -1390,6 +1397,7 @@ int vgc_batch_set_tuning(vgc_batch *b, const vgc_tune_result *t) {
   b->scratch.grid_instances = t->instances_blocks_per_sm * sms;
   b->scratch.grid_chunks = t->chunks_blocks_per_sm * sms;
   b->scratch.chunk_shift = (uint32_t)__builtin_ctz(c);
+  b->scratch.chunk_tuned = true;
   return VGC_OK;
 }
 

@@ -46,6 +46,8 @@ struct HzbSlot {
   bool valid = false;
 };
 
+constexpr uint32_t kQueueMin = 262144;  // entries of the smallest meshlet work queue
+
 inline uint32_t pad32(uint32_t x) { return (x + 31u) & ~31u; }
 
 }  // namespace vgch
@@ -69,7 +71,8 @@ struct LaunchScratch {
   uint32_t *h_ctl = nullptr;      // pinned: control words 6 and 7 at the end of the last launch sequence
   uint32_t grid_instances = 0;    // persistent grids of k_instances / k_chunks (0: the context's occupancy defaults)
   uint32_t grid_chunks = 0;
-  uint32_t chunk_shift = kChunkShiftDefault;  // 2^chunk_shift meshlets per k_chunks work unit
+  uint32_t chunk_shift = kChunkShiftDefault;  // 2^chunk_shift meshlets per k_chunks work unit at most,
+  bool chunk_tuned = false;                   //   or exactly (autotuned or set by the caller)
   uint32_t view_capacity = 0;
   size_t unit_capacity = 0;
   size_t units_total = 0;         // (view, cell) units of the prepared launch (each view: its scene's cells, padded)
@@ -161,6 +164,7 @@ struct vgc_batch {
   const uint4 *graph_queue = nullptr;  // work queue the graph was captured with
   uint32_t graph_grids[2] = {0, 0};    // persistent grids the graph was captured with
   uint32_t graph_chunk_shift = 0;      // chunk size it was captured with
+  bool graph_chunk_tuned = false;
 };
 
 namespace vgch {

@@ -42,8 +42,15 @@ constexpr uint32_t kChunkShiftMin = 8, kChunkShiftDefault = 9, kChunkShiftMax = 
 // 0.48 ms, but 7% slower when most views redo)
 #define VGC_RETRY_CHUNK_SHIFT 8
 #endif
-constexpr uint32_t kChunkShiftRetry = VGC_RETRY_CHUNK_SHIFT, kChunkShiftFloor = 6;
+constexpr uint32_t kChunkShiftRetry = VGC_RETRY_CHUNK_SHIFT, kChunkShiftFloor = 5;
 constexpr uint32_t kLevelSamples = 64;     // per level: samples of the meshlets in test order (item trimming)
+
+// Bounds of how a pass may be cut up (pass_shape): chunks of 2^chunk_min .. 2^chunk_max meshlets, 32 instances per warp
+// below `fine_units` visible units.
+struct PassLimits {
+  uint32_t chunk_min = kChunkShiftDefault, chunk_max = kChunkShiftDefault, fine_units = 0;
+  bool valid() const { return chunk_min >= kChunkShiftFloor && chunk_min <= chunk_max && chunk_max <= kChunkShiftMax; }
+};
 
 struct MeshRec {  // 96 bytes
   float4 sphere;
