@@ -696,7 +696,7 @@ int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st,
     in.plan_vecs = (uint32_t)(hzb_plan_bytes(count) / 16);
   }
   CUDA_TRY(timed(ctx, capture, VGC_KERNEL_RESET, st,
-                 [&] { return launch_reset(in, s.d_views, count, s.d_unit_count, st); }));
+                 [&] { return launch_reset(in, s.d_views, count, s.d_unit_count, st, s.shared); }));
   // the HZB build (after the reset, which clears the counter word a failed wait of the build reports in) and the
   // cell pass do not depend on each other: the cell pass runs on a second stream beside the build (a parallel branch
   // of the captured graph), submitted after it so that the build's persistent blocks are resident first, and joins
@@ -756,7 +756,7 @@ int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st,
                                    round, s.d_overflow, redo_grid, st, lim, s.shared);
     }));
     CUDA_TRY(timed(ctx, capture, VGC_KERNEL_FINISH, st, [&] {
-      return launch_finish(s.d_views, count, s.d_unit_count, round, round == 2 ? s.h_ctl : nullptr, st, s.shared);
+      return launch_finish(s.d_views, count, s.d_unit_count, round, s.h_ctl, st, s.shared);
     }));
   }
   return VGC_OK;

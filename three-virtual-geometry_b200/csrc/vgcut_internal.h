@@ -151,7 +151,7 @@ struct ViewConst {
   uint4 *draw_list;     // 2 * max_drawn
   uint32_t *draw_args;  // 2 cuts * slot_capacity * 2 parts * 5
   float *dyn;           // [0] error threshold of this frame (errorThreshold or the budget search result),
-                        // [1..5] its bands: low (cut 0, 1), high (cut 0, 1), fade scale
+                        // [1..5] its bands: low (cut 0, 1), high (cut 0, 1), fade scale; [6] 1: no further round
   unsigned long long *hist;  // 2 * kBudgetBins: triangles entering / leaving the cut per threshold bin
   unsigned long long budget_tris;  // triangleBudget as an integer (the search compares T(t) <= budget_tris)
   const HzbDesc *hzb_desc;  // the HZB slot's descriptor in the view's context (null without an HZB; HZB builds)

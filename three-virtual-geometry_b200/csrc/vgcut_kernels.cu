@@ -1307,18 +1307,17 @@ __global__ void __launch_bounds__(128) k_budget(const ViewConst *__restrict__ vi
 }
 
 // ------------------------------------------------------------------------------------------------ k_finish
-__device__ __forceinline__ float fill_of(const ViewConst &V, uint32_t cut) {
-  const float requested = float(V.counters[C_CUT(cut) + VGC_CUT_REQUESTED]);
-  const float selected = float(V.counters[C_CUT(cut) + VGC_CUT_SELECTED]);
-  return fmx(requested / float(V.index_capacity[cut]), selected / float(V.max_drawn));
-}
-
+// One warp per view and round: prefix, capacity check, and for a view that needs no further round the steer and its
+// counters' mirror (dyn[6] then marks it settled, and the later rounds' k_finish leave it alone). Bound by the latency
+// of its loads, so both cuts' are issued together, and of the mirror's writes to the host (about 3 us of the 5 that round
+// 0 takes for one view); the later rounds of a launch without retries 3.3 -> 1.3 us each.
 __global__ void __launch_bounds__(128) k_finish(const ViewConst *__restrict__ views, uint32_t nviews,
                                                 uint32_t *__restrict__ ctl, int round,
                                                 uint32_t *__restrict__ host_ctl) {
   wait_previous_kernel();
   const uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
+  if (round > 0 && ctl[round] == 0) return;  // every view has settled, and this round's passes did nothing
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     retire_queue(ctl);  // the next round's work queue starts empty
     if (host_ctl) {     // the peak queue demand, for the host's next launch (pinned memory)
@@ -1330,95 +1329,106 @@ __global__ void __launch_bounds__(128) k_finish(const ViewConst *__restrict__ vi
   const ViewConst &V = views[v];
   const uint32_t slot_capacity = V.slot_capacity, slots_used = V.slots_used;
   uint32_t *ctr = V.counters;
+  if (round > 0 && V.dyn[6] != 0.0f) return;
   const bool redo[2] = {round == 0 || ctr[VGC_COUNTER_REDO0] != 0, round == 0 || ctr[VGC_COUNTER_REDO1] != 0};
-  // prefix (GeometryPool.ts:973-995)
-  for (uint32_t cut = 0; cut < 2; cut++) {
-    if (!redo[cut]) continue;
-    const uint32_t capacity = V.index_capacity[cut];
-    uint32_t carry = 0;
-    for (uint32_t b = 0; b < slots_used; b += 32) {
-      const uint32_t slot = b + lane;
-      uint32_t r0 = 0, r1 = 0;
-      if (slot < slots_used) {
-        r0 = mesh_count(V, slot_capacity, cut, slot, 0)[0];
-        r1 = mesh_count(V, slot_capacity, cut, slot, 1)[0];
-      }
-      const uint32_t sum = r0 + r1;
-      uint32_t incl = sum;
+  const uint32_t selected[2] = {ctr[C_CUT(0) + VGC_CUT_SELECTED], ctr[C_CUT(1) + VGC_CUT_SELECTED]};
+  uint32_t requested[2] = {ctr[C_CUT(0) + VGC_CUT_REQUESTED], ctr[C_CUT(1) + VGC_CUT_REQUESTED]};
+  float scale[2] = {get_state(V.state, 0), get_state(V.state, 1)};
+  // prefix (GeometryPool.ts:973-995): a slot's record is (count, start) of part 0, then of part 1
+  uint32_t carry[2] = {0, 0};
+  for (uint32_t b = 0; b < slots_used; b += 32) {
+    const uint32_t slot = b + lane;
+    uint4 rec[2];
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (uint32_t)o) incl += t;
-      }
+    for (uint32_t cut = 0; cut < 2; cut++)
+      rec[cut] = slot < slots_used && redo[cut] ? *reinterpret_cast<const uint4 *>(mesh_count(V, slot_capacity, cut, slot, 0))
+                                                : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (uint32_t cut = 0; cut < 2; cut++) {
+      if (!redo[cut]) continue;
+      const uint32_t capacity = V.index_capacity[cut], sum = rec[cut].x + rec[cut].z;
+      const uint32_t incl = warp_scan_incl(sum);
       if (slot < slots_used) {
-        const uint32_t starts[2] = {carry + (incl - sum), carry + (incl - sum) + r0};
-        const uint32_t req[2] = {r0, r1};
-        for (uint32_t p = 0; p < 2; p++) {
-          mesh_count(V, slot_capacity, cut, slot, p)[1] = starts[p];
-          const uint32_t room = starts[p] < capacity ? capacity - starts[p] : 0u;
-          uint32_t *a = V.draw_args + ((cut * slot_capacity + slot) * 2 + p) * 5;
-          a[0] = min(req[p], room);
-          a[1] = 1;
-          a[2] = starts[p];
-          a[3] = 0;
-          a[4] = 0;
-        }
+        const uint32_t s0 = carry[cut] + (incl - sum), s1 = s0 + rec[cut].x;
+        *reinterpret_cast<uint4 *>(mesh_count(V, slot_capacity, cut, slot, 0)) = make_uint4(rec[cut].x, s0, rec[cut].z, s1);
+        const uint32_t room0 = s0 < capacity ? capacity - s0 : 0u, room1 = s1 < capacity ? capacity - s1 : 0u;
+        uint2 *a = reinterpret_cast<uint2 *>(V.draw_args + (cut * slot_capacity + slot) * 10);
+        a[0] = make_uint2(min(rec[cut].x, room0), 1u);
+        a[1] = make_uint2(s0, 0u);
+        a[2] = make_uint2(0u, min(rec[cut].z, room1));
+        a[3] = make_uint2(1u, s1);
+        a[4] = make_uint2(0u, 0u);
       }
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) {
-      ctr[C_CUT(cut) + VGC_CUT_REQUESTED] = carry;
-      ctr[C_CUT(cut) + VGC_CUT_DRAWN] = min(ctr[C_CUT(cut) + VGC_CUT_SELECTED], V.max_drawn);
+      carry[cut] += __shfl_sync(0xffffffffu, incl, 31);
     }
   }
-  __syncwarp();
+#pragma unroll
+  for (uint32_t cut = 0; cut < 2; cut++) {
+    if (!redo[cut]) continue;
+    requested[cut] = carry[cut];
+    if (lane == 0) {
+      ctr[C_CUT(cut) + VGC_CUT_REQUESTED] = carry[cut];
+      ctr[C_CUT(cut) + VGC_CUT_DRAWN] = min(selected[cut], V.max_drawn);
+    }
+  }
+  float fill[2];
+#pragma unroll
+  for (uint32_t cut = 0; cut < 2; cut++)
+    fill[cut] = fmx(float(requested[cut]) / float(V.index_capacity[cut]), float(selected[cut]) / float(V.max_drawn));
+  uint32_t again = 0;
   if (round < 2) {
     // capacity check: an overflowing cut is redone at a coarser threshold (GeometryPool.ts:1032-1054)
-    uint32_t again = 0;
-    if (lane == 0) {
-      for (uint32_t cut = 0; cut < 2; cut++) {
-        const float fill = fill_of(V, cut);
-        const float scale = get_state(V.state, cut);
-        V.state[4 + cut] = 0;
-        if (fill > 1.0f && scale < V.lod_scale_limit) {
-          const float q = fmn(fmx(sqrtf(fill / float(0.82)), float(1.1)), 4.0f);
-          V.state[cut] = to_state(fmn(scale * q, V.lod_scale_limit));
-          V.state[4 + cut] = 10000u;
-          again |= 1u << cut;
+#pragma unroll
+    for (uint32_t cut = 0; cut < 2; cut++) {
+      const bool over = fill[cut] > 1.0f && scale[cut] < V.lod_scale_limit;
+      if (over) {
+        const float q = fmn(fmx(sqrtf(fill[cut] / float(0.82)), float(1.1)), 4.0f);
+        scale[cut] = fmn(scale[cut] * q, V.lod_scale_limit);
+        again |= 1u << cut;
+      }
+      if (lane == 0) {
+        V.state[4 + cut] = over ? 10000u : 0u;
+        if (over) {
+          V.state[cut] = to_state(scale[cut]);
           for (int c = 0; c < 5; c++) ctr[C_CUT(cut) + c] = 0;
           if (cut == 0) ctr[VGC_COUNTER_OCCLUDED] = 0;
         }
-        ctr[VGC_COUNTER_REDO0 + cut] = (again >> cut) & 1u;
-      }
-      if (again) store_bands(V, V.dyn[0]);  // the redone round selects with the new scale
-      if (again) {
-        ctr[VGC_COUNTER_ROUNDS] += 1;
-        atomicOr(&ctl[1 + round], 1u);
+        ctr[VGC_COUNTER_REDO0 + cut] = over ? 1u : 0u;
       }
     }
-    again = __shfl_sync(0xffffffffu, again, 0);
+  }
+  if (again) {
+    if (lane == 0) {
+      store_bands(V, V.dyn[0]);  // the redone round selects with the new scale
+      V.dyn[6] = 0.0f;
+      ctr[VGC_COUNTER_ROUNDS] += 1;
+      atomicOr(&ctl[1 + round], 1u);
+    }
     for (uint32_t cut = 0; cut < 2; cut++)
       if ((again >> cut) & 1u)
         for (uint32_t slot = lane; slot < slots_used; slot += 32) {
           mesh_count(V, slot_capacity, cut, slot, 0)[0] = 0;
           mesh_count(V, slot_capacity, cut, slot, 1)[0] = 0;
         }
-  } else if (lane == 0) {
+    return;
+  }
+  if (lane == 0) {
     // steer between frames (GeometryPool.ts:1056-1069)
+#pragma unroll
     for (uint32_t cut = 0; cut < 2; cut++) {
-      const float fill = fill_of(V, cut);
-      float scale = get_state(V.state, cut);
-      if (fill > float(0.9)) {
-        scale = scale * fmn(sqrtf(fill / float(0.82)), float(1.03));
-      } else if (fill < float(0.75)) {
-        scale = scale / float(1.01);
+      float next = scale[cut];
+      if (fill[cut] > float(0.9)) {
+        next = next * fmn(sqrtf(fill[cut] / float(0.82)), float(1.03));
+      } else if (fill[cut] < float(0.75)) {
+        next = next / float(1.01);
       }
-      V.state[cut] = to_state(fmx(fmn(scale, V.lod_scale_limit), 1.0f));
-      V.state[2 + cut] = to_state(fill);
+      V.state[cut] = to_state(fmx(fmn(next, V.lod_scale_limit), 1.0f));
+      V.state[2 + cut] = to_state(fill[cut]);
     }
+    V.dyn[6] = 1.0f;
     ctr[VGC_COUNTER_ROUNDS] += 1;
   }
-  if (round == 2 && V.host_stats) {  // the counters and the threshold, mirrored in pinned memory for vgc_read_stats
+  if (V.host_stats) {  // the counters and the threshold, mirrored in pinned memory for vgc_read_stats
     __syncwarp();
     uint32_t w = 0;
     if (lane < VGC_COUNTER_HEADER) w = ctr[lane];
@@ -1963,24 +1973,32 @@ __global__ void __launch_bounds__(256) k_select_cut(Scene S, uint32_t slot, uint
 // Zeroes each view's counter block (reset pass, GeometryPool.ts:714-725) and the batch's unit count; reads the
 // output pointers from the view constants, so a captured graph serves any output slots. The launch's inputs (view
 // constants, HZB plan, scene table) come from pinned host memory by this kernel's own reads: as copies before it they
-// cost 6 us more in a stream and 20 us in a graph (the gap between a copy node and the first kernel).
+// cost 6 us more in a stream and 20 us in a graph (the gap between a copy node and the first kernel). blocks <= views.
 __global__ void __launch_bounds__(256) k_reset(const LaunchInputs in, ViewConst *__restrict__ views, uint32_t nviews,
                                                uint32_t *__restrict__ ctl) {
   __shared__ __align__(16) uint32_t staged[sizeof(ViewConst) / 4];
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (blockIdx.x == 0 && threadIdx.x < 16) ctl[threadIdx.x] = 0;
+  static_assert(sizeof(ViewConst) / 4 <= 256, "a block stages a view's constants with one word per thread");
   const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  for (uint32_t i = first; i < in.plan_vecs; i += stride) in.plan_dst[i] = in.plan_src[i];
+  // the reads over PCIe of this thread's first pieces overlap the end of the kernel before (they are the host's alone)
+  const bool host_view = in.views && threadIdx.x < sizeof(ViewConst) / 4;
+  uint32_t view_word = 0;
+  if (host_view) view_word = reinterpret_cast<const uint32_t *>(in.views + blockIdx.x)[threadIdx.x];
+  uint4 plan_vec = make_uint4(0u, 0u, 0u, 0u);
+  if (first < in.plan_vecs) plan_vec = in.plan_src[first];
+  wait_previous_kernel();
+  if (blockIdx.x == 0 && threadIdx.x < 16) ctl[threadIdx.x] = 0;
+  if (first < in.plan_vecs) in.plan_dst[first] = plan_vec;
+  for (uint32_t i = first + stride; i < in.plan_vecs; i += stride) in.plan_dst[i] = in.plan_src[i];
   for (uint32_t i = first; i < in.scene_words; i += stride) in.scenes_dst[i] = in.scenes_src[i];
   if (in.plan_vecs) asm volatile("fence.proxy.tensormap::generic.release.gpu;" ::: "memory");
   for (uint32_t v = blockIdx.x; v < nviews; v += gridDim.x) {
-    const uint32_t *src = reinterpret_cast<const uint32_t *>((in.views ? in.views : views) + v);
-    uint32_t *dst = reinterpret_cast<uint32_t *>(views + v);
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < sizeof(ViewConst) / 4; i += blockDim.x) {
-      const uint32_t w = src[i];
-      staged[i] = w;
-      if (in.views) dst[i] = w;
+    if (threadIdx.x < sizeof(ViewConst) / 4) {
+      uint32_t w = view_word;
+      if (!in.views) w = reinterpret_cast<const uint32_t *>(views + v)[threadIdx.x];
+      else if (v != blockIdx.x) w = reinterpret_cast<const uint32_t *>(in.views + v)[threadIdx.x];
+      staged[threadIdx.x] = w;
+      if (in.views) reinterpret_cast<uint32_t *>(views + v)[threadIdx.x] = w;
     }
     __syncthreads();
     const ViewConst &V = *reinterpret_cast<const ViewConst *>(staged);
@@ -2091,10 +2109,10 @@ static cudaError_t launch_after(bool plain, void (*kernel)(P...), uint32_t grid,
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
-cudaError_t launch_reset(const LaunchInputs &in, ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st) {
-  const uint32_t blocks = nviews < 1024 ? (nviews ? nviews : 1) : 1024;
-  k_reset<<<blocks, 256, 0, st>>>(in, views, nviews, ctl);
-  return cudaGetLastError();
+cudaError_t launch_reset(const LaunchInputs &in, ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st,
+                         bool plain) {
+  if (nviews == 0) return cudaErrorInvalidValue;
+  return launch_after(plain, k_reset, nviews < 1024 ? nviews : 1024, 256, 0, st, in, views, nviews, ctl);
 }
 
 cudaError_t launch_cells(const Scene &S, const Scene *scenes, const ViewConst *views, uint32_t nviews,

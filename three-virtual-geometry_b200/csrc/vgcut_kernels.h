@@ -21,7 +21,8 @@ struct LaunchInputs {
   uint32_t *scenes_dst = nullptr;
 };
 // ctl: per-batch control words: [0] visible units, [1..2] a view redoes a cut in round 1..2, [3] chunks queued
-cudaError_t launch_reset(const LaunchInputs &in, ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st);
+cudaError_t launch_reset(const LaunchInputs &in, ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st,
+                         bool plain = false);
 // plain: launched without programmatic serialization (launch_after).
 // Scene arguments: a launch over one context passes its Scene and scenes = nullptr; a multi-scene launch passes
 // a device table of Scene records that each view's `scene` indexes (S is then unused).
@@ -51,7 +52,7 @@ cudaError_t launch_chunks(const Scene &S, const Scene *scenes, const ViewConst *
 cudaError_t launch_cells_update(const float4 *inst, const double sphere[4], uint32_t instance_base,
                                 uint32_t instance_count, uint32_t cell_base, uint32_t slot, uint32_t c0, uint32_t n,
                                 CellRec *cells, cudaStream_t st);
-// host_ctl (round 2, optional, pinned): receives control words 6 and 7, the peak queue demand of the sequence.
+// host_ctl (optional, pinned): receives control words 6 and 7, the peak queue demand of the sequence so far.
 cudaError_t launch_finish(const ViewConst *views, uint32_t nviews, uint32_t *ctl, int round, uint32_t *host_ctl,
                           cudaStream_t st, bool plain = false);
 struct ExpandView {  // what index expansion reads of an output slot
