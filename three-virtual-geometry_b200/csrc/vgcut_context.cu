@@ -370,6 +370,7 @@ HzbDesc hzb_layout(uint32_t width, uint32_t height, size_t *total_floats) {
     lh = lh > 1 ? (lh + 1) / 2 : 1;
   }
   desc.levels = n;
+  desc.size = width | height << 16;
   *total_floats = total;
   return desc;
 }

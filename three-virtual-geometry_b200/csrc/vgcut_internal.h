@@ -19,6 +19,7 @@
 //   cells       CellRec[C] 128 consecutive instances of one mesh (GeometryPool.ts:519-545)
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -93,11 +94,22 @@ struct Scene {
   uint32_t cell_count, instance_count, meshlet_count, slot_capacity, slots_used;
 };
 
-struct HzbDesc {
+struct HzbHead {  // the start of a descriptor, read at once
   const float *data;
-  uint32_t levels;
-  uint32_t off[kMaxHzbLevels], w[kMaxHzbLevels], h[kMaxHzbLevels];
+  uint32_t levels, size;  // w[0] | h[0] << 16
 };
+struct alignas(16) HzbDesc {
+  const float *data;
+  uint32_t levels, size;
+  uint32_t off[kMaxHzbLevels], w[kMaxHzbLevels], h[kMaxHzbLevels];
+#ifdef __CUDACC__
+  __device__ __forceinline__ HzbHead head() const {
+    const uint4 q = *reinterpret_cast<const uint4 *>(this);
+    return HzbHead{reinterpret_cast<const float *>((uint64_t)q.x | (uint64_t)q.y << 32), q.z, q.w};
+  }
+#endif
+};
+static_assert(offsetof(HzbDesc, size) == 12, "HzbDesc::head reads the first 16 bytes");
 
 // The HZB builds of one launch sequence as one stream of 128 x 32 mip-0 strips (k_hzb_stream): a header, one job per
 // view that brings a depth image, then one tensor map per job. Written on the host into pinned memory and copied
@@ -127,12 +139,14 @@ __host__ __device__ constexpr size_t hzb_plan_bytes(uint32_t jobs) {
 static_assert(sizeof(HzbJob) == 32 && sizeof(HzbPlanHead) == 64, "plan layout");
 
 // Per-view constants derived on the host in double precision (VirtualGeometry.ts:414-442) and stored as float.
-struct ViewConst {
+// Aligned, and its fields grouped, so that a warp reads it 16 bytes at a time.
+struct alignas(16) ViewConst {
   float V[12];        // rows 0..2 of world->view, row-major 3x4
   float plane[24];    // 6 view-space frustum planes (xyz normal, w), normalised (a cascade's: its clip volume)
+  float P0, P5, P8, P9;
+  float P10, P14, near_, inv_proj_scale;  // inv_proj_scale: 1 / proj_scale, rounded once from double
   float sweep[6];     // per-plane max(dot(world normal, shadowSweep), 0)
-  float proj_scale, near_, P0, P5, P8, P9, P10, P14;
-  float inv_proj_scale;  // 1 / proj_scale, rounded once from double
+  float proj_scale;
   float error_threshold, lod_blend_max, shadow_error_scale, lod_scale_limit, min_pixel_radius;
   float budget, budget_lo, budget_hi;  // triangleBudget search (0 = off)
   uint32_t frustum, occl_active;
@@ -162,30 +176,26 @@ struct ViewConst {
 };
 
 #ifdef __CUDACC__
-// Work handed out to warps from a counter, B consecutive pieces at a time (a warp that drew cheap pieces takes more,
-// so a persistent grid finishes together). Lane 0 requests the warp's next batch a whole batch ahead, so the
-// counter's round trip overlaps the work; B > 1 keeps the counter's rate of atomics down when pieces are short.
-// All lanes of the warp call start() and next() together; `i` is the current piece.
-template <uint32_t B>
+// Work handed out to warps: a warp starts with the piece of its own number and takes further ones from a counter (a warp
+// that drew cheap pieces takes more, so a persistent grid finishes together). Lane 0 requests the warp's next piece a
+// whole piece ahead, so the counter's round trip overlaps the work. All lanes of the warp call start() and next()
+// together; `i` is the current piece.
 struct WarpFeed {
   uint32_t *ctr;
-  uint32_t ahead;  // lane 0: the batch after the current one
-  uint32_t i, end;
+  uint32_t ahead;  // lane 0: the piece after the current one
+  uint32_t i;
+  __device__ __forceinline__ uint32_t grab() {
+    return (threadIdx.x & 31) == 0 ? atomicAdd(ctr, 1u) + (gridDim.x * blockDim.x >> 5) : 0u;
+  }
   __device__ __forceinline__ void start(uint32_t *counter) {
     ctr = counter;
-    ahead = 0;
-    if ((threadIdx.x & 31) == 0) ahead = atomicAdd(ctr, 1u);
-    take();
-  }
-  __device__ __forceinline__ void take() {
-    const uint32_t b = __shfl_sync(0xffffffffu, ahead, 0);
-    if ((threadIdx.x & 31) == 0) ahead = atomicAdd(ctr, 1u);
-    i = b * B;
-    end = i + B;
+    i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    ahead = grab();
   }
   // moves to the next piece and returns it
   __device__ __forceinline__ uint32_t next() {
-    if (++i == end) take();
+    i = __shfl_sync(0xffffffffu, ahead, 0);
+    ahead = grab();
     return i;
   }
 };

@@ -774,7 +774,7 @@ __global__ void __launch_bounds__(128, 7) k_visibility(const __grid_constant__ S
   const uint32_t share = total / (gridDim.x * 16u) & ~31u, length = min(max(share, kVisRunMin), kVisRunMax);
   const uint32_t runs = (total + length - 1) / length;
   const uint32_t lane = threadIdx.x & 31;
-  WarpFeed<1> feed;
+  WarpFeed feed;
   feed.start(R.ctl);
   uint32_t slot = kNoTri, known = 0;  // the cached draw slot and how many of its vertices are cached
   uint32_t head = 0, waiting = 0;     // the ring of small triangles
