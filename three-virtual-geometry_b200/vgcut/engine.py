@@ -579,8 +579,8 @@ class VirtualGeometry:
         nr = np.ascontiguousarray(np.broadcast_to(np.asarray(near, np.float64), (n,)))
         sc = np.ascontiguousarray(np.broadcast_to(np.asarray(scale, np.float64), (n,)))
         mcount = next(m for m in self.meshes if m.slot == slot).data.meshlet_count
-        lo = np.zeros((n, mcount), np.uint8)
-        hi = np.zeros((n, mcount), np.uint8)
+        lo = np.empty((n, mcount), np.uint8)
+        hi = np.empty((n, mcount), np.uint8)
         D = C.POINTER(C.c_double)
         check(lib().vgc_select_cut(self.handle, slot, n, vm.ctypes.data_as(D), ps.ctypes.data_as(D),
                                    nr.ctypes.data_as(D), sc.ctypes.data_as(D), threshold, blend,
