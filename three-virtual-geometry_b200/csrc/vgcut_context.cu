@@ -847,6 +847,22 @@ void compute_cell(vgc_context *ctx, uint32_t slot, uint32_t cell) {
   r.count = end - first;
 }
 
+int refresh_mirror(vgc_context *ctx) {
+  bool synced = false;
+  for (uint32_t slot = 0; slot < ctx->slots_used; slot++) {
+    MeshHost &m = ctx->mesh_host[slot];
+    if (!m.moved) continue;
+    cudaSetDevice(ctx->device);
+    if (!synced) CUDA_TRY(cudaDeviceSynchronize());
+    synced = true;
+    CUDA_TRY(cudaMemcpy(&ctx->inst[(size_t)m.instance_base * 4], (const float4 *)ctx->d_inst.ptr + (size_t)m.instance_base * 4,
+                        (size_t)m.instance_count * 64, cudaMemcpyDeviceToHost));
+    for (uint32_t c = 0; c < m.cell_count; c++) compute_cell(ctx, slot, c);
+    m.moved = false;
+  }
+  return VGC_OK;
+}
+
 uint32_t spread10(uint32_t v) {
   v &= 0x3ff;
   uint32_t r = 0;
@@ -1049,6 +1065,7 @@ int vgc_mesh_add(vgc_context *ctx, const vgc_mesh_data *d, const float *matrices
     for (uint32_t i = 0; i < d->meshlet_vertex_count; i++)
       if (d->meshlet_vertices[i] >= d->vertex_count) return fail(VGC_INVALID_ARG, "meshlet_vertices id out of range");
   std::lock_guard<std::mutex> lock(ctx->mu);
+  if (const int rc = refresh_mirror(ctx)) return rc;  // the next upload carries the whole mirror
   uint32_t slot = 0;
   while (slot < ctx->slots_used && ctx->mesh_host[slot].used) slot++;
   if (slot >= ctx->slot_capacity) {
@@ -1184,20 +1201,20 @@ int vgc_instances_update(vgc_context *ctx, uint32_t slot, uint32_t first, uint32
   MeshHost &m = ctx->mesh_host[slot];
   if ((uint64_t)first + count > m.instance_count) return fail(VGC_INVALID_ARG, "instance range out of bounds");
   if (count == 0) return VGC_OK;
-  for (uint32_t g = 0; g < count; g++) {
-    const float *e = matrices + (size_t)g * 16;
-    for (int c = 0; c < 4; c++) ctx->inst[(size_t)(m.instance_base + first + g) * 4 + c] = make_float4(e[c * 4], e[c * 4 + 1], e[c * 4 + 2], e[c * 4 + 3]);
-  }
   const uint32_t c0 = first / kCellSize, c1 = (first + count - 1) / kCellSize;
-  for (uint32_t c = c0; c <= c1; c++) compute_cell(ctx, slot, c);  // the host mirror stays current
-  if (ctx->dirty) return VGC_OK;  // a full upload is pending anyway
+  if (ctx->dirty) {  // a full upload is pending: it carries the host mirror (which mesh_add brought up to date)
+    std::memcpy(&ctx->inst[(size_t)(m.instance_base + first) * 4], matrices, (size_t)count * 64);
+    for (uint32_t c = c0; c <= c1; c++) compute_cell(ctx, slot, c);
+    return VGC_OK;
+  }
   // resident scene: upload the changed matrices and recompute their cells on the device (GeometryPool.ts:505-512
-  // commitInstances), after every launch that may still read them and before any later one
+  // commitInstances), after every launch that may still read them and before any later one. The host mirror stays as it
+  // is until someone needs it (recomputing it here, cells in double, took 1 ms of a call that moves 50,000 instances).
   cudaSetDevice(ctx->device);
   CUDA_TRY(cudaDeviceSynchronize());
+  m.moved = true;
   float4 *d_inst = (float4 *)ctx->d_inst.ptr + (size_t)(m.instance_base + first) * 4;
-  CUDA_TRY(cudaMemcpyAsync(d_inst, &ctx->inst[(size_t)(m.instance_base + first) * 4], (size_t)count * 64,
-                           cudaMemcpyHostToDevice, ctx->stream));
+  CUDA_TRY(cudaMemcpyAsync(d_inst, matrices, (size_t)count * 64, cudaMemcpyHostToDevice, ctx->stream));
   const double sphere[4] = {m.sphere[0], m.sphere[1], m.sphere[2], m.sphere[3]};
   CUDA_TRY(launch_cells_update((const float4 *)ctx->d_inst.ptr, sphere, m.instance_base, m.instance_count, m.cell_base,
                                slot, c0, c1 - c0 + 1, (CellRec *)ctx->d_cells.ptr, ctx->stream));
@@ -1625,6 +1642,8 @@ int vgc_kernel_times(vgc_context *ctx, double *ms, uint32_t *launches, int reset
 int vgc_debug_scene(const vgc_context *ctx, float *cells, uint32_t cell_capacity, float *matrices,
                     uint32_t matrix_capacity, uint32_t *cell_count, uint32_t *instance_count) {
   if (!ctx) return fail(VGC_INVALID_ARG, "null context");
+  if (cells || matrices)
+    if (const int rc = refresh_mirror(const_cast<vgc_context *>(ctx))) return rc;
   if (cell_count) *cell_count = (uint32_t)ctx->cells.size();
   if (instance_count) *instance_count = (uint32_t)ctx->inst_slot.size();
   if (cells)

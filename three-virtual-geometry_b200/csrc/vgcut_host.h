@@ -37,6 +37,7 @@ struct MeshHost {
   uint32_t instance_base = 0, instance_count = 0;
   uint32_t cell_base = 0, cell_count = 0;
   uint32_t vertex_base = 0, vertex_count = 0;  // vertex data (0 when the mesh has none)
+  bool moved = false;  // the device holds newer instances than the host mirror (refresh_mirror)
   float sphere[4];
 };
 
@@ -196,6 +197,9 @@ int prepare_multi(vgc_context *const *ctxs, uint32_t nctx, LaunchScratch &s, con
 int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st, bool capture);
 // vgc_stats of one view from its counter header and dyn[0] (the threshold the cut used).
 void decode_stats(const vgc_context *ctx, const uint32_t *counters, float threshold, vgc_stats *s);
+// Brings the host mirror of moved instances and their cells up to date from the device. While a scene is resident,
+// instance updates and re-sorts leave the mirror alone; whoever reads or extends it calls this first.
+int refresh_mirror(vgc_context *ctx);
 // Host mirror: cell `cell` of mesh `slot` from its instances (computeCell, GeometryPool.ts:519-545).
 void compute_cell(vgc_context *ctx, uint32_t slot, uint32_t cell);
 // Host mirror: mortonOrder (GeometryPool.ts:1263-1284) of n column-major matrices.

@@ -8,9 +8,11 @@
 //
 // Every double expression rounds step by step in the host's order (the library is compiled with -fmad=false), so
 // the codes equal the host's. The sort is CUB's stable LSD radix sort over the 30 key bits; the permutation and the
-// cells (k_cells_update, double, in the host's operation order) follow on the device, and the host mirror is
-// permuted and its cells recomputed from the same matrices.
+// cells (k_cells_update, double, in the host's operation order) follow on the device; the host mirror of a resident
+// scene follows when someone needs it (refresh_mirror).
 #include <cub/device/device_radix_sort.cuh>
+
+#include <cstring>
 
 #include "vgcut_host.h"
 #include "vgcut_kernels.h"
@@ -63,17 +65,25 @@ __global__ void __launch_bounds__(kBlock) k_morton_centres(const float4 *__restr
   }
 }
 
-// One block: the mesh's lo / hi from the blocks' partials, then extent (bounds[0..2] lo, bounds[3] extent).
+// One block: the mesh's lo / hi from the blocks' partials, then extent (bounds[0..2] lo, bounds[3] extent). Minima and
+// maxima by shuffles (exact in any order): one thread over the block's values took 11 us.
 __global__ void __launch_bounds__(kBlock) k_morton_bounds(const double *__restrict__ partial, uint32_t blocks,
                                                           double *__restrict__ bounds) {
-  __shared__ double red[6][kBlock];
+  __shared__ double red[6][kBlock / 32];
   double v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
   for (uint32_t b = threadIdx.x; b < blocks; b += kBlock)
     for (int a = 0; a < 6; a++) v[a] = a < 3 ? fmin(v[a], partial[(size_t)b * 6 + a]) : fmax(v[a], partial[(size_t)b * 6 + a]);
-  for (int a = 0; a < 6; a++) red[a][threadIdx.x] = v[a];
+  const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int a = 0; a < 6; a++)
+    for (int o = 16; o > 0; o >>= 1) {
+      const double t = __shfl_down_sync(0xffffffffu, v[a], o);
+      v[a] = a < 3 ? fmin(v[a], t) : fmax(v[a], t);
+    }
+  if (lane == 0)
+    for (int a = 0; a < 6; a++) red[a][w] = v[a];
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (uint32_t k = 1; k < kBlock; k++)
+    for (uint32_t k = 1; k < kBlock / 32; k++)
       for (int a = 0; a < 6; a++) v[a] = a < 3 ? fmin(v[a], red[a][k]) : fmax(v[a], red[a][k]);
     double extent = v[3] - v[0];
     extent = fmax(extent, v[4] - v[1]);
@@ -114,7 +124,6 @@ extern "C" int vgc_instances_resort(vgc_context *ctx, uint32_t slot, uint32_t *n
   if (slot >= ctx->slots_used || !ctx->mesh_host[slot].used) return fail(VGC_NOT_FOUND, "no mesh in slot");
   MeshHost &m = ctx->mesh_host[slot];
   const uint32_t n = m.instance_count;
-  std::vector<uint32_t> order(n);
   if (!ctx->dirty && n > 1) {
     // resident scene: codes, sort, permutation and cells on the device
     cudaSetDevice(ctx->device);
@@ -167,31 +176,28 @@ extern "C" int vgc_instances_resort(vgc_context *ctx, uint32_t slot, uint32_t *n
       e = launch_cells_update((const float4 *)ctx->d_inst.ptr, sphere, m.instance_base, n, m.cell_base, slot, 0,
                               m.cell_count, (CellRec *)ctx->d_cells.ptr, ctx->stream);
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(order.data(), idx_out, keys_b, cudaMemcpyDeviceToHost, ctx->stream);
+    m.moved = true;
+    if (e == cudaSuccess && new_to_old)
+      e = cudaMemcpyAsync(new_to_old, idx_out, keys_b, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(VGC_DEVICE_ERROR, std::string("vgc_instances_resort: ") + cudaGetErrorString(e));
     }
-  } else if (n > 1) {
+    return VGC_OK;
+  }
+  std::vector<uint32_t> order(n);
+  if (n > 1) {
     // the scene is not resident (a full upload is pending): the host order, which that upload carries
     std::vector<float> mats((size_t)n * 16);
-    for (uint32_t g = 0; g < n; g++)
-      for (int c = 0; c < 4; c++) {
-        const float4 v = ctx->inst[(size_t)(m.instance_base + g) * 4 + c];
-        mats[(size_t)g * 16 + c * 4] = v.x, mats[(size_t)g * 16 + c * 4 + 1] = v.y;
-        mats[(size_t)g * 16 + c * 4 + 2] = v.z, mats[(size_t)g * 16 + c * 4 + 3] = v.w;
-      }
+    std::memcpy(mats.data(), &ctx->inst[(size_t)m.instance_base * 4], (size_t)n * 64);
     morton_order(mats.data(), n, m.sphere, order);
+    for (uint32_t g = 0; g < n; g++)
+      std::memcpy(&ctx->inst[(size_t)(m.instance_base + g) * 4], &mats[(size_t)order[g] * 16], 64);
+    for (uint32_t c = 0; c < m.cell_count; c++) compute_cell(ctx, slot, c);
   } else {
     for (uint32_t g = 0; g < n; g++) order[g] = g;
   }
-  // the host mirror: the same permutation, cells recomputed from the same matrices
-  std::vector<float4> old(ctx->inst.begin() + (size_t)m.instance_base * 4,
-                          ctx->inst.begin() + (size_t)(m.instance_base + n) * 4);
-  for (uint32_t g = 0; g < n; g++)
-    for (int c = 0; c < 4; c++) ctx->inst[(size_t)(m.instance_base + g) * 4 + c] = old[(size_t)order[g] * 4 + c];
-  for (uint32_t c = 0; c < m.cell_count; c++) compute_cell(ctx, slot, c);
   if (new_to_old)
     for (uint32_t g = 0; g < n; g++) new_to_old[g] = order[g];
   return VGC_OK;

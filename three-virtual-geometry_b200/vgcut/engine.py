@@ -297,10 +297,18 @@ class VirtualMesh:
         check(lib().vgc_mesh_add(vg.handle, C.byref(md), _fp(m), self.instance_count, C.byref(self._opts()),
                                  C.byref(slot), _up(self.gpu_to_input)))
         self.slot = slot.value
-        self.gpu_index_of = np.empty_like(self.gpu_to_input)
-        self.gpu_index_of[self.gpu_to_input] = np.arange(self.instance_count, dtype=np.uint32)
-        self._matrices = m[self.gpu_to_input].copy()  # GPU (Morton) order
+        self._gpu_index_of = None
+        self._matrices = m.copy()  # caller order: a re-sort leaves it alone
         self._dirty: set[int] = set()
+        self._upload = None  # commit_instances' block in GPU order
+
+    @property
+    def gpu_index_of(self) -> np.ndarray:
+        """GPU (Morton) index of each caller index: the inverse of gpu_to_input, made when first asked for."""
+        if self._gpu_index_of is None:
+            self._gpu_index_of = np.empty_like(self.gpu_to_input)
+            self._gpu_index_of[self.gpu_to_input] = np.arange(self.instance_count, dtype=np.uint32)
+        return self._gpu_index_of
 
     def _opts(self) -> MeshOpts:
         f = self._flags
@@ -326,14 +334,12 @@ class VirtualMesh:
 
     def set_matrix_at(self, index: int, matrix: np.ndarray) -> None:
         """Updates one instance (caller index). Call ``commit_instances`` afterwards (VirtualMesh.ts:305-309)."""
-        g = int(self.gpu_index_of[index])
-        self._matrices[g] = np.asarray(matrix, np.float32).reshape(16)
-        self._dirty.add(g)
+        self._matrices[index] = np.asarray(matrix, np.float32).reshape(16)
+        self._dirty.add(int(self.gpu_index_of[index]))
 
     def set_matrices(self, matrices: np.ndarray) -> None:
         """Updates every instance (caller order, (n, 16)); ``commit_instances`` uploads them in one call."""
-        m = np.ascontiguousarray(matrices, np.float32).reshape(self.instance_count, 16)
-        self._matrices[:] = m[self.gpu_to_input]
+        self._matrices[:] = np.asarray(matrices, np.float32).reshape(self.instance_count, 16)
         if self.instance_count:
             self._dirty.update((0, self.instance_count - 1))
 
@@ -341,7 +347,10 @@ class VirtualMesh:
         if not self._dirty:
             return
         lo, hi = min(self._dirty), max(self._dirty)
-        block = np.ascontiguousarray(self._matrices[lo:hi + 1])
+        if self._upload is None or len(self._upload) < hi - lo + 1:
+            self._upload = np.empty((self.instance_count, 16), np.float32)
+        block = self._upload[:hi - lo + 1]  # kept: fresh pages for each call cost more than the gather itself
+        np.take(self._matrices, self.gpu_to_input[lo:hi + 1], axis=0, out=block, mode="clip")
         check(lib().vgc_instances_update(self.vg.handle, self.slot, lo, hi - lo + 1, _fp(block)))
         self._dirty.clear()
 
@@ -352,8 +361,7 @@ class VirtualMesh:
         new_to_old = np.zeros(self.instance_count, np.uint32)
         check(lib().vgc_instances_resort(self.vg.handle, self.slot, _up(new_to_old)))
         self.gpu_to_input = self.gpu_to_input[new_to_old]
-        self.gpu_index_of[self.gpu_to_input] = np.arange(self.instance_count, dtype=np.uint32)
-        self._matrices = self._matrices[new_to_old]
+        self._gpu_index_of = None
         return new_to_old
 
     def dispose(self) -> None:
