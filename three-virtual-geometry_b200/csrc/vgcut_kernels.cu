@@ -1763,7 +1763,6 @@ struct StripDesc {
   float *out;
   uint32_t levels;
   uint32_t off[5], w[5], h[5];
-  bool pairs;  // levels 1..4 exist and pairs of level-1 texels are 8-byte aligned
 };
 
 __device__ __forceinline__ void strip_desc(const HzbDesc &H, StripDesc &D) {
@@ -1771,7 +1770,6 @@ __device__ __forceinline__ void strip_desc(const HzbDesc &H, StripDesc &D) {
   D.levels = H.levels;
 #pragma unroll
   for (int l = 0; l < 5; l++) D.off[l] = H.off[l], D.w[l] = H.w[l], D.h[l] = H.h[l];
-  D.pairs = H.levels > 4 && ((D.off[1] | D.w[1]) & 1u) == 0 && (reinterpret_cast<uintptr_t>(H.data) & 7u) == 0;
 }
 
 __device__ __forceinline__ void strip_store(const StripDesc &D, uint32_t l, uint32_t x, uint32_t y, float v) {
@@ -1918,32 +1916,18 @@ __global__ void __launch_bounds__(kHzbStreamThreads, VGC_HZB_BLOCKS_PER_SM) k_hz
 #pragma unroll
     for (int i = 0; i < 2; i++)
 #pragma unroll
-      for (int j = 0; j < 2; j++)
+      for (int j = 0; j < 2; j++) {
         a[i][j] = fmaxf(fmaxf(v[2 * i][2 * j], v[2 * i][2 * j + 1]), fmaxf(v[2 * i + 1][2 * j], v[2 * i + 1][2 * j + 1]));
+        strip_store(D, 1, gx / 2 + j, gy / 2 + i, a[i][j]);
+      }
     const float b = fmaxf(fmaxf(a[0][0], a[0][1]), fmaxf(a[1][0], a[1][1]));
+    strip_store(D, 2, gx / 4, gy / 4, b);
     float m3 = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, 1));
     m3 = fmaxf(m3, __shfl_xor_sync(0xffffffffu, m3, 8));
+    if ((lane & 9u) == 0) strip_store(D, 3, gx / 8, gy / 8, m3);
     float m4 = fmaxf(m3, __shfl_xor_sync(0xffffffffu, m3, 2));
     m4 = fmaxf(m4, __shfl_xor_sync(0xffffffffu, m4, 16));
-    if (inside && D.pairs) {
-      // a strip wholly inside the image has all its texels of levels 1..4: no checks, level 1 in pairs
-      float *o1 = D.out + D.off[1] + (size_t)(gy / 2) * D.w[1] + gx / 2;
-      *reinterpret_cast<float2 *>(o1) = make_float2(a[0][0], a[0][1]);
-      *reinterpret_cast<float2 *>(o1 + D.w[1]) = make_float2(a[1][0], a[1][1]);
-      D.out[D.off[2] + (size_t)(gy / 4) * D.w[2] + gx / 4] = b;
-      if ((lane & 9u) == 0) {
-        D.out[D.off[3] + (size_t)(gy / 8) * D.w[3] + gx / 8] = m3;
-        if ((lane & 27u) == 0) D.out[D.off[4] + (size_t)(gy / 16) * D.w[4] + gx / 16] = m4;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 2; j++) strip_store(D, 1, gx / 2 + j, gy / 2 + i, a[i][j]);
-      strip_store(D, 2, gx / 4, gy / 4, b);
-      if ((lane & 9u) == 0) strip_store(D, 3, gx / 8, gy / 8, m3);
-      if ((lane & 27u) == 0) strip_store(D, 4, gx / 16, gy / 16, m4);
-    }
+    if ((lane & 27u) == 0) strip_store(D, 4, gx / 16, gy / 16, m4);
     if (*flag) return;  // another warp gave up
   }
 }
