@@ -1487,169 +1487,172 @@ __global__ void __launch_bounds__(256) k_expand(Scene S, const ExpandView V, uin
 // induction every texel of mip i is the max over its mip-0 footprint [2^i x, 2^i (x+1)) x [2^i y, 2^i (y+1)) inside
 // the image, so a reduction whose loads clamp to the image edge gives the same values.
 //
-// One 64x64 tile of mip 0 per block of 256 threads: each thread reduces a 4x4 patch (float4 rows when the image
-// allows) to its 2x2 texels of mip 1 and its texel of mip 2 in registers; mips 3..6 of the tile come from shared
-// memory (tiles are aligned to 64, so every clamped neighbour lies inside the tile); mips 7+ by the tail kernel.
-constexpr uint32_t kHzbTile = 64, kHzbTileLevels = 7;
+// One 64 x 64 tile of mip 0 per block of four warps: warp w reduces rows 16 w .. 16 w + 15 of the tile to level 4 in
+// registers, warp 0 the four warps' level 4 to levels 5 and 6 (tiles are aligned to 64, so every clamped neighbour lies
+// inside the tile); levels 7 and up by the tail kernel.
+constexpr uint32_t kHzbTile = 64, kHzbTileThreads = 128, kHzbTileLevels = 7;
 
 __device__ __forceinline__ void hzb_store(const HzbDesc &H, float *__restrict__ out, uint32_t l, uint32_t x, uint32_t y,
                                           float v) {
   if (l < H.levels && x < H.w[l] && y < H.h[l]) out[H.off[l] + (size_t)y * H.w[l] + x] = v;
 }
 
-// Levels 3..6 of the tile use no clamped reads: a texel's neighbour past the level's edge holds the max over the
-// edge texels of the same rows (or columns), which the in-range texel's footprint already contains, so the max over
-// the 2x2 block equals the max over its clamped reads. Level 3 is warp-local (a warp holds two rows of level 2); one
-// barrier hands the tile's 8x8 level-3 texels to warp 0 for levels 4..6.
-// This thread's 4x4 patch of mip 0 of the tile at (ox, oy) (loads clamped to the image).
-__device__ __forceinline__ void hzb_load(const float *__restrict__ depth, const HzbDesc &H, uint32_t ox, uint32_t oy,
-                                         float v[4][4]) {
-  const uint32_t t = threadIdx.x, tx = t & 15u, ty = t >> 4;
-  const uint32_t W = H.w[0], Hh = H.h[0];
-  const uint32_t gx = ox + 4 * tx, gy = oy + 4 * ty;
-  const bool vec = (W & 3u) == 0 && (reinterpret_cast<uintptr_t>(depth) & 15u) == 0 && gx + 3 < W;
-#pragma unroll
-  for (int r = 0; r < 4; r++) {
-    const uint32_t y = min(gy + r, Hh - 1);
-    const float *row = depth + (size_t)y * W;
-    if (vec) {
-      const float4 q = __ldg(reinterpret_cast<const float4 *>(row + gx));
-      v[r][0] = q.x, v[r][1] = q.y, v[r][2] = q.z, v[r][3] = q.w;
-    } else {
-#pragma unroll
-      for (int c = 0; c < 4; c++) v[r][c] = __ldg(row + min(gx + c, W - 1));
-    }
-  }
-}
-
-// Mips 0..6 of the tile at (ox, oy) from the patches hzb_load read (every thread of the block calls it).
+// Mips 0..6 of the tile at (ox, oy) (every thread of the block calls it). Memory-bound; what costs is that an odd width
+// puts no row but the first on a 16-byte boundary. So lane l reads and copies single floats, columns l and l + 32 of
+// a row: whichever the width, a warp's access covers 128 consecutive bytes, and the 32 loads of a lane are in flight
+// together. At 2,555 x 1,437 this kernel takes 6.6 us (34 MB read and written, most of it within L2) where float4-shaped
+// patches read element by element took 10.9; a build with its tail 10.8 us where it took 17.1, at 2,560 x 1,440 10.5
+// where the patches' float4 rows took 12.4.
+//
+// A reduction step halves the columns by one shuffle for two values a lane: the lane keeps one, hands the other to its
+// partner, and the pair's lanes go on with different texels, so that no lane holds a copy until level 3. A level's
+// texel past the level's edge holds the max over the edge texels of the same rows (or columns), which the in-range
+// texel's footprint already contains, so the max over the 2 x 2 block equals the max over its clamped reads.
 __device__ __forceinline__ void hzb_tile64(const float *__restrict__ depth, const HzbDesc &H, float *__restrict__ out,
-                                           bool copy_mip0, uint32_t ox, uint32_t oy, float (*s3)[9],
-                                           const float (&v)[4][4]) {
-  const uint32_t t = threadIdx.x, tx = t & 15u, ty = t >> 4, lane = t & 31u, warp = t >> 5;
+                                           bool copy_mip0, uint32_t ox, uint32_t oy, float (*s4)[4]) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t W = H.w[0], Hh = H.h[0];
-  const uint32_t gx = ox + 4 * tx, gy = oy + 4 * ty;
-  const bool vec = (W & 3u) == 0 && (reinterpret_cast<uintptr_t>(depth) & 15u) == 0 && gx + 3 < W;
+  const uint32_t x0 = ox + lane, x1 = x0 + 32, y0 = oy + 16 * warp;
+  float v[16][2];
+#pragma unroll
+  for (int r = 0; r < 16; r++) {
+    const float *row = depth + (size_t)min(y0 + r, Hh - 1) * W;
+    v[r][0] = __ldg(row + min(x0, W - 1));
+    v[r][1] = __ldg(row + min(x1, W - 1));
+  }
   if (copy_mip0) {
-    float *o0 = out + H.off[0];
+    float *o = out + H.off[0];
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-      if (gy + r >= Hh) continue;
-      float *row = o0 + (size_t)(gy + r) * W;
-      if (vec && (reinterpret_cast<uintptr_t>(o0) & 15u) == 0) {
-        *reinterpret_cast<float4 *>(row + gx) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
-      } else {
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-          if (gx + c < W) row[gx + c] = v[r][c];
-      }
+    for (int r = 0; r < 16; r++) {
+      if (y0 + r >= Hh) break;
+      float *row = o + (size_t)(y0 + r) * W;
+      if (x0 < W) row[x0] = v[r][0];
+      if (x1 < W) row[x1] = v[r][1];
     }
   }
-  float a[2][2];
+  const bool odd = lane & 1u, hi2 = lane & 2u, hi4 = lane & 4u;
+  // level 1: lane 2 c holds column c, lane 2 c + 1 column 16 + c of the tile's 32
+  float a[8];
 #pragma unroll
-  for (int i = 0; i < 2; i++)
-#pragma unroll
-    for (int j = 0; j < 2; j++)
-      a[i][j] = fmaxf(fmaxf(v[2 * i][2 * j], v[2 * i][2 * j + 1]), fmaxf(v[2 * i + 1][2 * j], v[2 * i + 1][2 * j + 1]));
+  for (int i = 0; i < 8; i++) {
+    const float p = fmaxf(v[2 * i][0], v[2 * i + 1][0]), q = fmaxf(v[2 * i][1], v[2 * i + 1][1]);
+    a[i] = fmaxf(odd ? q : p, __shfl_xor_sync(0xffffffffu, odd ? p : q, 1));
+  }
   if (H.levels > 1) {
-    float *o1 = out + H.off[1];
+    const uint32_t x = (ox >> 1) + (odd ? 16u : 0u) + (lane >> 1);
+    float *o = out + H.off[1];
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int i = 0; i < 8; i++) {
+      const uint32_t y = (y0 >> 1) + i;
+      if (x < H.w[1] && y < H.h[1]) o[(size_t)y * H.w[1] + x] = a[i];
+    }
+  }
+  // level 2: rows 2 i + bit 1 of the lane, column c2
+  float b[2];
+  const uint32_t c2 = (odd ? 8u : 0u) + (lane >> 2);
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const uint32_t x = gx / 2 + j, y = gy / 2 + i;
-        if (x < H.w[1] && y < H.h[1]) o1[(size_t)y * H.w[1] + x] = a[i][j];
-      }
+  for (int i = 0; i < 2; i++) {
+    const float p = fmaxf(a[4 * i], a[4 * i + 1]), q = fmaxf(a[4 * i + 2], a[4 * i + 3]);
+    b[i] = fmaxf(hi2 ? q : p, __shfl_xor_sync(0xffffffffu, hi2 ? p : q, 2));
+    hzb_store(H, out, 2, (ox >> 2) + c2, (y0 >> 2) + 2 * i + (hi2 ? 1u : 0u), b[i]);
   }
-  const float b = fmaxf(fmaxf(a[0][0], a[0][1]), fmaxf(a[1][0], a[1][1]));
-  hzb_store(H, out, 2, gx / 4, gy / 4, b);
-  // level 3: texel (tx / 2, warp) of the tile from lanes tx, tx ^ 1 of rows 2 warp, 2 warp + 1
-  float m = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, 1));
-  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
-  if ((lane & 17u) == 0) {
-    hzb_store(H, out, 3, (ox >> 3) + (tx >> 1), (oy >> 3) + warp, m);
-    s3[warp][tx >> 1] = m;
+  // level 3: row = bit 2 of the lane, column c2 / 2 (both lanes of bit 1 hold it)
+#pragma unroll
+  for (int i = 0; i < 2; i++) b[i] = fmaxf(b[i], __shfl_xor_sync(0xffffffffu, b[i], 2));
+  float m = fmaxf(hi4 ? b[1] : b[0], __shfl_xor_sync(0xffffffffu, hi4 ? b[0] : b[1], 4));
+  if (!hi2) hzb_store(H, out, 3, (ox >> 3) + (c2 >> 1), (y0 >> 3) + (hi4 ? 1u : 0u), m);
+  // level 4: one row of four texels
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+  if ((lane & 14u) == 0) {
+    hzb_store(H, out, 4, (ox >> 4) + (c2 >> 2), y0 >> 4, m);
+    s4[warp][c2 >> 2] = m;
   }
+  if (H.levels <= 5) return;  // uniform over the block
   __syncthreads();
-  if (warp != 0 || H.levels <= 4) return;
-  // levels 4..6 by warp 0: lane = 4 y + x of level 4 (16 lanes), then xor 1 / 4 and xor 2 / 8 pair up the blocks
-  const uint32_t x4 = lane & 3u, y4 = (lane >> 2) & 3u;
-  float m4 = fmaxf(fmaxf(s3[2 * y4][2 * x4], s3[2 * y4][2 * x4 + 1]), fmaxf(s3[2 * y4 + 1][2 * x4], s3[2 * y4 + 1][2 * x4 + 1]));
-  if (lane < 16) hzb_store(H, out, 4, (ox >> 4) + x4, (oy >> 4) + y4, m4);
-  float m5 = fmaxf(m4, __shfl_xor_sync(0xffffffffu, m4, 1));
-  m5 = fmaxf(m5, __shfl_xor_sync(0xffffffffu, m5, 4));
-  if (lane < 16 && (lane & 5u) == 0) hzb_store(H, out, 5, (ox >> 5) + (x4 >> 1), (oy >> 5) + (y4 >> 1), m5);
-  float m6 = fmaxf(m5, __shfl_xor_sync(0xffffffffu, m5, 2));
-  m6 = fmaxf(m6, __shfl_xor_sync(0xffffffffu, m6, 8));
-  if (lane == 0) hzb_store(H, out, 6, ox >> 6, oy >> 6, m6);
+  if (warp != 0) return;
+  // levels 5 and 6: lane = 4 y + x of level 4 (16 lanes)
+  m = s4[(lane >> 2) & 3u][lane & 3u];
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+  if (lane < 16 && (lane & 5u) == 0) hzb_store(H, out, 5, (ox >> 5) + ((lane >> 1) & 1u), (oy >> 5) + (lane >> 3), m);
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+  if (lane == 0) hzb_store(H, out, 6, ox >> 6, oy >> 6, m);
 }
 
-// Two vertically adjacent tiles per block: both tiles' loads are in flight before the first tile is reduced.
-__device__ __forceinline__ void hzb_tile_pair(const float *__restrict__ depth, const HzbDesc &H, float *__restrict__ out,
-                                              bool copy_mip0, uint32_t ox, uint32_t oy, float (*s3)[9]) {
-  const bool second = oy + kHzbTile < H.h[0];  // uniform over the block
-  float a[4][4], b[4][4];
-  hzb_load(depth, H, ox, oy, a);
-  if (second) hzb_load(depth, H, ox, oy + kHzbTile, b);
-  hzb_tile64(depth, H, out, copy_mip0, ox, oy, s3, a);
-  if (second) {
-    __syncthreads();  // warp 0 has read the first tile's level 3 from s3
-    hzb_tile64(depth, H, out, copy_mip0, ox, oy + kHzbTile, s3, b);
-  }
-}
-
-__global__ void __launch_bounds__(256) k_hzb_tiles(const float *__restrict__ depth, HzbDesc H, float *__restrict__ out,
-                                                   int copy_mip0) {
-  __shared__ float s3[8][9];
-  hzb_tile_pair(depth, H, out, copy_mip0 != 0, blockIdx.x * kHzbTile, blockIdx.y * 2 * kHzbTile, s3);
+__global__ void __launch_bounds__(kHzbTileThreads) k_hzb_tiles(const float *__restrict__ depth, HzbDesc H,
+                                                               float *__restrict__ out, int copy_mip0) {
+  __shared__ float s4[4][4];
+  wait_previous_kernel();
+  hzb_tile64(depth, H, out, copy_mip0 != 0, blockIdx.x * kHzbTile, blockIdx.y * kHzbTile, s4);
 }
 
 // The HZB builds of a batch: grid.z = view, views without a depth image skip.
-__global__ void __launch_bounds__(256) k_hzb_tiles_views(const ViewConst *__restrict__ views) {
-  __shared__ float s3[8][9];
+__global__ void __launch_bounds__(kHzbTileThreads) k_hzb_tiles_views(const ViewConst *__restrict__ views) {
+  __shared__ float s4[4][4];
+  wait_previous_kernel();
   const ViewConst &V = views[blockIdx.z];
   if (!V.build_hzb) return;
   const HzbDesc &H = *V.hzb_desc;
-  const uint32_t ox = blockIdx.x * kHzbTile, oy = blockIdx.y * 2 * kHzbTile;
+  const uint32_t ox = blockIdx.x * kHzbTile, oy = blockIdx.y * kHzbTile;
   if (ox >= H.w[0] || oy >= H.h[0]) return;
-  hzb_tile_pair(V.depth, H, const_cast<float *>(H.data), V.hzb_mip0 == nullptr, ox, oy, s3);
+  hzb_tile64(V.depth, H, const_cast<float *>(H.data), V.hzb_mip0 == nullptr, ox, oy, s4);
 }
 
-// Levels `first` and up of each building view's HZB, one block per view (the tile kernels wrote the levels below).
+// Levels `first` and up of one HZB by one block (the tile or strip kernel wrote the level below). The kernel is a chain
+// of short dependent steps, and a level read back from memory puts an L2 round trip into each: so a level of up to
+// 4,096 texels is also kept in shared memory for the next one (all of a 4K image's from level 5; the larger levels of
+// wider images go through memory). Launched behind the tile kernel's last blocks it adds 2 us to a build, which it
+// added 5.5 us to.
+constexpr uint32_t kTailTexels = 4096;
+struct TailSmem {
+  uint32_t off[kMaxHzbLevels], w[kMaxHzbLevels], h[kMaxHzbLevels];
+  float even[kTailTexels], odd[kTailTexels / 2];  // a level of 4,096 texels has at most 2,048 in the next
+};
+
+__device__ __forceinline__ void hzb_tail(const HzbDesc &H, float *__restrict__ out, uint32_t first, TailSmem &S) {
+  const uint32_t levels = H.levels;
+  if (threadIdx.x < kMaxHzbLevels) {
+    S.off[threadIdx.x] = H.off[threadIdx.x];
+    S.w[threadIdx.x] = H.w[threadIdx.x];
+    S.h[threadIdx.x] = H.h[threadIdx.x];
+  }
+  __syncthreads();
+  const float *src = out + S.off[first - 1];
+  uint32_t kept = 0;
+  for (uint32_t l = first; l < levels; l++) {
+    const uint32_t sw = S.w[l - 1], sh = S.h[l - 1], w = S.w[l], n = w * S.h[l];
+    float *dst = out + S.off[l], *keep = n > kTailTexels ? nullptr : kept++ & 1u ? S.odd : S.even;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+      const uint32_t y = i / w, x = i - y * w;
+      const uint32_t x0 = 2 * x, y0 = 2 * y, x1 = min(x0 + 1, sw - 1), y1 = min(y0 + 1, sh - 1);
+      const float a = fmaxf(src[y0 * sw + x0], src[y0 * sw + x1]);
+      const float b = fmaxf(src[y1 * sw + x0], src[y1 * sw + x1]);
+      const float m = fmaxf(a, b);
+      dst[i] = m;
+      if (keep) keep[i] = m;
+    }
+    __syncthreads();
+    src = keep ? keep : dst;
+  }
+}
+
+// The tails of a launch's building views, one block per view.
 __global__ void __launch_bounds__(1024) k_hzb_tail_views(const ViewConst *__restrict__ views, uint32_t first) {
+  __shared__ TailSmem S;
   wait_previous_kernel();
   const ViewConst &V = views[blockIdx.x];
   if (!V.build_hzb) return;
   const HzbDesc &H = *V.hzb_desc;
-  float *out = const_cast<float *>(H.data);
-  for (uint32_t l = first; l < H.levels; l++) {
-    const float *src = out + H.off[l - 1];
-    const uint32_t sw = H.w[l - 1], sh = H.h[l - 1];
-    for (uint32_t i = threadIdx.x; i < H.w[l] * H.h[l]; i += blockDim.x) {
-      const uint32_t x = i % H.w[l], y = i / H.w[l];
-      const uint32_t x0 = 2 * x, y0 = 2 * y, x1 = min(x0 + 1, sw - 1), y1 = min(y0 + 1, sh - 1);
-      const float a = fmaxf(src[y0 * sw + x0], src[y0 * sw + x1]);
-      const float b = fmaxf(src[y1 * sw + x0], src[y1 * sw + x1]);
-      out[H.off[l] + i] = fmaxf(a, b);
-    }
-    __syncthreads();
-  }
+  if (first < H.levels) hzb_tail(H, const_cast<float *>(H.data), first, S);
 }
 
-// Levels 7 and up (at most 15 x 9 texels for a 1080p mip 0) by one block.
+// Levels 7 and up (at most 15 x 9 texels for a 1080p mip 0).
 __global__ void __launch_bounds__(1024) k_hzb_tail(HzbDesc H, float *__restrict__ out) {
-  for (uint32_t l = kHzbTileLevels; l < H.levels; l++) {
-    const float *src = out + H.off[l - 1];
-    const uint32_t sw = H.w[l - 1], sh = H.h[l - 1];
-    for (uint32_t i = threadIdx.x; i < H.w[l] * H.h[l]; i += blockDim.x) {
-      const uint32_t x = i % H.w[l], y = i / H.w[l];
-      const uint32_t x0 = 2 * x, y0 = 2 * y, x1 = min(x0 + 1, sw - 1), y1 = min(y0 + 1, sh - 1);
-      const float a = fmaxf(src[y0 * sw + x0], src[y0 * sw + x1]);
-      const float b = fmaxf(src[y1 * sw + x0], src[y1 * sw + x1]);
-      out[H.off[l] + i] = fmaxf(a, b);
-    }
-    __syncthreads();
-  }
+  __shared__ TailSmem S;
+  wait_previous_kernel();
+  hzb_tail(H, out, kHzbTileLevels, S);
 }
 
 // ------------------------------------------------------------------------------------------------ HZB strip stream
@@ -2116,10 +2119,10 @@ cudaError_t launch_cells_update(const float4 *inst, const double sphere[4], uint
 // without, because it follows an event of another stream, or because other streams' batches share the device (blocks
 // that wait would keep their places from them).
 template <class... P, class... A>
-static cudaError_t launch_after(bool plain, void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem,
+static cudaError_t launch_after(bool plain, void (*kernel)(P...), dim3 grid, uint32_t block, size_t smem,
                                 cudaStream_t st, A &&...args) {
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -2228,22 +2231,19 @@ cudaError_t launch_expand(const Scene &S, const ExpandView &view, uint32_t cut, 
 }
 
 cudaError_t launch_hzb(const float *depth, const HzbDesc &H, float *out, int copy_mip0, cudaStream_t st) {
-  dim3 grid((H.w[0] + kHzbTile - 1) / kHzbTile, (H.h[0] + 2 * kHzbTile - 1) / (2 * kHzbTile));
-  k_hzb_tiles<<<grid, 256, 0, st>>>(depth, H, out, copy_mip0);
-  cudaError_t e = cudaGetLastError();
+  const dim3 grid((H.w[0] + kHzbTile - 1) / kHzbTile, (H.h[0] + kHzbTile - 1) / kHzbTile);
+  cudaError_t e = launch_after(false, k_hzb_tiles, grid, kHzbTileThreads, 0, st, depth, H, out, copy_mip0);
   if (e != cudaSuccess || H.levels <= kHzbTileLevels) return e;
-  k_hzb_tail<<<1, 1024, 0, st>>>(H, out);
-  return cudaGetLastError();
+  return launch_after(false, k_hzb_tail, 1, 1024, 0, st, H, out);
 }
 
 cudaError_t launch_hzb_views(const ViewConst *views, uint32_t nviews, uint32_t max_w,
                              uint32_t max_h, bool tail, cudaStream_t st) {
-  dim3 grid((max_w + kHzbTile - 1) / kHzbTile, (max_h + 2 * kHzbTile - 1) / (2 * kHzbTile), nviews);
-  k_hzb_tiles_views<<<grid, 256, 0, st>>>(views);
+  const dim3 grid((max_w + kHzbTile - 1) / kHzbTile, (max_h + kHzbTile - 1) / kHzbTile, nviews);
+  k_hzb_tiles_views<<<grid, kHzbTileThreads, 0, st>>>(views);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !tail) return e;
-  k_hzb_tail_views<<<nviews, 1024, 0, st>>>(views, kHzbTileLevels);
-  return cudaGetLastError();
+  return launch_after(false, k_hzb_tail_views, nviews, 1024, 0, st, views, kHzbTileLevels);
 }
 
 cudaError_t launch_wait_probe(uint64_t limit_ns, unsigned long long *out, cudaStream_t st) {
