@@ -67,31 +67,35 @@ static void free_select(vgc_context *ctx) {
   if (ctx->d_select.ptr) {
     cudaFree(ctx->d_select.ptr);
     ctx->bytes -= ctx->d_select.bytes;
+    ctx->uncharged -= ctx->d_select.bytes;
   }
-  if (ctx->h_select) cudaFreeHost(ctx->h_select);
-  if (ctx->select_lo) cudaEventDestroy(ctx->select_lo);
   ctx->d_select = DevBuf();
-  ctx->h_select = nullptr;
-  ctx->select_lo = nullptr;
 }
 
-// The kept workspace, for `bytes` at least (at most kSelectKeep): device buffer, pinned buffer of the same size, event.
-// It is never what the context's HBM budget refuses: dev_alloc gives it back first.
+// The kept workspace: a device buffer for `bytes` at least (at most kSelectKeep), and the pinned pieces its results
+// come back through. Not charged to the context's HBM budget, and given back when the device runs out of memory.
+// Pinned memory costs 1.2 ms for the first 2 MB and 0.4 ms for each further MB, which a context's first call pays: so
+// results pass through kSelectPieces small pieces instead of a buffer of their size.
 constexpr size_t kSelectKeep = 32u << 20;
+constexpr size_t kSelectPiece = 256u << 10;
 static int select_workspace(vgc_context *ctx, size_t bytes) {
-  if (ctx->d_select.bytes >= bytes) return VGC_OK;
-  free_select(ctx);
-  size_t want = size_t(1) << 20;
-  while (want < bytes) want *= 2;
-  cudaError_t e = cudaMalloc(&ctx->d_select.ptr, want);
-  if (e == cudaSuccess) {
-    ctx->d_select.bytes = want;
-    ctx->bytes += want;
-    e = cudaMallocHost(&ctx->h_select, want);
-  } else {
-    ctx->d_select.ptr = nullptr;
+  cudaError_t e = cudaSuccess;
+  if (ctx->d_select.bytes < bytes) {
+    free_select(ctx);
+    size_t want = size_t(1) << 20;
+    while (want < bytes) want *= 2;
+    e = cudaMalloc(&ctx->d_select.ptr, want);
+    if (e == cudaSuccess) {
+      ctx->d_select.bytes = want;
+      ctx->bytes += want;
+      ctx->uncharged += want;
+    } else {
+      ctx->d_select.ptr = nullptr;
+    }
   }
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->select_lo, cudaEventDisableTiming);
+  if (e == cudaSuccess && !ctx->h_select) e = cudaMallocHost(&ctx->h_select, kSelectPieces * kSelectPiece);
+  for (uint32_t i = 0; i < kSelectPieces && e == cudaSuccess; i++)
+    if (!ctx->select_piece[i]) e = cudaEventCreateWithFlags(&ctx->select_piece[i], cudaEventDisableTiming);
   if (e != cudaSuccess) {
     cudaGetLastError();
     free_select(ctx);
@@ -100,11 +104,34 @@ static int select_workspace(vgc_context *ctx, size_t bytes) {
   return VGC_OK;
 }
 
+// `bytes` of a select call's results from `src` to lo and, from byte `half` on, hi, through the pinned pieces: while
+// the host copies one piece out, the others are on their way.
+static cudaError_t select_results(vgc_context *ctx, const uint8_t *src, size_t half, uint8_t *lo, uint8_t *hi,
+                                  cudaStream_t st) {
+  const size_t bytes = 2 * half, pieces = (bytes + kSelectPiece - 1) / kSelectPiece;
+  const auto size = [&](size_t k) { return std::min(kSelectPiece, bytes - k * kSelectPiece); };
+  const auto issue = [&](size_t k) {
+    const cudaError_t e = cudaMemcpyAsync(ctx->h_select + k % kSelectPieces * kSelectPiece, src + k * kSelectPiece, size(k),
+                                          cudaMemcpyDeviceToHost, st);
+    return e != cudaSuccess ? e : cudaEventRecord(ctx->select_piece[k % kSelectPieces], st);
+  };
+  cudaError_t e = cudaSuccess;
+  for (size_t k = 0; k < pieces && k < kSelectPieces && e == cudaSuccess; k++) e = issue(k);
+  for (size_t k = 0; k < pieces && e == cudaSuccess; k++) {
+    if ((e = cudaEventSynchronize(ctx->select_piece[k % kSelectPieces])) != cudaSuccess) break;
+    const unsigned char *h = ctx->h_select + k % kSelectPieces * kSelectPiece;
+    const size_t a = k * kSelectPiece, b = a + size(k), cut = std::clamp(half, a, b);
+    if (cut > a) std::memcpy(lo + a, h, cut - a);
+    if (b > cut) std::memcpy(hi + (cut - half), h + (cut - a), b - cut);
+    if (k + kSelectPieces < pieces) e = issue(k + kSelectPieces);
+  }
+  return e;
+}
+
 int dev_alloc(vgc_context *ctx, DevBuf &b, size_t bytes) {
   if (b.bytes >= bytes && b.ptr) return VGC_OK;
   size_t want = std::max<size_t>(bytes, 256);
-  if (ctx->opts.hbm_budget_bytes && ctx->bytes - b.bytes + want > ctx->opts.hbm_budget_bytes) free_select(ctx);
-  if (ctx->opts.hbm_budget_bytes && ctx->bytes - b.bytes + want > ctx->opts.hbm_budget_bytes)
+  if (ctx->opts.hbm_budget_bytes && ctx->bytes - ctx->uncharged - b.bytes + want > ctx->opts.hbm_budget_bytes)
     return fail(VGC_OVER_BUDGET, "allocation of " + std::to_string(want) + " bytes exceeds the context's HBM budget");
   void *p = nullptr;
   cudaError_t e = cudaMalloc(&p, want);
@@ -319,13 +346,20 @@ int ensure_scratch(vgc_context *ctx, LaunchScratch &s, uint32_t views, size_t un
   // queue costs time, not correctness.
   const uint32_t want_chunks = std::max<uint32_t>(std::max<uint32_t>(kQueueMin, views * 65536u), s.queue_want);
   if (want_chunks > s.chunk_capacity) {
+    // what a launch of few views gets above 64k entries a view serves its small chunks and is not charged to the budget
+    const uint32_t charged = std::max<uint32_t>(std::max<uint32_t>(65536, views * 65536u), s.queue_want);
     if (s.d_chunks) {
       cudaFree(s.d_chunks);
       ctx->bytes -= (size_t)s.chunk_capacity * sizeof(uint4);
+      ctx->uncharged -= s.queue_uncharged;
     }
     s.d_chunks = nullptr;
+    s.queue_uncharged = 0;
+    s.chunk_capacity = 0;
     CUDA_TRY(cudaMalloc(&s.d_chunks, (size_t)want_chunks * sizeof(uint4)));
     ctx->bytes += (size_t)want_chunks * sizeof(uint4);
+    s.queue_uncharged = (size_t)(want_chunks - charged) * sizeof(uint4);
+    ctx->uncharged += s.queue_uncharged;
     s.chunk_capacity = want_chunks;
   }
   if (!s.done) CUDA_TRY(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
@@ -1005,6 +1039,9 @@ int vgc_context_destroy(vgc_context *ctx) {
   for (auto &h : ctx->hzb) dev_free(ctx, h.data);
   if (ctx->h_stats) cudaFreeHost(ctx->h_stats);
   free_select(ctx);
+  if (ctx->h_select) cudaFreeHost(ctx->h_select);
+  for (cudaEvent_t &ev : ctx->select_piece)
+    if (ev) cudaEventDestroy(ev);
   for (auto &p : ctx->prof_pending) {
     cudaEventDestroy(p.second.first);
     cudaEventDestroy(p.second.second);
@@ -1474,6 +1511,8 @@ int vgc_batch_destroy(vgc_batch *b) {
   if (b->scratch.d_views)
     b->ctx->bytes -= sizeof(ViewConst) * b->scratch.view_capacity + hzb_plan_bytes(b->scratch.view_capacity);
   if (b->scratch.d_units) b->ctx->bytes -= unit_bytes(b->scratch.unit_capacity);
+  b->ctx->bytes -= b->scratch.queue_uncharged;
+  b->ctx->uncharged -= b->scratch.queue_uncharged;
   free_scratch(b->scratch);
   delete b;
   return VGC_OK;
@@ -1567,15 +1606,14 @@ int vgc_select_cut(vgc_context *ctx, uint32_t slot, uint32_t count, const double
     p[i * 3 + 2] = (float)scale[i];
   }
   // Inputs, then lo, then hi in one device buffer; calls of ordinary size use the context's (kept, as cudaMalloc and
-  // cudaFree took most of such a call) and go through its pinned buffer: lo reaches the caller while hi is on its way.
+  // cudaFree took most of such a call) and its pinned pieces.
   const size_t outn = (size_t)count * mcount, in_bytes = ((m.size() + p.size()) * 4 + 255) & ~size_t(255);
   const size_t total = in_bytes + outn * 2;
   const bool kept = total <= kSelectKeep;
   void *d = nullptr;
-  unsigned char *h = nullptr;
   if (kept) {
     if ((rc = select_workspace(ctx, total))) return rc;
-    d = ctx->d_select.ptr, h = ctx->h_select;
+    d = ctx->d_select.ptr;
   } else {
     CUDA_TRY(cudaMalloc(&d, total));
   }
@@ -1583,26 +1621,21 @@ int vgc_select_cut(vgc_context *ctx, uint32_t slot, uint32_t count, const double
   uint8_t *dlo = (uint8_t *)d + in_bytes, *dhi = dlo + outn;
   cudaStream_t st = ctx->stream;
   cudaError_t e = cudaSuccess;
-  if (kept) {
-    std::memcpy(h, m.data(), m.size() * 4);
-    std::memcpy(h + m.size() * 4, p.data(), p.size() * 4);
-    e = cudaMemcpyAsync(d, h, (m.size() + p.size()) * 4, cudaMemcpyHostToDevice, st);
+  if (kept && in_bytes <= kSelectPieces * kSelectPiece) {
+    std::memcpy(ctx->h_select, m.data(), m.size() * 4);
+    std::memcpy(ctx->h_select + m.size() * 4, p.data(), p.size() * 4);
+    e = cudaMemcpyAsync(d, ctx->h_select, (m.size() + p.size()) * 4, cudaMemcpyHostToDevice, st);
   } else {
     e = cudaMemcpyAsync(dm, m.data(), m.size() * 4, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dp, p.data(), p.size() * 4, cudaMemcpyHostToDevice, st);
   }
   if (e == cudaSuccess)
     e = launch_select_cut(scene_of(ctx), slot, mcount, count, dm, dp, (float)threshold, (float)blend, dlo, dhi, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(kept ? h + in_bytes : lo, dlo, outn, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess && kept) e = cudaEventRecord(ctx->select_lo, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(kept ? h + in_bytes + outn : hi, dhi, outn, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess && kept) {
-    e = cudaEventSynchronize(ctx->select_lo);
-    if (e == cudaSuccess) std::memcpy(lo, h + in_bytes, outn);
-  }
+  if (e == cudaSuccess && kept) e = select_results(ctx, dlo, outn, lo, hi, st);
+  if (e == cudaSuccess && !kept) e = cudaMemcpyAsync(lo, dlo, outn, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess && !kept) e = cudaMemcpyAsync(hi, dhi, outn, cudaMemcpyDeviceToHost, st);
   const cudaError_t done = cudaStreamSynchronize(st);
   if (e == cudaSuccess) e = done;
-  if (e == cudaSuccess && kept) std::memcpy(hi, h + in_bytes + outn, outn);
   if (!kept) cudaFree(d);
   if (e != cudaSuccess) return fail(VGC_DEVICE_ERROR, std::string("select_cut: ") + cudaGetErrorString(e));
   return VGC_OK;

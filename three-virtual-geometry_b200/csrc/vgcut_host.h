@@ -47,6 +47,7 @@ struct HzbSlot {
   bool valid = false;
 };
 
+constexpr uint32_t kSelectPieces = 4;   // pinned pieces a selectCut's results come back through
 constexpr uint32_t kQueueMin = 262144;  // entries of the smallest meshlet work queue
 
 inline uint32_t pad32(uint32_t x) { return (x + 31u) & ~31u; }
@@ -68,6 +69,7 @@ struct LaunchScratch {
   uint32_t *d_unit_count = nullptr;  // control words (see launch_reset)
   uint4 *d_chunks = nullptr;      // meshlet work queue (spans and chunks)
   uint32_t chunk_capacity = 0;    // its entries
+  size_t queue_uncharged = 0;     // bytes of it that the owner's HBM budget does not count
   uint32_t queue_want = 0;        // entries the last launch sequence asked for (grown to before the next one)
   uint32_t *h_ctl = nullptr;      // pinned: control words 6 and 7 at the end of the last launch sequence
   uint32_t grid_instances = 0;    // persistent grids of k_instances / k_chunks (0: the context's occupancy defaults)
@@ -105,6 +107,7 @@ struct vgc_context {
   uint32_t chunk_grid = 0;   // persistent grid of k_chunks
   uint32_t hzb_grid = 0;     // persistent grid of k_hzb_stream (0: the per-view tile kernel instead)
   uint64_t bytes = 0;
+  uint64_t uncharged = 0;  // of `bytes`: workspaces that the HBM budget does not count
   std::mutex mu;
   // host mirrors of the resident scene
   std::vector<MeshHost> mesh_host;
@@ -126,9 +129,9 @@ struct vgc_context {
   DevBuf d_meshes, d_levels, d_m_lod, d_m_parent, d_m_err, d_m_cull, d_m_info, d_m_tris, d_inst, d_inst_slot, d_cells;
   DevBuf d_lsamples, d_positions, d_m_verts;
   DevBuf d_raster;  // occluder depth pass: the tile pass's work lists
-  DevBuf d_select;  // selectCut workspace (kept while small), its pinned counterpart, and lo's arrival in it
+  DevBuf d_select;  // selectCut workspace (kept while small), the pinned pieces of its results and their arrivals
   unsigned char *h_select = nullptr;
-  cudaEvent_t select_lo = nullptr;
+  cudaEvent_t select_piece[kSelectPieces] = {};
   DevBuf d_resort;  // instance re-sort: centres, keys, permutation scratch (grows only)
   // output slots
   uint32_t out_slots = 0;
