@@ -23,7 +23,7 @@
 //    of their bounding box, a warp per tile. The second kernel spreads both over the whole grid: a meshlet close to
 //    the camera, with a hundred triangles of a few hundred pixels each, would otherwise keep one warp drawing long
 //    after the rest have finished. When a queue is full its triangles are drawn by the warp that set them up.
-//    16 two-pass images of 960x540 (steady state): occluder kernel 650 -> 275 us, queue kernel 215 -> 272 us;
+//    16 two-pass images of 960x540 (steady state): occluder kernel 650 -> 275 us, queue kernel 215 -> 250 us;
 //  * the atomics' results are unused, so they do not wait (a load-then-atomic early depth test measured slower: it
 //    puts an L2 round trip on every pixel). The image is the minimum over all drawn pixels, whatever the order.
 //
@@ -213,12 +213,19 @@ __device__ __forceinline__ ScreenTri read_record(const float4 *r, uint32_t &tx, 
   return t;
 }
 
+// q / w of a small triangle's pixel q < 128 and width w <= 128 as q * inv >> 15, inv = floor(2^15 / w) + 1 (an
+// approximate quotient may give one more): 0 < inv w - 2^15 <= 2 w, so q (inv w - 2^15) < 2^15 and the result is exact
+constexpr uint32_t kInvShift = 15;
+
 // The whole warp over t's bounding box, 32 consecutive pixels (row-major) per step.
 template <bool VIS>
 __device__ __forceinline__ void warp_draw(const RasterArgs &R, const ScreenTri &t, const TriTag &g, uint32_t lane) {
   const uint32_t bw = uint32_t(t.x1 - t.x0 + 1), count = bw * uint32_t(t.y1 - t.y0 + 1);
-  const uint32_t q = 32 / bw, r = 32 % bw;  // a step of 32 pixels: q rows and r columns
-  uint32_t x = lane % bw, y = lane / bw;
+  // a step of 32 pixels: q rows and r columns. The quotients of 32 and of the lane as at kInvShift, exact for every
+  // width: up to 511, 32 * 2 bw < 2^15; above, inv <= 66 and both quotients are 0
+  const uint32_t inv = uint32_t(__fdividef(float(1u << kInvShift), float(bw))) + 1u;
+  const uint32_t q = (32u * inv) >> kInvShift, r = 32u - q * bw;
+  uint32_t y = (lane * inv) >> kInvShift, x = lane - y * bw;
   for (uint32_t i = lane; i < count; i += 32) {
     shade_pixel<VIS>(R, t, g, t.x0 + int(x), t.y0 + int(y));
     x += r, y += q;
@@ -245,9 +252,6 @@ struct TriRing {
   uint2 d[kRing];   // lo | hi << 8, id
   uint8_t order[32];
 };
-// q / w of a small triangle's pixel q < 128 and width w <= 128 as q * inv >> 15, inv = floor(2^15 / w) + 1 (an
-// approximate quotient may give one more): 0 < inv w - 2^15 <= 2 w, so q (inv w - 2^15) < 2^15 and the result is exact
-constexpr uint32_t kInvShift = 15;
 static_assert(kLaneRasterMax <= 128, "the packed division covers boxes of 128 pixels");
 
 __device__ __forceinline__ ScreenTri ring_triangle(const TriRing &ring, uint32_t j, TriTag &g, uint32_t &meta,
@@ -595,17 +599,16 @@ __global__ void __launch_bounds__(128) k_raster_queued(const __grid_constant__ R
   const uint32_t n_medium = most * kSubQueues;
   const uint32_t n = n_medium + (uint32_t)min(*reinterpret_cast<const unsigned long long *>(R.ctl + 2),
                                               (unsigned long long)kTileUnits);
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += warps) {
-    uint32_t tx;
-    TriTag g;
-    if (u < n_medium) {
-      if (u / kSubQueues < counts[u % kSubQueues]) {
-        const ScreenTri t = read_record(R.medium + (size_t)u * kRecord, tx, g);
-        warp_draw<VIS>(R, t, g, lane);
-      }
-      continue;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5, mine = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  uint32_t tx;
+  TriTag g;
+  uint32_t u = mine;
+  for (; u < n_medium; u += warps)
+    if (u / kSubQueues < counts[u % kSubQueues]) {
+      const ScreenTri t = read_record(R.medium + (size_t)u * kRecord, tx, g);
+      warp_draw<VIS>(R, t, g, lane);
     }
+  for (; u < n; u += warps) {
     const uint2 tile = R.tiles[u - n_medium];
     if (tile.x == kNoTri) continue;
     const ScreenTri t = read_record(R.large + (size_t)tile.x * kRecord, tx, g);
