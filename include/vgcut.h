@@ -162,8 +162,9 @@ enum {
 };
 /* Device-side failures a kernel reports instead of waiting on: VGC_FAULT_HZB_WAIT = a tile copy of the HZB
  * build did not arrive within about a second (the launch's HZBs are incomplete; its cuts may keep occluded geometry
- * or drop visible geometry). */
-enum { VGC_FAULT_HZB_WAIT = 1 };
+ * or drop visible geometry); VGC_FAULT_RETRY_WAIT = a piece of a retry round (a cut that overflowed its capacity,
+ * redone at a coarser threshold) did not complete within about a second (the view's cut is incomplete). */
+enum { VGC_FAULT_HZB_WAIT = 1, VGC_FAULT_RETRY_WAIT = 2 };
 enum { VGC_CUT_SELECTED = 0, VGC_CUT_DRAWN = 1, VGC_CUT_SURVIVED = 2, VGC_CUT_WORK = 3, VGC_CUT_REQUESTED = 4 };
 
 /* Stats of one output slot: VirtualGeometryStats (VirtualGeometry.ts:24-47) per view. */

@@ -340,7 +340,7 @@ int ensure_scratch(vgc_context *ctx, LaunchScratch &s, uint32_t views, size_t un
     ctx->bytes += unit_bytes(n);
     s.unit_capacity = n;
   }
-  if (!s.d_unit_count) CUDA_TRY(cudaMalloc(&s.d_unit_count, 64));
+  if (!s.d_unit_count) CUDA_TRY(cudaMalloc(&s.d_unit_count, kLaunchCtlWords * 4));
   // meshlet work queue: about one span per instance with a level range and cut, one chunk per 512 meshlets of a
   // warp's items (fewer in a launch of few views: pass_shape). Sized for 64k entries per view, 256k at least; a warp that cannot reserve tests its items itself, so a full
   // queue costs time, not correctness.
@@ -698,7 +698,7 @@ cudaError_t timed(vgc_context *ctx, bool capture, int kind, cudaStream_t st, F &
   return e;
 }
 
-// The launch sequence of one frame: reset, cells, then select + finish for the first round and two retry rounds
+// The launch sequence of one frame: reset, cells, then select + finish for the first round, and the two retry rounds
 // (GeometryPool.ts:1081-1092 without the dispatch-argument kernels, which persistent launches do not need).
 int prepare_multi(vgc_context *const *ctxs, uint32_t nctx, LaunchScratch &s, const vgc_view *views,
                   const uint32_t *scene, uint32_t count, const uint32_t *slots) {
@@ -806,38 +806,40 @@ int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st,
   lim.fine_units = select_grid * 4 / 2;  // fewer half-units than warps
   if (s.any_budget) {  // the triangleBudget search: histogram pass, then the threshold of each budget view
     CUDA_TRY(timed(ctx, capture, VGC_KERNEL_BUDGET, st, [&] {
-      cudaError_t e = launch_instances(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, -1,
+      cudaError_t e = launch_instances(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, true,
                                        select_grid, s.d_overflow, st, lim, plain);
       plain = s.shared;
       if (e == cudaSuccess)
-        e = launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, -1, chunk_grid, st,
+        e = launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, true, chunk_grid, st,
                           s.shared);
       if (e == cudaSuccess)
-        e = launch_instances_redo(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, -1,
+        e = launch_instances_redo(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, true,
                                   s.d_overflow, redo_grid, st, lim, s.shared);
       if (e == cudaSuccess) e = launch_budget(s.d_views, count, s.d_unit_count, st, s.shared);
       return e;
     }));
   }
-  for (int round = 0; round < 3; round++) {
-    if (round > 0 && kChunkShiftRetry) lim.chunk_max = kChunkShiftRetry, lim.chunk_min = std::min(lim.chunk_min, kChunkShiftRetry);
-    CUDA_TRY(timed(ctx, capture, round == 0 ? VGC_KERNEL_SELECT0 : VGC_KERNEL_SELECT_RETRY, st, [&] {
-      return launch_instances(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, round,
-                              select_grid, s.d_overflow, st, lim, round == 0 ? plain : s.shared);
-    }));
-    CUDA_TRY(timed(ctx, capture, round == 0 ? VGC_KERNEL_CHUNKS0 : VGC_KERNEL_SELECT_RETRY, st, [&] {
-      return launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, round, chunk_grid, st,
-                           s.shared);
-    }));
-    // units whose items did not fit the queue (returns at once when there are none)
-    CUDA_TRY(timed(ctx, capture, VGC_KERNEL_SELECT_RETRY, st, [&] {
-      return launch_instances_redo(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity,
-                                   round, s.d_overflow, redo_grid, st, lim, s.shared);
-    }));
-    CUDA_TRY(timed(ctx, capture, VGC_KERNEL_FINISH, st, [&] {
-      return launch_finish(s.d_views, count, s.d_unit_count, round, s.h_ctl, st, s.shared);
-    }));
-  }
+  CUDA_TRY(timed(ctx, capture, VGC_KERNEL_SELECT0, st, [&] {
+    return launch_instances(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, false,
+                            select_grid, s.d_overflow, st, lim, plain);
+  }));
+  CUDA_TRY(timed(ctx, capture, VGC_KERNEL_CHUNKS0, st, [&] {
+    return launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, false, chunk_grid, st,
+                         s.shared);
+  }));
+  // units whose items did not fit the queue (returns at once when there are none)
+  CUDA_TRY(timed(ctx, capture, VGC_KERNEL_SELECT_RETRY, st, [&] {
+    return launch_instances_redo(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, false,
+                                 s.d_overflow, redo_grid, st, lim, s.shared);
+  }));
+  CUDA_TRY(timed(ctx, capture, VGC_KERNEL_FINISH, st,
+                 [&] { return launch_finish(s.d_views, count, s.d_unit_count, s.h_ctl, st, s.shared); }));
+  // rounds 1 and 2
+  if (kChunkShiftRetry) lim.chunk_max = kChunkShiftRetry, lim.chunk_min = std::min(lim.chunk_min, kChunkShiftRetry);
+  CUDA_TRY(timed(ctx, capture, VGC_KERNEL_SELECT_RETRY, st, [&] {
+    return launch_retry(S, scenes, s.d_views, count, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity,
+                        s.d_overflow, s.h_ctl, (uint32_t)ctx->sm_count * kRetryBlocks, st, lim, s.shared);
+  }));
   return VGC_OK;
 }
 
@@ -1701,7 +1703,7 @@ int vgc_debug_scene(const vgc_context *ctx, float *cells, uint32_t cell_capacity
 // queue - lives in this fixed file-scope device array instead of the context's launch scratch. Every GPU that loads
 // the library holds the array until the process exits.
 namespace {
-constexpr size_t kNoAllocCtl = 0;                                   // 16 control words
+constexpr size_t kNoAllocCtl = 0;                                   // kLaunchCtlWords control words
 constexpr size_t kNoAllocView = 256;                                // one ViewConst
 constexpr uint32_t kNoAllocMaxUnits = 65536;                        // visible (view, cell) units: cells of the scene
 constexpr uint32_t kNoAllocMaxChunks = 65536;                       // meshlet work queue entries (beyond: tested in place)
@@ -1710,6 +1712,7 @@ constexpr size_t kNoAllocChunks = kNoAllocUnits + (size_t)kNoAllocMaxUnits * siz
 constexpr size_t kNoAllocOverflow = kNoAllocChunks + (size_t)kNoAllocMaxChunks * sizeof(uint4);
 constexpr size_t kNoAllocBytes = kNoAllocOverflow + (size_t)kNoAllocMaxUnits * 4 / 32 * sizeof(uint32_t);  // 1.53 MiB
 static_assert(sizeof(ViewConst) <= kNoAllocUnits - kNoAllocView, "view constants must fit their scratch slot");
+static_assert(kLaunchCtlWords * 4 <= kNoAllocView, "control words must fit before the view");
 static_assert(kNoAllocChunks % 256 == 0, "chunk queue must stay 256-byte aligned");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -1803,20 +1806,20 @@ extern "C" int vgc_cut_noalloc(vgc_context *ctx, const vgc_view *view, uint32_t 
   CUDA_TRY(launch_reset(LaunchInputs(), d_view, 1, ctl, st));
   CUDA_TRY(launch_cells(S, nullptr, d_view, 1, cells, units, ctl, st));
   if (view->triangle_budget > 0) {
-    CUDA_TRY(launch_instances(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, -1, ctx->select_grid, overflow,
+    CUDA_TRY(launch_instances(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, true, ctx->select_grid, overflow,
                               st));
-    CUDA_TRY(launch_chunks(S, nullptr, d_view, chunks, ctl, kNoAllocMaxChunks, -1, ctx->chunk_grid, st));
-    CUDA_TRY(launch_instances_redo(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, -1, overflow, redo_grid,
+    CUDA_TRY(launch_chunks(S, nullptr, d_view, chunks, ctl, kNoAllocMaxChunks, true, ctx->chunk_grid, st));
+    CUDA_TRY(launch_instances_redo(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, true, overflow, redo_grid,
                                    st));
     CUDA_TRY(launch_budget(d_view, 1, ctl, st));
   }
-  for (int round = 0; round < 3; round++) {
-    CUDA_TRY(launch_instances(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, round, ctx->select_grid,
-                              overflow, st));
-    CUDA_TRY(launch_chunks(S, nullptr, d_view, chunks, ctl, kNoAllocMaxChunks, round, ctx->chunk_grid, st));
-    CUDA_TRY(launch_instances_redo(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, round, overflow,
-                                   redo_grid, st));
-    CUDA_TRY(launch_finish(d_view, 1, ctl, round, nullptr, st));
-  }
+  CUDA_TRY(launch_instances(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, false, ctx->select_grid, overflow,
+                            st));
+  CUDA_TRY(launch_chunks(S, nullptr, d_view, chunks, ctl, kNoAllocMaxChunks, false, ctx->chunk_grid, st));
+  CUDA_TRY(launch_instances_redo(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, false, overflow, redo_grid,
+                                 st));
+  CUDA_TRY(launch_finish(d_view, 1, ctl, nullptr, st));
+  CUDA_TRY(launch_retry(S, nullptr, d_view, 1, units, ctl, chunks, kNoAllocMaxChunks, overflow, nullptr,
+                        (uint32_t)ctx->sm_count * kRetryBlocks, st));
   return VGC_OK;
 }

@@ -3,15 +3,16 @@
 // Pass structure for a batch of views (all views of one scene in each launch):
 //   k_cells    one thread per (view, cell): the cell tests of GeometryPool.ts:728-760; surviving (view, cell)
 //              units are compacted with one atomic per warp (__ballot_sync / __popc).
-//   k_instances one warp per 32 instances of a visible unit: the instance tests (GeometryPool.ts:846-913) and the
+//   k_instances one warp per 64 (or 32) instances of a visible unit: the instance tests (GeometryPool.ts:846-913) and the
 //              LOD level range (selectLevels :771-843). Fast-path instances emit their meshlets with warp-aggregated
-//              atomics; the others queue their range as chunks of <= 256 meshlets (one warp-wide reservation).
+//              atomics; the others queue their range as chunks of 32 to 512 meshlets (one warp-wide reservation).
 //   k_chunks   one warp per chunk: the meshlet tests (GeometryPool.ts:916-970), reading the struct-of-arrays
 //              bounds coalesced; drawn meshlets are staged per warp and placed with one atomic per cut and part.
 //   k_finish   one warp per view: the prefix pass (GeometryPool.ts:973-995) as a warp scan over mesh slots, the
-//              capacity check that schedules a retry round (:1032-1054), and after the last round the steer (:1056-1069).
+//              capacity check that schedules a retry round (:1032-1054), and for a settled view the steer (:1056-1069).
+//   k_retry    the retry rounds: the passes above again for the cuts that overflowed.
 //   k_expand   one warp per drawn meshlet: index expansion (GeometryPool.ts:998-1021).
-//   k_hzb_*    HZB mip chain (OcclusionCulling.ts:302-350): 32x32 tiles reduce five levels in shared memory, one
+//   k_hzb_*    HZB mip chain (OcclusionCulling.ts:302-350): strips or tiles reduce the large levels in registers, one
 //              block finishes the small top levels.
 //
 // Arithmetic: this file is compiled with -fmad=false and IEEE division / square root, so every decision
@@ -35,6 +36,13 @@ namespace vgc {
 __device__ __forceinline__ void wait_previous_kernel() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+constexpr uint64_t kWaitLimitNs = 1000000000ull;  // after which a wait of a kernel gives up
+__device__ __forceinline__ uint64_t global_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
 }
 
 __device__ __forceinline__ float fmn(float a, float b) { return a < b ? a : b; }
@@ -312,9 +320,9 @@ __device__ __forceinline__ unsigned long long *queue_counter(uint32_t *ctl) {
 // queue.
 constexpr uint32_t kCtlNextChunk = 8, kCtlNextUnit = 9;
 constexpr uint32_t kCtlOverflowed = 10, kCtlNextRedo = 11;  // a unit's items did not fit the queue; k_instances_redo's counter
-__device__ __forceinline__ uint32_t warp_grab(uint32_t *ctl, uint32_t word) {
+__device__ __forceinline__ uint32_t warp_grab(uint32_t *counter) {
   uint32_t i = 0;
-  if ((threadIdx.x & 31) == 0) i = atomicAdd(ctl + word, 1u);
+  if ((threadIdx.x & 31) == 0) i = atomicAdd(counter, 1u);
   return __shfl_sync(0xffffffffu, i, 0);
 }
 
@@ -1090,53 +1098,60 @@ __global__ void __launch_bounds__(128, MULTI ? 6 : 8) k_instances(Scene S0, cons
                                                    const ViewConst *__restrict__ views,
                                                    const HzbDesc *__restrict__ hzbs0, const uint2 *__restrict__ units,
                                                    uint32_t *__restrict__ ctl, uint4 *__restrict__ queue,
-                                                   uint32_t capacity, int round, PassLimits lim,
+                                                   uint32_t capacity, PassLimits lim,
                                                    uint32_t *__restrict__ overflow) {
   __shared__ Survivor lists[4][kHalfUnit];
   wait_previous_kernel();
-  if (round > 0 && ctl[round] == 0) return;  // no view redoes a cut in this round
   const PassShape shape = pass_shape(ctl, lim);
   const uint32_t work = ctl[0] * (shape.fine ? 4 : 2);
   WarpFeed feed;
   feed.start(ctl + kCtlNextUnit);
   for (uint32_t w = feed.i; w < work; w = feed.next()) {
-    instance_unit<HIST, MULTI, false>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, round, shape, overflow, nullptr,
+    instance_unit<HIST, MULTI, false>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, 0, shape, overflow, nullptr,
                                        lists[threadIdx.x >> 5], w, 0);
     __syncwarp();  // the survivor list is rewritten by the next half-unit
   }
 }
 
-// The survivor passes k_instances found the chunk queue full for (bits of `overflow`: bit 2 w + p for pass p of
-// half-unit w, cleared here), their items tested in place by the whole warp. Launched after each pass's k_chunks;
-// returns at once when nothing overflowed.
+// The survivor passes k_instances found the chunk queue full for (bits of word i of `overflow`: bit 2 w + p for pass p
+// of half-unit w, cleared here), their items tested in place by the whole warp.
+template <bool HIST, bool MULTI>
+__device__ __forceinline__ void redo_word(const Scene &S0, const Scene *__restrict__ scenes,
+                                          const ViewConst *__restrict__ views, const HzbDesc *__restrict__ hzbs0,
+                                          const uint2 *__restrict__ units, uint32_t *__restrict__ ctl,
+                                          uint4 *__restrict__ queue, uint32_t capacity, int round,
+                                          const PassShape &shape, uint32_t *__restrict__ overflow, WarpStage *ws,
+                                          Survivor *__restrict__ list, uint32_t i) {
+  uint32_t bits = overflow[i];
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0 && bits) overflow[i] = 0;
+  while (bits) {
+    const uint32_t b = __ffs(bits) - 1;
+    bits &= bits - 1;
+    const uint32_t bit = i * 32 + b;
+    instance_unit<HIST, MULTI, true>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, round, shape, overflow, ws,
+                                     list, shape.fine ? bit : bit >> 1, shape.fine ? 0u : bit & 1u);
+    __syncwarp();
+  }
+}
+
+// Launched after each pass's k_chunks; returns at once when nothing overflowed.
 template <bool HIST, bool MULTI>
 __global__ void __launch_bounds__(128, 4) k_instances_redo(Scene S0, const Scene *__restrict__ scenes,
                                                             const ViewConst *__restrict__ views,
                                                             const HzbDesc *__restrict__ hzbs0,
                                                             const uint2 *__restrict__ units, uint32_t *__restrict__ ctl,
-                                                            uint4 *__restrict__ queue, uint32_t capacity, int round,
+                                                            uint4 *__restrict__ queue, uint32_t capacity,
                                                             PassLimits lim, uint32_t *__restrict__ overflow) {
   __shared__ WarpStage stage[4];
   __shared__ Survivor lists[4][kHalfUnit];
   wait_previous_kernel();
-  if (round > 0 && ctl[round] == 0) return;
   if (ctl[kCtlOverflowed] == 0) return;
   const PassShape shape = pass_shape(ctl, lim);
   const uint32_t words = (ctl[0] * 4 + 31) / 32;
-  for (uint32_t i = warp_grab(ctl, kCtlNextRedo); i < words; i = warp_grab(ctl, kCtlNextRedo)) {
-    uint32_t bits = overflow[i];
-    __syncwarp();
-    if ((threadIdx.x & 31) == 0 && bits) overflow[i] = 0;
-    while (bits) {
-      const uint32_t b = __ffs(bits) - 1;
-      bits &= bits - 1;
-      const uint32_t bit = i * 32 + b;
-      instance_unit<HIST, MULTI, true>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, round, shape, overflow,
-                                       &stage[threadIdx.x >> 5], lists[threadIdx.x >> 5], shape.fine ? bit : bit >> 1,
-                                       shape.fine ? 0u : bit & 1u);
-      __syncwarp();
-    }
-  }
+  for (uint32_t i = warp_grab(ctl + kCtlNextRedo); i < words; i = warp_grab(ctl + kCtlNextRedo))
+    redo_word<HIST, MULTI>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, 0, shape, overflow,
+                           &stage[threadIdx.x >> 5], lists[threadIdx.x >> 5], i);
 }
 
 // ------------------------------------------------------------------------------------------------ k_chunks
@@ -1146,133 +1161,136 @@ __global__ void __launch_bounds__(128, 4) k_instances_redo(Scene S0, const Scene
 // meshlets that pass queue up and finish 32 at a time (drain_queue). One draw-list flush per chunk.
 // HIST: the budget histogram of the chunks the budget pass queued.
 template <bool HIST, bool MULTI>
+__device__ __forceinline__ void chunk_work(const Scene &S0, const Scene *__restrict__ scenes,
+                                           const ViewConst *__restrict__ views, const HzbDesc *__restrict__ hzbs0,
+                                           const WorkQueue &Q, const uint4 ch, WarpStage &ws, LodQueue &q, SpanFrame &F,
+                                           BudgetWork<HIST> &bw, uint32_t &hist_view, uint32_t &hist_chunks) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t ns = ch.z >> 8;
+  if (ns == 0) return;
+  const ViewConst &V = views[ch.x];
+  const auto &S = SceneOf<MULTI>::get(S0, scenes, V);
+  const HzbDesc *__restrict__ hzbs = SceneOf<MULTI>::hzbs(hzbs0, S);
+  const CellRec cell = S.cells[ch.y];
+  const uint32_t cut = ch.z & 1u;
+  const bool occl_on = (ch.z & 2u) != 0;
+  const ViewBands b = bands_of(V);
+  const float low = cut ? b.low1 : b.low0, high = cut ? b.high1 : b.high0;
+  const float inv_low = 1.0f / low;
+  if constexpr (HIST) {
+    if (ch.x != hist_view || ++hist_chunks == kBudgetFlush) {
+      if (hist_view != ~0u) budget_flush(bw, views[hist_view].hist);
+      if (ch.x != hist_view) budget_begin(bw, V, get_state(V.state, 0));
+      hist_view = ch.x;
+      hist_chunks = 0;
+    }
+  }
+  // spans: one lane each, laid end to end from position 0
+  uint4 sp = make_uint4(0u, 0u, 0u, 0u);
+  if (lane < ns) sp = Q.spans[ch.w + lane];
+  const uint32_t sp_off = warp_scan_incl(sp.z) - sp.z;
+  const uint32_t total = __shfl_sync(0xffffffffu, sp_off + sp.z, 31);
+  if (lane < ns) {
+    const uint32_t instance = cell.first + (sp.x & 127u);
+    float VM[13];
+    model_view(V.V, S.inst + (size_t)instance * 4, VM, VM[12]);
+    F.vm[lane][0] = make_float4(VM[0], VM[1], VM[2], VM[3]);
+    F.vm[lane][1] = make_float4(VM[4], VM[5], VM[6], VM[7]);
+    F.vm[lane][2] = make_float4(VM[8], VM[9], VM[10], VM[11]);
+    F.vm[lane][3] = make_float4(VM[12], __uint_as_float(instance), __uint_as_float((sp.x >> 7) & 1u),
+                                __uint_as_float(sp.y - sp_off));
+  }
+  __syncwarp();
+  WarpCount wc{0, 0, 0};
+  uint32_t qn = 0;       // warp-uniform
+  uint32_t started = 0;  // warp-uniform: spans starting before this step's first position
+  const uint32_t lanes_le = (2u << lane) - 1u;
+  for (uint32_t base = 0; base < total; base += 32) {
+    const uint32_t p = base + lane;
+    // span of position p: the last span starting at or before it (spans are non-empty and in order, so each step
+    // holds a bit per span starting in it)
+    const uint32_t rel = sp_off - base;
+    const uint32_t starts = __reduce_or_sync(0xffffffffu, lane < ns && rel < 32u ? 1u << rel : 0u);
+    const uint32_t j = started + __popc(starts & lanes_le) - 1u;
+    started += __popc(starts);
+    bool pass = false;
+    float own = 0.0f, parent = 0.0f;
+    uint32_t m = 0;
+    if (p < total) {
+      float VM[13];
+      uint32_t inst;
+      bool inside;
+      m = p + frame_vm(F, j, VM, inst, inside);
+      const float4 ls = __ldg(S.m_lod + m), ps = __ldg(S.m_parent + m);
+      const float2 er = __ldg(reinterpret_cast<const float2 *>(S.m_err + m));
+      const ProjErr po = proj_parts(V, VM, VM[12], ls, er.x), pp = proj_parts(V, VM, VM[12], ps, er.y);
+      if constexpr (HIST) {
+        const uint32_t bo = first_bin([&](uint32_t k) { return err_le(po, er.x, bw.high[k]); });
+        const uint32_t bp = first_bin([&](uint32_t k) { return err_le(pp, er.y, bw.e[k]); });
+        pass = bo < bp;
+        own = __uint_as_float(bo);
+        parent = __uint_as_float(bp);
+      } else {
+        pass = err_le(po, er.x, high) && err_gt(pp, er.y, low);
+        own = po.dist;
+        parent = pp.dist;
+      }
+    }
+    const uint32_t mask = __ballot_sync(0xffffffffu, pass);
+    if (pass) {
+      const uint32_t at = qn + __popc(mask & ((1u << lane) - 1u));
+      q.pos[at] = m;
+      q.span[at] = j;
+      q.own[at] = own;
+      q.parent[at] = parent;
+    }
+    qn += __popc(mask);
+    __syncwarp();
+    if (qn >= 32) {
+      drain_queue<HIST>(S, V, hzbs, q, F, 32, ws, wc, inv_low, b.fade_scale, b.high0, cut, occl_on, cell.slot,
+                        bw);
+      qn -= 32;
+      __syncwarp();
+      if (lane < qn) {
+        q.pos[lane] = q.pos[32 + lane];
+        q.span[lane] = q.span[32 + lane];
+        q.own[lane] = q.own[32 + lane];
+        q.parent[lane] = q.parent[32 + lane];
+      }
+      __syncwarp();
+    }
+  }
+  if (qn)
+    drain_queue<HIST>(S, V, hzbs, q, F, qn, ws, wc, inv_low, b.fade_scale, b.high0, cut, occl_on, cell.slot, bw);
+  __syncwarp();
+  if (!HIST) warp_flush(ws, wc, V, S.slot_capacity, cell.slot, cut);
+  __syncwarp();  // the frame and queue are rewritten by the next chunk
+}
+
+template <bool HIST, bool MULTI>
 __global__ void __launch_bounds__(128, MULTI || HIST ? 6 : 8) k_chunks(Scene S0, const Scene *__restrict__ scenes,
                                                             const ViewConst *__restrict__ views,
                                                             const HzbDesc *__restrict__ hzbs0,
                                                             uint4 *__restrict__ queue, uint32_t *__restrict__ ctl,
-                                                            uint32_t capacity, int round) {
+                                                            uint32_t capacity) {
   __shared__ WarpStage stage[4];
   __shared__ LodQueue queues[4];
   __shared__ SpanFrame frames[4];
   __shared__ BudgetWork<HIST> budgets[4];
   BudgetWork<HIST> &bw = budgets[threadIdx.x >> 5];
-  WarpStage &ws = stage[threadIdx.x >> 5];
-  LodQueue &q = queues[threadIdx.x >> 5];
-  SpanFrame &F = frames[threadIdx.x >> 5];
   wait_previous_kernel();
-  if (round > 0 && ctl[round] == 0) return;  // no view redoes a cut in this round
   const WorkQueue Q = work_queue(queue, capacity);
   const uint32_t n_chunks = min(uint32_t(*queue_counter(ctl) >> 32), Q.chunk_cap);
-  const uint32_t lane = threadIdx.x & 31;
   uint32_t hist_view = ~0u, hist_chunks = 0;  // HIST: the view the warp's histogram belongs to
   if constexpr (HIST) {
-    for (uint32_t i = lane; i < 2 * kBudgetBins; i += 32) bw.hist[i] = 0;
+    for (uint32_t i = threadIdx.x & 31; i < 2 * kBudgetBins; i += 32) bw.hist[i] = 0;
     __syncwarp();
   }
   WarpFeed feed;
   feed.start(ctl + kCtlNextChunk);
-  for (uint32_t c = feed.i; c < n_chunks; c = feed.next()) {
-    const uint4 ch = Q.chunks[c];
-    const uint32_t ns = ch.z >> 8;
-    if (ns == 0) continue;
-    const ViewConst &V = views[ch.x];
-    const auto &S = SceneOf<MULTI>::get(S0, scenes, V);
-    const HzbDesc *__restrict__ hzbs = SceneOf<MULTI>::hzbs(hzbs0, S);
-    const CellRec cell = S.cells[ch.y];
-    const uint32_t cut = ch.z & 1u;
-    const bool occl_on = (ch.z & 2u) != 0;
-    const ViewBands b = bands_of(V);
-    const float low = cut ? b.low1 : b.low0, high = cut ? b.high1 : b.high0;
-    const float inv_low = 1.0f / low;
-    if constexpr (HIST) {
-      if (ch.x != hist_view || ++hist_chunks == kBudgetFlush) {
-        if (hist_view != ~0u) budget_flush(bw, views[hist_view].hist);
-        if (ch.x != hist_view) budget_begin(bw, V, get_state(V.state, 0));
-        hist_view = ch.x;
-        hist_chunks = 0;
-      }
-    }
-    // spans: one lane each, laid end to end from position 0
-    uint4 sp = make_uint4(0u, 0u, 0u, 0u);
-    if (lane < ns) sp = Q.spans[ch.w + lane];
-    const uint32_t sp_off = warp_scan_incl(sp.z) - sp.z;
-    const uint32_t total = __shfl_sync(0xffffffffu, sp_off + sp.z, 31);
-    if (lane < ns) {
-      const uint32_t instance = cell.first + (sp.x & 127u);
-      float VM[13];
-      model_view(V.V, S.inst + (size_t)instance * 4, VM, VM[12]);
-      F.vm[lane][0] = make_float4(VM[0], VM[1], VM[2], VM[3]);
-      F.vm[lane][1] = make_float4(VM[4], VM[5], VM[6], VM[7]);
-      F.vm[lane][2] = make_float4(VM[8], VM[9], VM[10], VM[11]);
-      F.vm[lane][3] = make_float4(VM[12], __uint_as_float(instance), __uint_as_float((sp.x >> 7) & 1u),
-                                  __uint_as_float(sp.y - sp_off));
-    }
-    __syncwarp();
-    WarpCount wc{0, 0, 0};
-    uint32_t qn = 0;       // warp-uniform
-    uint32_t started = 0;  // warp-uniform: spans starting before this step's first position
-    const uint32_t lanes_le = (2u << lane) - 1u;
-    for (uint32_t base = 0; base < total; base += 32) {
-      const uint32_t p = base + lane;
-      // span of position p: the last span starting at or before it (spans are non-empty and in order, so each step
-      // holds a bit per span starting in it)
-      const uint32_t rel = sp_off - base;
-      const uint32_t starts = __reduce_or_sync(0xffffffffu, lane < ns && rel < 32u ? 1u << rel : 0u);
-      const uint32_t j = started + __popc(starts & lanes_le) - 1u;
-      started += __popc(starts);
-      bool pass = false;
-      float own = 0.0f, parent = 0.0f;
-      uint32_t m = 0;
-      if (p < total) {
-        float VM[13];
-        uint32_t inst;
-        bool inside;
-        m = p + frame_vm(F, j, VM, inst, inside);
-        const float4 ls = __ldg(S.m_lod + m), ps = __ldg(S.m_parent + m);
-        const float2 er = __ldg(reinterpret_cast<const float2 *>(S.m_err + m));
-        const ProjErr po = proj_parts(V, VM, VM[12], ls, er.x), pp = proj_parts(V, VM, VM[12], ps, er.y);
-        if constexpr (HIST) {
-          const uint32_t bo = first_bin([&](uint32_t k) { return err_le(po, er.x, bw.high[k]); });
-          const uint32_t bp = first_bin([&](uint32_t k) { return err_le(pp, er.y, bw.e[k]); });
-          pass = bo < bp;
-          own = __uint_as_float(bo);
-          parent = __uint_as_float(bp);
-        } else {
-          pass = err_le(po, er.x, high) && err_gt(pp, er.y, low);
-          own = po.dist;
-          parent = pp.dist;
-        }
-      }
-      const uint32_t mask = __ballot_sync(0xffffffffu, pass);
-      if (pass) {
-        const uint32_t at = qn + __popc(mask & ((1u << lane) - 1u));
-        q.pos[at] = m;
-        q.span[at] = j;
-        q.own[at] = own;
-        q.parent[at] = parent;
-      }
-      qn += __popc(mask);
-      __syncwarp();
-      if (qn >= 32) {
-        drain_queue<HIST>(S, V, hzbs, q, F, 32, ws, wc, inv_low, b.fade_scale, b.high0, cut, occl_on, cell.slot,
-                          bw);
-        qn -= 32;
-        __syncwarp();
-        if (lane < qn) {
-          q.pos[lane] = q.pos[32 + lane];
-          q.span[lane] = q.span[32 + lane];
-          q.own[lane] = q.own[32 + lane];
-          q.parent[lane] = q.parent[32 + lane];
-        }
-        __syncwarp();
-      }
-    }
-    if (qn)
-      drain_queue<HIST>(S, V, hzbs, q, F, qn, ws, wc, inv_low, b.fade_scale, b.high0, cut, occl_on, cell.slot, bw);
-    __syncwarp();
-    if (!HIST) warp_flush(ws, wc, V, S.slot_capacity, cell.slot, cut);
-    __syncwarp();  // the frame and queue are rewritten by the next chunk
-  }
+  for (uint32_t c = feed.i; c < n_chunks; c = feed.next())
+    chunk_work<HIST, MULTI>(S0, scenes, views, hzbs0, Q, Q.chunks[c], stage[threadIdx.x >> 5], queues[threadIdx.x >> 5],
+                            frames[threadIdx.x >> 5], bw, hist_view, hist_chunks);
   if constexpr (HIST) {
     if (hist_view != ~0u) budget_flush(bw, views[hist_view].hist);
   }
@@ -1328,22 +1346,16 @@ __global__ void __launch_bounds__(128) k_budget(const ViewConst *__restrict__ vi
 // counters' mirror (dyn[6] then marks it settled, and the later rounds' k_finish leave it alone). Bound by the latency
 // of its loads, so both cuts' are issued together, and of the mirror's writes to the host (about 3 us of the 5 that round
 // 0 takes for one view); the later rounds of a launch without retries 3.3 -> 1.3 us each.
-__global__ void __launch_bounds__(128) k_finish(const ViewConst *__restrict__ views, uint32_t nviews,
-                                                uint32_t *__restrict__ ctl, int round,
-                                                uint32_t *__restrict__ host_ctl) {
-  wait_previous_kernel();
-  const uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31;
-  if (round > 0 && ctl[round] == 0) return;  // every view has settled, and this round's passes did nothing
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    retire_queue(ctl);  // the next round's work queue starts empty
-    if (host_ctl) {     // the peak queue demand, for the host's next launch (pinned memory)
-      host_ctl[6] = ctl[6];
-      host_ctl[7] = ctl[7];
-    }
+__device__ __forceinline__ void end_round(uint32_t *ctl, uint32_t *host_ctl) {
+  retire_queue(ctl);  // the next round's work queue starts empty
+  if (host_ctl) {     // the peak queue demand, for the host's next launch (pinned memory)
+    host_ctl[6] = ctl[6];
+    host_ctl[7] = ctl[7];
   }
-  if (v >= nviews) return;
-  const ViewConst &V = views[v];
+}
+
+__device__ __forceinline__ void finish_view(const ViewConst &V, uint32_t *ctl, int round) {
+  const uint32_t lane = threadIdx.x & 31;
   const uint32_t slot_capacity = V.slot_capacity, slots_used = V.slots_used;
   uint32_t *ctr = V.counters;
   if (round > 0 && V.dyn[6] != 0.0f) return;
@@ -1451,6 +1463,147 @@ __global__ void __launch_bounds__(128) k_finish(const ViewConst *__restrict__ vi
     if (lane < VGC_COUNTER_HEADER) w = ctr[lane];
     else if (lane == VGC_COUNTER_HEADER) w = __float_as_uint(V.dyn[0]);
     V.host_stats[lane] = w;
+  }
+}
+
+__global__ void __launch_bounds__(128) k_finish(const ViewConst *__restrict__ views, uint32_t nviews,
+                                                uint32_t *__restrict__ ctl, uint32_t *__restrict__ host_ctl) {
+  wait_previous_kernel();
+  if (blockIdx.x == 0 && threadIdx.x == 0) end_round(ctl, host_ctl);
+  const uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (v < nviews) finish_view(views[v], ctl, 0);
+}
+
+// ------------------------------------------------------------------------------------------------ k_retry
+// Rounds 1 and 2, for the cuts whose draw list or index capacity overflowed in the round before: instance pass, meshlet
+// pass, the in-place tests of what the queue did not hold, and the finish, as four phases of one kernel. Nearly every
+// launch has no such cut, and as kernels of their own the eight passes that then return at once cost their launches:
+// 2 us each of the host's time and 1.3 of the device's. As one kernel: a frame of 64 objects 42 -> 32 us, one of 113k
+// instances 72 -> 62, a batch of 32 views 289 -> 278, eight views of cascades 244 -> 232. What a retried round loses is the
+// 4 us a phase change takes and registers: 113k instances redone twice 131 -> 154 us, eight such views at once 258 -> 304
+// (4 / 5 / 6 / 8 blocks per SM: 144, 310 / 150, 311 / 154, 304 / 177, 334).
+//
+// The phases follow one another by counters, not by a barrier over the grid: a warp takes pieces of the current
+// phase (part p of its round: word 2 p of the round's control words) until none is left, counts those it did (2 p + 1),
+// and the warp that counts the last ones sets the next phase. A waiting block thus waits only for pieces that running
+// warps hold: blocks that are not resident yet hold none, and find the phase where it is when they start. A piece's
+// results are visible to the next phase by the fences around its count and behind the phase word's reading. One thread
+// of a block polls, without a fence: a fence at each poll, which empties the L1 of the warps still at work, cost 25 us of
+// the eight views' frame. Every wait gives up after about a second: the views then report VGC_FAULT_RETRY_WAIT, and the
+// kernel leaves.
+constexpr uint32_t kCtlPhase = 16, kCtlRetry = 17, kRetryWords = 10, kRetryChunks = 8, kRetryRedos = 9;
+static_assert(kCtlRetry + 2 * kRetryWords <= kLaunchCtlWords, "the control words hold both rounds");
+
+__device__ __forceinline__ uint32_t load_relaxed(const uint32_t *word) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+  return v;
+}
+
+// redo_word as a call: its registers would cost k_retry half of its warps, and nearly no round overflows the queue
+template <bool MULTI>
+__device__ __noinline__ void redo_call(const Scene &S0, const Scene *scenes, const ViewConst *views, const HzbDesc *hzbs0,
+                                       const uint2 *units, uint32_t *ctl, uint4 *queue, uint32_t capacity, int round,
+                                       const PassShape &shape, uint32_t *overflow, WarpStage *ws, Survivor *list,
+                                       uint32_t i) {
+  redo_word<false, MULTI>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, round, shape, overflow, ws, list, i);
+}
+
+template <bool MULTI>
+__global__ void __launch_bounds__(128, kRetryBlocks) k_retry(Scene S0, const Scene *__restrict__ scenes,
+                                                  const ViewConst *__restrict__ views, uint32_t nviews,
+                                                  const HzbDesc *__restrict__ hzbs0, const uint2 *__restrict__ units,
+                                                  uint32_t *__restrict__ ctl, uint4 *__restrict__ queue,
+                                                  uint32_t capacity, PassLimits lim, uint32_t *__restrict__ overflow,
+                                                  uint32_t *__restrict__ host_ctl, uint64_t limit_ns) {
+  __shared__ WarpStage stage[4];
+  __shared__ LodQueue queues[4];
+  __shared__ SpanFrame frames[4];
+  __shared__ Survivor lists[4][kHalfUnit];
+  __shared__ BudgetWork<false> no_budget;
+  __shared__ uint32_t current, claimed;  // the phase the block works in, its warps' first pieces there
+  wait_previous_kernel();
+  if (ctl[1] == 0) return;  // no view redoes a cut
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t *const phase = ctl + kCtlPhase;
+  const PassShape shape = pass_shape(ctl, lim);
+  const uint32_t visible = ctl[0];
+  const WorkQueue Q = work_queue(queue, capacity);
+  // thread 0: enters the phase it saw, and takes the warps' first pieces with one atomic
+  const auto enter = [&](uint32_t to) {
+    if (to < 8) claimed = atomicAdd(ctl + kCtlRetry + (to >> 2) * kRetryWords + 2 * (to & 3u), 4u);
+    current = to;
+  };
+  if (threadIdx.x == 0) enter(load_relaxed(phase));
+  for (;;) {
+    __syncthreads();
+    const uint32_t at = current, part = at & 3u;
+    if (at >= 8) return;
+    __threadfence();  // what was written before the phase was set
+    const int round = 1 + int(at >> 2);
+    uint32_t *const words = ctl + kCtlRetry + (at >> 2) * kRetryWords;
+    const uint32_t n = part == 0   ? visible * (shape.fine ? 4 : 2)
+                       : part == 1 ? __ldcg(words + kRetryChunks)
+                       : part == 2 ? __ldcg(words + kRetryRedos)
+                                   : nviews;
+    uint32_t held = 0;
+    for (uint32_t i = claimed + warp, next = 0; i < n; i = __shfl_sync(0xffffffffu, next, 0), held++) {
+      if (lane == 0) next = atomicAdd(words + 2 * part, 1u);  // on its way while this piece is worked on
+      if (part == 0) {
+        instance_unit<false, MULTI, false>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, round, shape, overflow,
+                                           nullptr, lists[warp], i, 0);
+      } else if (part == 1) {
+        uint32_t unused = 0;
+        chunk_work<false, MULTI>(S0, scenes, views, hzbs0, Q, __ldcg(Q.chunks + i), stage[warp], queues[warp],
+                                 frames[warp], no_budget, unused, unused);
+      } else if (part == 2) {
+        redo_call<MULTI>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, round, shape, overflow, &stage[warp],
+                         lists[warp], i);
+      } else {
+        finish_view(views[i], ctl, round);
+      }
+      __syncwarp();
+    }
+    if (held) {
+      __threadfence();
+      __syncwarp();
+      if (lane == 0 && atomicAdd(words + 2 * part + 1, held) + held == n) {  // the phase's last pieces
+        __threadfence();
+        uint32_t next = at + 1;
+        if (part == 0) {
+          const uint32_t chunks = min(uint32_t(__ldcg(queue_counter(ctl)) >> 32), Q.chunk_cap);
+          const uint32_t redos = __ldcg(ctl + kCtlOverflowed) ? (visible * 4 + 31) / 32 : 0u;
+          words[kRetryChunks] = chunks;
+          words[kRetryRedos] = redos;
+          next = at + (chunks ? 1 : redos ? 2 : 3);
+        } else if (part == 1) {
+          next = at + (__ldcg(words + kRetryRedos) ? 1 : 2);
+        } else if (part == 3) {
+          end_round(ctl, host_ctl);
+          next = round == 1 && __ldcg(ctl + 2) ? 4 : 8;
+        }
+        __threadfence();
+        atomicExch(phase, next);
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {  // the pieces left are with other blocks' warps
+      const uint64_t t0 = global_ns();
+      uint32_t now = load_relaxed(phase);
+      for (uint32_t polls = 1; now == at; polls++, now = load_relaxed(phase)) {
+        __nanosleep(100);
+        if ((polls & 31u) == 0 && global_ns() - t0 > limit_ns) {
+          for (uint32_t v = 0; v < nviews; v++) {
+            const uint32_t fault = atomicOr(views[v].counters + VGC_COUNTER_ERROR, (uint32_t)VGC_FAULT_RETRY_WAIT);
+            if (views[v].host_stats) views[v].host_stats[VGC_COUNTER_ERROR] = fault | (uint32_t)VGC_FAULT_RETRY_WAIT;
+          }
+          now = 8;
+          break;
+        }
+      }
+      enter(now);
+    }
   }
 }
 
@@ -1682,7 +1835,6 @@ constexpr uint32_t kStripW = kHzbStripW, kStripH = kHzbStripH, kStripFloats = kS
 constexpr uint32_t kStripBytes = kStripFloats * 4;
 constexpr uint32_t kHzbStripLevels = 5;  // levels 1..4 per strip; k_hzb_tail_views from level 5
 constexpr size_t kHzbStreamSmem = (size_t)kHzbStages * kStripBytes + 128;  // + slack to align the stages to 128
-constexpr uint64_t kWaitLimitNs = 1000000000ull;
 constexpr uint32_t kHzbConsumerWarps = 8, kHzbStreamThreads = 32 * (kHzbConsumerWarps + 1);
 static_assert(kStripW == 128 && kStripH == 32, "the consumer layout covers 128 x 32 strips with 8 warps");
 
@@ -1708,12 +1860,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
       : "r"(smem_addr(bar)), "r"(parity)
       : "memory");
   return done != 0;
-}
-
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
 }
 
 // Phase `parity` of `bar` completed: false once `limit_ns` (or 2^30 polls) passed without it, or once `*abort`
@@ -2011,7 +2157,7 @@ __global__ void __launch_bounds__(256) k_reset(const LaunchInputs in, ViewConst 
   uint4 plan_vec = make_uint4(0u, 0u, 0u, 0u);
   if (first < in.plan_vecs) plan_vec = in.plan_src[first];
   wait_previous_kernel();
-  if (blockIdx.x == 0 && threadIdx.x < 16) ctl[threadIdx.x] = 0;
+  if (blockIdx.x == 0 && threadIdx.x < kLaunchCtlWords) ctl[threadIdx.x] = 0;
   if (first < in.plan_vecs) in.plan_dst[first] = plan_vec;
   for (uint32_t i = first + stride; i < in.plan_vecs; i += stride) in.plan_dst[i] = in.plan_src[i];
   for (uint32_t i = first; i < in.scene_words; i += stride) in.scenes_dst[i] = in.scenes_src[i];
@@ -2158,59 +2304,59 @@ cudaError_t configure_select(bool multi, int *instances_per_sm, int *chunks_per_
 
 template <bool MULTI>
 static cudaError_t instances_kernel(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
-                             uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t grid,
+                             uint32_t *ctl, uint4 *queue, uint32_t capacity, bool hist, uint32_t grid,
                                     const PassLimits &lim, uint32_t *overflow, cudaStream_t st, bool plain) {
-  if (round < 0)  // the budget search's pass
+  if (hist)  // the budget search's pass
     return launch_after(plain, k_instances<true, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, units, ctl, queue,
-                        capacity, 0, lim, overflow);
+                        capacity, lim, overflow);
   return launch_after(plain, k_instances<false, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, units, ctl, queue,
-                      capacity, round, lim, overflow);
+                      capacity, lim, overflow);
 }
 
 cudaError_t launch_instances(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
-                             uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t grid,
+                             uint32_t *ctl, uint4 *queue, uint32_t capacity, bool hist, uint32_t grid,
                              uint32_t *overflow, cudaStream_t st, const PassLimits &lim, bool plain) {
   if (!lim.valid() || !overflow) return cudaErrorInvalidValue;
   if (scenes)
-    return instances_kernel<true>(S, scenes, views, units, ctl, queue, capacity, round, grid, lim, overflow, st, plain);
-  return instances_kernel<false>(S, nullptr, views, units, ctl, queue, capacity, round, grid, lim, overflow, st, plain);
+    return instances_kernel<true>(S, scenes, views, units, ctl, queue, capacity, hist, grid, lim, overflow, st, plain);
+  return instances_kernel<false>(S, nullptr, views, units, ctl, queue, capacity, hist, grid, lim, overflow, st, plain);
 }
 
 template <bool MULTI>
 static cudaError_t instances_redo_kernel(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
-                                  uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, const PassLimits &lim,
+                                  uint32_t *ctl, uint4 *queue, uint32_t capacity, bool hist, const PassLimits &lim,
                                          uint32_t *overflow, uint32_t grid, cudaStream_t st, bool plain) {
-  if (round < 0)
+  if (hist)
     return launch_after(plain, k_instances_redo<true, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, units, ctl, queue,
-                        capacity, 0, lim, overflow);
+                        capacity, lim, overflow);
   return launch_after(plain, k_instances_redo<false, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, units, ctl, queue,
-                      capacity, round, lim, overflow);
+                      capacity, lim, overflow);
 }
 
 cudaError_t launch_instances_redo(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
-                                  uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t *overflow,
+                                  uint32_t *ctl, uint4 *queue, uint32_t capacity, bool hist, uint32_t *overflow,
                                   uint32_t grid, cudaStream_t st, const PassLimits &lim, bool plain) {
   if (!lim.valid() || !overflow || grid == 0)
     return cudaErrorInvalidValue;
   if (scenes)
-    return instances_redo_kernel<true>(S, scenes, views, units, ctl, queue, capacity, round, lim, overflow, grid, st,
+    return instances_redo_kernel<true>(S, scenes, views, units, ctl, queue, capacity, hist, lim, overflow, grid, st,
                                        plain);
-  return instances_redo_kernel<false>(S, nullptr, views, units, ctl, queue, capacity, round, lim, overflow, grid, st,
+  return instances_redo_kernel<false>(S, nullptr, views, units, ctl, queue, capacity, hist, lim, overflow, grid, st,
                                       plain);
 }
 
 template <bool MULTI>
 static cudaError_t chunks_kernel(const Scene &S, const Scene *scenes, const ViewConst *views, uint4 *queue, uint32_t *ctl,
-                          uint32_t capacity, int round, uint32_t grid, cudaStream_t st, bool plain) {
-  if (round < 0)
-    return launch_after(plain, k_chunks<true, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, queue, ctl, capacity, 0);
-  return launch_after(plain, k_chunks<false, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, queue, ctl, capacity, round);
+                          uint32_t capacity, bool hist, uint32_t grid, cudaStream_t st, bool plain) {
+  if (hist)
+    return launch_after(plain, k_chunks<true, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, queue, ctl, capacity);
+  return launch_after(plain, k_chunks<false, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, queue, ctl, capacity);
 }
 
 cudaError_t launch_chunks(const Scene &S, const Scene *scenes, const ViewConst *views, uint4 *queue, uint32_t *ctl,
-                          uint32_t capacity, int round, uint32_t grid, cudaStream_t st, bool plain) {
-  if (scenes) return chunks_kernel<true>(S, scenes, views, queue, ctl, capacity, round, grid, st, plain);
-  return chunks_kernel<false>(S, nullptr, views, queue, ctl, capacity, round, grid, st, plain);
+                          uint32_t capacity, bool hist, uint32_t grid, cudaStream_t st, bool plain) {
+  if (scenes) return chunks_kernel<true>(S, scenes, views, queue, ctl, capacity, hist, grid, st, plain);
+  return chunks_kernel<false>(S, nullptr, views, queue, ctl, capacity, hist, grid, st, plain);
 }
 
 cudaError_t launch_budget(const ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st, bool plain) {
@@ -2218,10 +2364,21 @@ cudaError_t launch_budget(const ViewConst *views, uint32_t nviews, uint32_t *ctl
   return launch_after(plain, k_budget, blocks, 128, 0, st, views, nviews, ctl);
 }
 
-cudaError_t launch_finish(const ViewConst *views, uint32_t nviews, uint32_t *ctl, int round, uint32_t *host_ctl,
-                          cudaStream_t st, bool plain) {
+cudaError_t launch_finish(const ViewConst *views, uint32_t nviews, uint32_t *ctl, uint32_t *host_ctl, cudaStream_t st,
+                          bool plain) {
   const uint32_t blocks = (nviews * 32 + 127) / 128;
-  return launch_after(plain, k_finish, blocks, 128, 0, st, views, nviews, ctl, round, host_ctl);
+  return launch_after(plain, k_finish, blocks, 128, 0, st, views, nviews, ctl, host_ctl);
+}
+
+cudaError_t launch_retry(const Scene &S, const Scene *scenes, const ViewConst *views, uint32_t nviews,
+                         const uint2 *units, uint32_t *ctl, uint4 *queue, uint32_t capacity, uint32_t *overflow,
+                         uint32_t *host_ctl, uint32_t grid, cudaStream_t st, const PassLimits &lim, bool plain) {
+  if (!lim.valid() || !overflow || grid == 0 || nviews == 0) return cudaErrorInvalidValue;
+  if (scenes)
+    return launch_after(plain, k_retry<true>, grid, 128, 0, st, S, scenes, views, nviews, S.hzbs, units, ctl, queue,
+                        capacity, lim, overflow, host_ctl, kWaitLimitNs);
+  return launch_after(plain, k_retry<false>, grid, 128, 0, st, S, scenes, views, nviews, S.hzbs, units, ctl, queue,
+                      capacity, lim, overflow, host_ctl, kWaitLimitNs);
 }
 
 cudaError_t launch_expand(const Scene &S, const ExpandView &view, uint32_t cut, uint32_t *out, uint64_t capacity,
