@@ -407,6 +407,9 @@ int vgc_debug_cells_device(vgc_context *ctx, float *cells, uint32_t capacity, ui
    completes, with a limit of `limit_us` microseconds: *completed = 0 and *waited_ns = the time it waited before it
    gave up; the context stays usable. */
 int vgc_debug_wait_probe(vgc_context *ctx, uint32_t limit_us, uint32_t *completed, uint64_t *waited_ns);
+/* The same for the retry rounds' wait: a phase whose pieces are taken and never counted done, with a limit of
+   `limit_us` microseconds; *faults = what the waiting view reports (VGC_FAULT_RETRY_WAIT). */
+int vgc_debug_retry_probe(vgc_context *ctx, uint32_t limit_us, uint32_t *faults);
 
 #ifdef __cplusplus
 }

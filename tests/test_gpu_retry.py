@@ -1,6 +1,8 @@
 """Rounds 1 and 2 of a cut that overflows its index capacity (k_retry: four phases a round in one kernel): draw sets,
 counters, arguments and controller state equal the oracle's float mirror, for views that settle in different rounds of
 one launch, and when the meshlet queue overflows in a retried round too."""
+import ctypes as C
+import time
 from types import SimpleNamespace
 
 import numpy as np
@@ -83,4 +85,17 @@ def test_queue_overflows_in_a_retried_round(mesh):
         for k in ("rounds", "selected", "drawn", "requested_indices", "work", "faults", "effective_threshold"):
             assert got[k] == want[k], k
         assert key_set(h.vg.draw_list(1, 0), (0, 1, 3)) == key_set(lists[0], (0, 1, 3))
+    h.vg.dispose()
+
+
+@pytest.mark.parametrize("limit_us", [2000, 20000])
+def test_wait_gives_up(mesh, limit_us):
+    """The wait for a phase that nothing completes ends at its limit with a fault; the context then cuts exactly."""
+    spec = SimpleNamespace(meshes=[mesh], instances=[grid_matrices(33, 2.0, 1)])
+    h = Harness(spec, [{}])
+    faults = C.c_uint32()
+    t = time.perf_counter()
+    engine.check(engine.lib().vgc_debug_retry_probe(h.vg.handle, limit_us, C.byref(faults)))
+    assert faults.value == 2 and limit_us * 1e-6 <= time.perf_counter() - t < 2.0
+    h.compare(_camera(33, 2.0), engine.ViewParams(error_threshold=1.0, fresh_state=True))
     h.vg.dispose()

@@ -1286,6 +1286,29 @@ int vgc_debug_wait_probe(vgc_context *ctx, uint32_t limit_us, uint32_t *complete
   return VGC_OK;
 }
 
+int vgc_debug_retry_probe(vgc_context *ctx, uint32_t limit_us, uint32_t *faults) {
+  if (!ctx || !faults || limit_us == 0 || limit_us > 2000000)
+    return fail(VGC_INVALID_ARG, "vgc_debug_retry_probe: bad arguments (limit 1 us .. 2 s)");
+  cudaSetDevice(ctx->device);
+  constexpr size_t counters = 1024, ctl = 2048, overflow = 3072, bytes = 4096;
+  static_assert(sizeof(ViewConst) <= counters && VGC_COUNTER_HEADER * 4 <= 1024 && kLaunchCtlWords * 4 <= 1024, "layout");
+  unsigned char *d = nullptr;
+  CUDA_TRY(cudaMalloc(&d, bytes));
+  ViewConst k;
+  std::memset(&k, 0, sizeof k);
+  k.counters = (uint32_t *)(d + counters);
+  cudaError_t e = cudaMemset(d, 0, bytes);
+  if (e == cudaSuccess) e = cudaMemcpy(d, &k, sizeof k, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess)
+    e = launch_retry_probe((ViewConst *)d, (uint32_t *)(d + ctl), (uint32_t *)(d + overflow), (uint64_t)limit_us * 1000u,
+                           ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (e == cudaSuccess) e = cudaMemcpy(faults, k.counters + VGC_COUNTER_ERROR, 4, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  if (e != cudaSuccess) return fail(VGC_DEVICE_ERROR, std::string("vgc_debug_retry_probe: ") + cudaGetErrorString(e));
+  return VGC_OK;
+}
+
 int vgc_debug_cells_device(vgc_context *ctx, float *cells, uint32_t capacity, uint32_t *count) {
   if (!ctx || !count) return fail(VGC_INVALID_ARG, "null argument");
   int rc = sync_scene(ctx);

@@ -2403,6 +2403,19 @@ cudaError_t launch_hzb_views(const ViewConst *views, uint32_t nviews, uint32_t m
   return launch_after(false, k_hzb_tail_views, nviews, 1024, 0, st, views, kHzbTileLevels);
 }
 
+cudaError_t launch_retry_probe(const ViewConst *view, uint32_t *ctl, uint32_t *overflow, uint64_t limit_ns,
+                               cudaStream_t st) {
+  uint32_t words[kLaunchCtlWords] = {};
+  words[1] = 1;               // a cut is to be redone
+  words[kCtlPhase] = 3;       // round 1, finish
+  words[kCtlRetry + 6] = 1u;  // the next view's index: past the only one
+  cudaError_t e = cudaMemcpyAsync(ctl, words, sizeof words, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return e;
+  return launch_after(true, k_retry<false>, 8, 128, 0, st, Scene(), nullptr, view, 1u, nullptr, nullptr, ctl, nullptr, 0u,
+                      PassLimits(), overflow, nullptr, limit_ns);
+}
+
 cudaError_t launch_wait_probe(uint64_t limit_ns, unsigned long long *out, cudaStream_t st) {
   k_wait_probe<<<1, 32, 0, st>>>(limit_ns, out);
   return cudaGetLastError();
