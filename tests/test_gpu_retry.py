@@ -1,4 +1,5 @@
-"""Rounds 1 and 2 of a cut that overflows its index capacity (k_retry: four phases a round in one kernel): draw sets,
+"""Rounds 1 and 2 of a cut that overflows its index capacity (k_retry: four phases a round in one kernel; after a
+launch that redid a cut, kernels of their own): draw sets,
 counters, arguments and controller state equal the oracle's float mirror, for views that settle in different rounds of
 one launch, and when the meshlet queue overflows in a retried round too."""
 import ctypes as C
@@ -38,7 +39,7 @@ def test_rounds_equal_the_oracle(mesh, n, share):
     whole.vg.dispose()
     assert res["rounds"] == 1 and wanted > 100
     h = Harness(spec, [{}], max_meshlets=1 << 20, max_triangles=max(1, int(wanted * share)))
-    for graph in (False, True):
+    for graph in (False, False, True, True):  # a launch after one that redid a cut has the rounds' own kernels
         _, res = h.compare(cam, p, graph=graph)
         assert res["rounds"] >= 2
     h.vg.dispose()
@@ -58,7 +59,7 @@ def test_views_of_one_launch_settle_in_their_own_round(mesh):
         rounds.append(res["rounds"])
     assert len(set(rounds)) >= 2
     views = [engine.make_view(cam, p) for p in params]
-    for graph in (False, True):
+    for graph in (False, False, True, True):
         h.vg.cut(views, graph=graph)
         for k in range(len(views)):
             s = h.vg.read_stats(k)

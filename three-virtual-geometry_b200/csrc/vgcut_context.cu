@@ -640,6 +640,9 @@ int prepare(vgc_context *ctx, LaunchScratch &s, const vgc_view *views, uint32_t 
   if (s.h_ctl) {  // the last sequence's peak queue demand (spans take 3/4 of the entries, chunks 1/4), plus 25%
     const uint64_t need = std::max<uint64_t>((uint64_t)s.h_ctl[6] * 4 / 3, (uint64_t)s.h_ctl[7] * 4) * 5 / 4;
     if (need > s.chunk_capacity) s.queue_want = (uint32_t)std::min<uint64_t>((need + 65535) & ~65535ull, 1u << 28);
+    if (s.h_ctl[8]) s.split_left = kSplitLaunches + 1;
+    if (s.split_left) s.split_left--;
+    s.h_ctl[8] = 0;
   }
   const uint32_t cells = pad32((uint32_t)ctx->cells.size());
   if ((rc = ensure_scratch(ctx, s, count, (size_t)count * cells))) return rc;
@@ -721,6 +724,9 @@ int prepare_multi(vgc_context *const *ctxs, uint32_t nctx, LaunchScratch &s, con
   if (s.h_ctl) {  // the last sequence's peak queue demand, as in prepare
     const uint64_t need = std::max<uint64_t>((uint64_t)s.h_ctl[6] * 4 / 3, (uint64_t)s.h_ctl[7] * 4) * 5 / 4;
     if (need > s.chunk_capacity) s.queue_want = (uint32_t)std::min<uint64_t>((need + 65535) & ~65535ull, 1u << 28);
+    if (s.h_ctl[8]) s.split_left = kSplitLaunches + 1;
+    if (s.split_left) s.split_left--;
+    s.h_ctl[8] = 0;
   }
   if ((rc = ensure_scratch(ctxs[0], s, count, units))) return rc;
   if (nctx > s.scene_capacity) {
@@ -806,35 +812,43 @@ int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st,
   lim.fine_units = select_grid * 4 / 2;  // fewer half-units than warps
   if (s.any_budget) {  // the triangleBudget search: histogram pass, then the threshold of each budget view
     CUDA_TRY(timed(ctx, capture, VGC_KERNEL_BUDGET, st, [&] {
-      cudaError_t e = launch_instances(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, true,
+      cudaError_t e = launch_instances(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, -1,
                                        select_grid, s.d_overflow, st, lim, plain);
       plain = s.shared;
       if (e == cudaSuccess)
-        e = launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, true, chunk_grid, st,
+        e = launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, -1, chunk_grid, st,
                           s.shared);
       if (e == cudaSuccess)
-        e = launch_instances_redo(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, true,
+        e = launch_instances_redo(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, -1,
                                   s.d_overflow, redo_grid, st, lim, s.shared);
       if (e == cudaSuccess) e = launch_budget(s.d_views, count, s.d_unit_count, st, s.shared);
       return e;
     }));
   }
-  CUDA_TRY(timed(ctx, capture, VGC_KERNEL_SELECT0, st, [&] {
-    return launch_instances(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, false,
-                            select_grid, s.d_overflow, st, lim, plain);
-  }));
-  CUDA_TRY(timed(ctx, capture, VGC_KERNEL_CHUNKS0, st, [&] {
-    return launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, false, chunk_grid, st,
-                         s.shared);
-  }));
-  // units whose items did not fit the queue (returns at once when there are none)
-  CUDA_TRY(timed(ctx, capture, VGC_KERNEL_SELECT_RETRY, st, [&] {
-    return launch_instances_redo(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, false,
-                                 s.d_overflow, redo_grid, st, lim, s.shared);
-  }));
-  CUDA_TRY(timed(ctx, capture, VGC_KERNEL_FINISH, st,
-                 [&] { return launch_finish(s.d_views, count, s.d_unit_count, s.h_ctl, st, s.shared); }));
-  // rounds 1 and 2
+  // The retry rounds are one kernel that returns at once when no cut overflowed (k_retry, which has the figures), until a
+  // sequence of this scratch redoes one: then, for kSplitLaunches sequences after the last that did, they are kernels of
+  // their own, with all of the chip's warps in each. 320 views of which an eighth overflow: @@.
+  const bool split = s.split_left != 0;
+  for (int round = 0; round < (split ? 3 : 1); round++) {
+    if (round > 0 && kChunkShiftRetry) lim.chunk_max = kChunkShiftRetry, lim.chunk_min = std::min(lim.chunk_min, kChunkShiftRetry);
+    CUDA_TRY(timed(ctx, capture, round == 0 ? VGC_KERNEL_SELECT0 : VGC_KERNEL_SELECT_RETRY, st, [&] {
+      return launch_instances(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity, round,
+                              select_grid, s.d_overflow, st, lim, round == 0 ? plain : s.shared);
+    }));
+    CUDA_TRY(timed(ctx, capture, round == 0 ? VGC_KERNEL_CHUNKS0 : VGC_KERNEL_SELECT_RETRY, st, [&] {
+      return launch_chunks(S, scenes, s.d_views, s.d_chunks, s.d_unit_count, s.chunk_capacity, round, chunk_grid, st,
+                           s.shared);
+    }));
+    // units whose items did not fit the queue (returns at once when there are none)
+    CUDA_TRY(timed(ctx, capture, VGC_KERNEL_SELECT_RETRY, st, [&] {
+      return launch_instances_redo(S, scenes, s.d_views, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity,
+                                   round, s.d_overflow, redo_grid, st, lim, s.shared);
+    }));
+    CUDA_TRY(timed(ctx, capture, VGC_KERNEL_FINISH, st, [&] {
+      return launch_finish(s.d_views, count, s.d_unit_count, round, s.h_ctl, st, s.shared);
+    }));
+  }
+  if (split) return VGC_OK;
   if (kChunkShiftRetry) lim.chunk_max = kChunkShiftRetry, lim.chunk_min = std::min(lim.chunk_min, kChunkShiftRetry);
   CUDA_TRY(timed(ctx, capture, VGC_KERNEL_SELECT_RETRY, st, [&] {
     return launch_retry(S, scenes, s.d_views, count, s.d_units, s.d_unit_count, s.d_chunks, s.chunk_capacity,
@@ -1413,6 +1427,7 @@ int vgc_batch_run(vgc_batch *b, const vgc_view *views, uint32_t count, uint32_t 
   const uint32_t cells = (uint32_t)ctx->cells.size();
   if (!b->exec || b->graph_views != count || b->graph_cells != cells || b->graph_slots != ctx->slot_capacity ||
       b->graph_hzb_w != b->scratch.hzb_w || b->graph_hzb_h != b->scratch.hzb_h || b->graph_hzb_tail != b->scratch.hzb_tail ||
+      b->graph_split != (b->scratch.split_left != 0) ||
       b->graph_budget != b->scratch.any_budget || b->graph_queue != b->scratch.d_chunks ||
       b->graph_grids[0] != b->scratch.grid_instances || b->graph_grids[1] != b->scratch.grid_chunks ||
       b->graph_chunk_shift != b->scratch.chunk_shift || b->graph_chunk_tuned != b->scratch.chunk_tuned) {
@@ -1437,6 +1452,7 @@ int vgc_batch_run(vgc_batch *b, const vgc_view *views, uint32_t count, uint32_t 
     b->graph_hzb_w = b->scratch.hzb_w;
     b->graph_hzb_h = b->scratch.hzb_h;
     b->graph_hzb_tail = b->scratch.hzb_tail;
+    b->graph_split = b->scratch.split_left != 0;
     b->graph_budget = b->scratch.any_budget;
     b->graph_queue = b->scratch.d_chunks;
     b->graph_grids[0] = b->scratch.grid_instances;
@@ -1829,19 +1845,19 @@ extern "C" int vgc_cut_noalloc(vgc_context *ctx, const vgc_view *view, uint32_t 
   CUDA_TRY(launch_reset(LaunchInputs(), d_view, 1, ctl, st));
   CUDA_TRY(launch_cells(S, nullptr, d_view, 1, cells, units, ctl, st));
   if (view->triangle_budget > 0) {
-    CUDA_TRY(launch_instances(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, true, ctx->select_grid, overflow,
+    CUDA_TRY(launch_instances(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, -1, ctx->select_grid, overflow,
                               st));
-    CUDA_TRY(launch_chunks(S, nullptr, d_view, chunks, ctl, kNoAllocMaxChunks, true, ctx->chunk_grid, st));
-    CUDA_TRY(launch_instances_redo(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, true, overflow, redo_grid,
+    CUDA_TRY(launch_chunks(S, nullptr, d_view, chunks, ctl, kNoAllocMaxChunks, -1, ctx->chunk_grid, st));
+    CUDA_TRY(launch_instances_redo(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, -1, overflow, redo_grid,
                                    st));
     CUDA_TRY(launch_budget(d_view, 1, ctl, st));
   }
-  CUDA_TRY(launch_instances(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, false, ctx->select_grid, overflow,
+  CUDA_TRY(launch_instances(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, 0, ctx->select_grid, overflow,
                             st));
-  CUDA_TRY(launch_chunks(S, nullptr, d_view, chunks, ctl, kNoAllocMaxChunks, false, ctx->chunk_grid, st));
-  CUDA_TRY(launch_instances_redo(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, false, overflow, redo_grid,
+  CUDA_TRY(launch_chunks(S, nullptr, d_view, chunks, ctl, kNoAllocMaxChunks, 0, ctx->chunk_grid, st));
+  CUDA_TRY(launch_instances_redo(S, nullptr, d_view, units, ctl, chunks, kNoAllocMaxChunks, 0, overflow, redo_grid,
                                  st));
-  CUDA_TRY(launch_finish(d_view, 1, ctl, nullptr, st));
+  CUDA_TRY(launch_finish(d_view, 1, ctl, 0, nullptr, st));
   CUDA_TRY(launch_retry(S, nullptr, d_view, 1, units, ctl, chunks, kNoAllocMaxChunks, overflow, nullptr,
                         (uint32_t)ctx->sm_count * kRetryBlocks, st));
   return VGC_OK;

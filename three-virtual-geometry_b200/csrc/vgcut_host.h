@@ -48,6 +48,7 @@ struct HzbSlot {
 };
 
 constexpr uint32_t kSelectPieces = 4;   // pinned pieces a selectCut's results come back through
+constexpr uint32_t kSplitLaunches = 64;  // after one that redid a cut, launch sequences with the retry rounds' own kernels
 constexpr uint32_t kQueueMin = 262144;  // entries of the smallest meshlet work queue
 
 inline uint32_t pad32(uint32_t x) { return (x + 31u) & ~31u; }
@@ -71,7 +72,8 @@ struct LaunchScratch {
   uint32_t chunk_capacity = 0;    // its entries
   size_t queue_uncharged = 0;     // bytes of it that the owner's HBM budget does not count
   uint32_t queue_want = 0;        // entries the last launch sequence asked for (grown to before the next one)
-  uint32_t *h_ctl = nullptr;      // pinned: control words 6 and 7 at the end of the last launch sequence
+  uint32_t *h_ctl = nullptr;      // pinned: control words 6 and 7 at the end of the last launch sequence; [8] it redid a cut
+  uint32_t split_left = 0;        // launch sequences from now on whose retry rounds are kernels of their own (see enqueue)
   uint32_t grid_instances = 0;    // persistent grids of k_instances / k_chunks (0: the context's occupancy defaults)
   uint32_t grid_chunks = 0;
   uint32_t chunk_shift = kChunkShiftDefault;  // 2^chunk_shift meshlets per k_chunks work unit at most,
@@ -167,6 +169,7 @@ struct vgc_batch {
   uint32_t graph_slots = 0;
   uint32_t graph_hzb_w = 0, graph_hzb_h = 0;
   bool graph_hzb_tail = false;
+  bool graph_split = false;
   bool graph_budget = false;
   const uint4 *graph_queue = nullptr;  // work queue the graph was captured with
   uint32_t graph_grids[2] = {0, 0};    // persistent grids the graph was captured with

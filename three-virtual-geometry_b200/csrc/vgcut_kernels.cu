@@ -1098,16 +1098,17 @@ __global__ void __launch_bounds__(128, MULTI ? 6 : 8) k_instances(Scene S0, cons
                                                    const ViewConst *__restrict__ views,
                                                    const HzbDesc *__restrict__ hzbs0, const uint2 *__restrict__ units,
                                                    uint32_t *__restrict__ ctl, uint4 *__restrict__ queue,
-                                                   uint32_t capacity, PassLimits lim,
+                                                   uint32_t capacity, int round, PassLimits lim,
                                                    uint32_t *__restrict__ overflow) {
   __shared__ Survivor lists[4][kHalfUnit];
   wait_previous_kernel();
+  if (round > 0 && ctl[round] == 0) return;  // no view redoes a cut in this round
   const PassShape shape = pass_shape(ctl, lim);
   const uint32_t work = ctl[0] * (shape.fine ? 4 : 2);
   WarpFeed feed;
   feed.start(ctl + kCtlNextUnit);
   for (uint32_t w = feed.i; w < work; w = feed.next()) {
-    instance_unit<HIST, MULTI, false>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, 0, shape, overflow, nullptr,
+    instance_unit<HIST, MULTI, false>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, round, shape, overflow, nullptr,
                                        lists[threadIdx.x >> 5], w, 0);
     __syncwarp();  // the survivor list is rewritten by the next half-unit
   }
@@ -1141,16 +1142,17 @@ __global__ void __launch_bounds__(128, 4) k_instances_redo(Scene S0, const Scene
                                                             const ViewConst *__restrict__ views,
                                                             const HzbDesc *__restrict__ hzbs0,
                                                             const uint2 *__restrict__ units, uint32_t *__restrict__ ctl,
-                                                            uint4 *__restrict__ queue, uint32_t capacity,
+                                                            uint4 *__restrict__ queue, uint32_t capacity, int round,
                                                             PassLimits lim, uint32_t *__restrict__ overflow) {
   __shared__ WarpStage stage[4];
   __shared__ Survivor lists[4][kHalfUnit];
   wait_previous_kernel();
+  if (round > 0 && ctl[round] == 0) return;
   if (ctl[kCtlOverflowed] == 0) return;
   const PassShape shape = pass_shape(ctl, lim);
   const uint32_t words = (ctl[0] * 4 + 31) / 32;
   for (uint32_t i = warp_grab(ctl + kCtlNextRedo); i < words; i = warp_grab(ctl + kCtlNextRedo))
-    redo_word<HIST, MULTI>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, 0, shape, overflow,
+    redo_word<HIST, MULTI>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, round, shape, overflow,
                            &stage[threadIdx.x >> 5], lists[threadIdx.x >> 5], i);
 }
 
@@ -1272,13 +1274,14 @@ __global__ void __launch_bounds__(128, MULTI || HIST ? 6 : 8) k_chunks(Scene S0,
                                                             const ViewConst *__restrict__ views,
                                                             const HzbDesc *__restrict__ hzbs0,
                                                             uint4 *__restrict__ queue, uint32_t *__restrict__ ctl,
-                                                            uint32_t capacity) {
+                                                            uint32_t capacity, int round) {
   __shared__ WarpStage stage[4];
   __shared__ LodQueue queues[4];
   __shared__ SpanFrame frames[4];
   __shared__ BudgetWork<HIST> budgets[4];
   BudgetWork<HIST> &bw = budgets[threadIdx.x >> 5];
   wait_previous_kernel();
+  if (round > 0 && ctl[round] == 0) return;
   const WorkQueue Q = work_queue(queue, capacity);
   const uint32_t n_chunks = min(uint32_t(*queue_counter(ctl) >> 32), Q.chunk_cap);
   uint32_t hist_view = ~0u, hist_chunks = 0;  // HIST: the view the warp's histogram belongs to
@@ -1346,11 +1349,12 @@ __global__ void __launch_bounds__(128) k_budget(const ViewConst *__restrict__ vi
 // counters' mirror (dyn[6] then marks it settled, and the later rounds' k_finish leave it alone). Bound by the latency
 // of its loads, so both cuts' are issued together, and of the mirror's writes to the host (about 3 us of the 5 that round
 // 0 takes for one view); the later rounds of a launch without retries 3.3 -> 1.3 us each.
-__device__ __forceinline__ void end_round(uint32_t *ctl, uint32_t *host_ctl) {
+__device__ __forceinline__ void end_round(uint32_t *ctl, int round, uint32_t *host_ctl) {
   retire_queue(ctl);  // the next round's work queue starts empty
-  if (host_ctl) {     // the peak queue demand, for the host's next launch (pinned memory)
+  if (host_ctl) {     // the peak queue demand and whether a cut was redone, for the host's next launch (pinned memory)
     host_ctl[6] = ctl[6];
     host_ctl[7] = ctl[7];
+    if (round > 0) host_ctl[8] = 1;
   }
 }
 
@@ -1467,11 +1471,13 @@ __device__ __forceinline__ void finish_view(const ViewConst &V, uint32_t *ctl, i
 }
 
 __global__ void __launch_bounds__(128) k_finish(const ViewConst *__restrict__ views, uint32_t nviews,
-                                                uint32_t *__restrict__ ctl, uint32_t *__restrict__ host_ctl) {
+                                                uint32_t *__restrict__ ctl, int round,
+                                                uint32_t *__restrict__ host_ctl) {
   wait_previous_kernel();
-  if (blockIdx.x == 0 && threadIdx.x == 0) end_round(ctl, host_ctl);
+  if (round > 0 && ctl[round] == 0) return;  // every view has settled, and this round's passes did nothing
+  if (blockIdx.x == 0 && threadIdx.x == 0) end_round(ctl, round, host_ctl);
   const uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (v < nviews) finish_view(views[v], ctl, 0);
+  if (v < nviews) finish_view(views[v], ctl, round);
 }
 
 // ------------------------------------------------------------------------------------------------ k_retry
@@ -1498,15 +1504,6 @@ __device__ __forceinline__ uint32_t load_relaxed(const uint32_t *word) {
   uint32_t v;
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
   return v;
-}
-
-// redo_word as a call: its registers would cost k_retry half of its warps, and nearly no round overflows the queue
-template <bool MULTI>
-__device__ __noinline__ void redo_call(const Scene &S0, const Scene *scenes, const ViewConst *views, const HzbDesc *hzbs0,
-                                       const uint2 *units, uint32_t *ctl, uint4 *queue, uint32_t capacity, int round,
-                                       const PassShape &shape, uint32_t *overflow, WarpStage *ws, Survivor *list,
-                                       uint32_t i) {
-  redo_word<false, MULTI>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, round, shape, overflow, ws, list, i);
 }
 
 template <bool MULTI>
@@ -1557,8 +1554,8 @@ __global__ void __launch_bounds__(128, kRetryBlocks) k_retry(Scene S0, const Sce
         chunk_work<false, MULTI>(S0, scenes, views, hzbs0, Q, __ldcg(Q.chunks + i), stage[warp], queues[warp],
                                  frames[warp], no_budget, unused, unused);
       } else if (part == 2) {
-        redo_call<MULTI>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, round, shape, overflow, &stage[warp],
-                         lists[warp], i);
+        redo_word<false, MULTI>(S0, scenes, views, hzbs0, units, ctl, queue, capacity, round, shape, overflow,
+                                &stage[warp], lists[warp], i);
       } else {
         finish_view(views[i], ctl, round);
       }
@@ -1579,7 +1576,7 @@ __global__ void __launch_bounds__(128, kRetryBlocks) k_retry(Scene S0, const Sce
         } else if (part == 1) {
           next = at + (__ldcg(words + kRetryRedos) ? 1 : 2);
         } else if (part == 3) {
-          end_round(ctl, host_ctl);
+          end_round(ctl, round, host_ctl);
           next = round == 1 && __ldcg(ctl + 2) ? 4 : 8;
         }
         __threadfence();
@@ -2304,59 +2301,59 @@ cudaError_t configure_select(bool multi, int *instances_per_sm, int *chunks_per_
 
 template <bool MULTI>
 static cudaError_t instances_kernel(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
-                             uint32_t *ctl, uint4 *queue, uint32_t capacity, bool hist, uint32_t grid,
+                             uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t grid,
                                     const PassLimits &lim, uint32_t *overflow, cudaStream_t st, bool plain) {
-  if (hist)  // the budget search's pass
+  if (round < 0)  // the budget search's pass
     return launch_after(plain, k_instances<true, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, units, ctl, queue,
-                        capacity, lim, overflow);
+                        capacity, 0, lim, overflow);
   return launch_after(plain, k_instances<false, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, units, ctl, queue,
-                      capacity, lim, overflow);
+                      capacity, round, lim, overflow);
 }
 
 cudaError_t launch_instances(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
-                             uint32_t *ctl, uint4 *queue, uint32_t capacity, bool hist, uint32_t grid,
+                             uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t grid,
                              uint32_t *overflow, cudaStream_t st, const PassLimits &lim, bool plain) {
   if (!lim.valid() || !overflow) return cudaErrorInvalidValue;
   if (scenes)
-    return instances_kernel<true>(S, scenes, views, units, ctl, queue, capacity, hist, grid, lim, overflow, st, plain);
-  return instances_kernel<false>(S, nullptr, views, units, ctl, queue, capacity, hist, grid, lim, overflow, st, plain);
+    return instances_kernel<true>(S, scenes, views, units, ctl, queue, capacity, round, grid, lim, overflow, st, plain);
+  return instances_kernel<false>(S, nullptr, views, units, ctl, queue, capacity, round, grid, lim, overflow, st, plain);
 }
 
 template <bool MULTI>
 static cudaError_t instances_redo_kernel(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
-                                  uint32_t *ctl, uint4 *queue, uint32_t capacity, bool hist, const PassLimits &lim,
+                                  uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, const PassLimits &lim,
                                          uint32_t *overflow, uint32_t grid, cudaStream_t st, bool plain) {
-  if (hist)
+  if (round < 0)
     return launch_after(plain, k_instances_redo<true, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, units, ctl, queue,
-                        capacity, lim, overflow);
+                        capacity, 0, lim, overflow);
   return launch_after(plain, k_instances_redo<false, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, units, ctl, queue,
-                      capacity, lim, overflow);
+                      capacity, round, lim, overflow);
 }
 
 cudaError_t launch_instances_redo(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
-                                  uint32_t *ctl, uint4 *queue, uint32_t capacity, bool hist, uint32_t *overflow,
+                                  uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t *overflow,
                                   uint32_t grid, cudaStream_t st, const PassLimits &lim, bool plain) {
   if (!lim.valid() || !overflow || grid == 0)
     return cudaErrorInvalidValue;
   if (scenes)
-    return instances_redo_kernel<true>(S, scenes, views, units, ctl, queue, capacity, hist, lim, overflow, grid, st,
+    return instances_redo_kernel<true>(S, scenes, views, units, ctl, queue, capacity, round, lim, overflow, grid, st,
                                        plain);
-  return instances_redo_kernel<false>(S, nullptr, views, units, ctl, queue, capacity, hist, lim, overflow, grid, st,
+  return instances_redo_kernel<false>(S, nullptr, views, units, ctl, queue, capacity, round, lim, overflow, grid, st,
                                       plain);
 }
 
 template <bool MULTI>
 static cudaError_t chunks_kernel(const Scene &S, const Scene *scenes, const ViewConst *views, uint4 *queue, uint32_t *ctl,
-                          uint32_t capacity, bool hist, uint32_t grid, cudaStream_t st, bool plain) {
-  if (hist)
-    return launch_after(plain, k_chunks<true, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, queue, ctl, capacity);
-  return launch_after(plain, k_chunks<false, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, queue, ctl, capacity);
+                          uint32_t capacity, int round, uint32_t grid, cudaStream_t st, bool plain) {
+  if (round < 0)
+    return launch_after(plain, k_chunks<true, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, queue, ctl, capacity, 0);
+  return launch_after(plain, k_chunks<false, MULTI>, grid, 128, 0, st, S, scenes, views, S.hzbs, queue, ctl, capacity, round);
 }
 
 cudaError_t launch_chunks(const Scene &S, const Scene *scenes, const ViewConst *views, uint4 *queue, uint32_t *ctl,
-                          uint32_t capacity, bool hist, uint32_t grid, cudaStream_t st, bool plain) {
-  if (scenes) return chunks_kernel<true>(S, scenes, views, queue, ctl, capacity, hist, grid, st, plain);
-  return chunks_kernel<false>(S, nullptr, views, queue, ctl, capacity, hist, grid, st, plain);
+                          uint32_t capacity, int round, uint32_t grid, cudaStream_t st, bool plain) {
+  if (scenes) return chunks_kernel<true>(S, scenes, views, queue, ctl, capacity, round, grid, st, plain);
+  return chunks_kernel<false>(S, nullptr, views, queue, ctl, capacity, round, grid, st, plain);
 }
 
 cudaError_t launch_budget(const ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st, bool plain) {
@@ -2364,10 +2361,10 @@ cudaError_t launch_budget(const ViewConst *views, uint32_t nviews, uint32_t *ctl
   return launch_after(plain, k_budget, blocks, 128, 0, st, views, nviews, ctl);
 }
 
-cudaError_t launch_finish(const ViewConst *views, uint32_t nviews, uint32_t *ctl, uint32_t *host_ctl, cudaStream_t st,
-                          bool plain) {
+cudaError_t launch_finish(const ViewConst *views, uint32_t nviews, uint32_t *ctl, int round, uint32_t *host_ctl,
+                          cudaStream_t st, bool plain) {
   const uint32_t blocks = (nviews * 32 + 127) / 128;
-  return launch_after(plain, k_finish, blocks, 128, 0, st, views, nviews, ctl, host_ctl);
+  return launch_after(plain, k_finish, blocks, 128, 0, st, views, nviews, ctl, round, host_ctl);
 }
 
 cudaError_t launch_retry(const Scene &S, const Scene *scenes, const ViewConst *views, uint32_t nviews,

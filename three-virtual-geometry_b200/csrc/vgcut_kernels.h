@@ -37,25 +37,25 @@ cudaError_t launch_budget(const ViewConst *views, uint32_t nviews, uint32_t *ctl
 // items did not fit the queue, and launch_instances_redo (after launch_chunks of the same pass) tests their items
 // in place and clears the bits.
 cudaError_t launch_instances(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
-                             uint32_t *ctl, uint4 *queue, uint32_t capacity, bool hist, uint32_t grid,
+                             uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t grid,
                              uint32_t *overflow, cudaStream_t st, const PassLimits &lim = PassLimits(),
                              bool plain = false);
 cudaError_t launch_instances_redo(const Scene &S, const Scene *scenes, const ViewConst *views, const uint2 *units,
-                                  uint32_t *ctl, uint4 *queue, uint32_t capacity, bool hist, uint32_t *overflow,
+                                  uint32_t *ctl, uint4 *queue, uint32_t capacity, int round, uint32_t *overflow,
                                   uint32_t grid, cudaStream_t st, const PassLimits &lim = PassLimits(),
                                   bool plain = false);
 // The meshlet work queue (spans and chunks) lives in `queue`, `capacity` uint4 entries; ctl[4..5] counts it.
 cudaError_t launch_chunks(const Scene &S, const Scene *scenes, const ViewConst *views, uint4 *queue,
-                          uint32_t *ctl, uint32_t capacity, bool hist, uint32_t grid, cudaStream_t st,
+                          uint32_t *ctl, uint32_t capacity, int round, uint32_t grid, cudaStream_t st,
                           bool plain = false);
 // computeCell on the device for n cells from c0 of one mesh (bit-identical to the host's computation).
 cudaError_t launch_cells_update(const float4 *inst, const double sphere[4], uint32_t instance_base,
                                 uint32_t instance_count, uint32_t cell_base, uint32_t slot, uint32_t c0, uint32_t n,
                                 CellRec *cells, cudaStream_t st);
 // host_ctl (optional, pinned): receives control words 6 and 7, the peak queue demand of the sequence so far.
-cudaError_t launch_finish(const ViewConst *views, uint32_t nviews, uint32_t *ctl, uint32_t *host_ctl, cudaStream_t st,
-                          bool plain = false);
-// Rounds 1 and 2 of the cuts that overflowed (returns at once when none did), after launch_finish.
+cudaError_t launch_finish(const ViewConst *views, uint32_t nviews, uint32_t *ctl, int round, uint32_t *host_ctl,
+                          cudaStream_t st, bool plain = false);
+// Rounds 1 and 2 of the cuts that overflowed in one kernel (returns at once when none did), after launch_finish.
 cudaError_t launch_retry(const Scene &S, const Scene *scenes, const ViewConst *views, uint32_t nviews,
                          const uint2 *units, uint32_t *ctl, uint4 *queue, uint32_t capacity, uint32_t *overflow,
                          uint32_t *host_ctl, uint32_t grid, cudaStream_t st, const PassLimits &lim = PassLimits(),
