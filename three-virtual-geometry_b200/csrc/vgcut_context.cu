@@ -827,7 +827,8 @@ int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st,
   }
   // The retry rounds are one kernel that returns at once when no cut overflowed (k_retry, which has the figures), until a
   // sequence of this scratch redoes one: then, for kSplitLaunches sequences after the last that did, they are kernels of
-  // their own, with all of the chip's warps in each. 320 views of which an eighth overflow: @@.
+  // their own, with all of the chip's warps in each. 320 views of which an eighth
+  // overflow: 4.00 ms, 4.71 with the one kernel throughout.
   const bool split = s.split_left != 0;
   for (int round = 0; round < (split ? 3 : 1); round++) {
     if (round > 0 && kChunkShiftRetry) lim.chunk_max = kChunkShiftRetry, lim.chunk_min = std::min(lim.chunk_min, kChunkShiftRetry);

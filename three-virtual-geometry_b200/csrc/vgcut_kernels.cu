@@ -1486,8 +1486,9 @@ __global__ void __launch_bounds__(128) k_finish(const ViewConst *__restrict__ vi
 // launch has no such cut, and as kernels of their own the eight passes that then return at once cost their launches:
 // 2 us each of the host's time and 1.3 of the device's. As one kernel: a frame of 64 objects 42 -> 32 us, one of 113k
 // instances 72 -> 62, a batch of 32 views 289 -> 278, eight views of cascades 244 -> 232. What a retried round loses is the
-// 4 us a phase change takes and registers: 113k instances redone twice 131 -> 154 us, eight such views at once 258 -> 304
-// (4 / 5 / 6 / 8 blocks per SM: 144, 310 / 150, 311 / 154, 304 / 177, 334).
+// 4 us a phase change takes and half of the warps: 113k instances redone twice 131 -> 144 us, eight such views at once
+// 258 -> 310 (5 / 6 / 8 blocks per SM: 150, 311 / 154, 304 / 177, 334, with spills). So a launch sequence whose last ones
+// redid a cut has the rounds as kernels of their own (enqueue).
 //
 // The phases follow one another by counters, not by a barrier over the grid: a warp takes pieces of the current
 // phase (part p of its round: word 2 p of the round's control words) until none is left, counts those it did (2 p + 1),
