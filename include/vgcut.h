@@ -365,10 +365,11 @@ int vgc_hzb_info(const vgc_context *ctx, int32_t hzb, uint32_t *levels, uint32_t
 
 /* Device pointers of an output slot (valid after the cut's stream work completes). */
 int vgc_get_output(const vgc_context *ctx, uint32_t slot, vgc_output *out);
-/* vg.readStats (VirtualGeometry.ts:591-632) for one output slot; synchronises with `stream`. */
+/* vg.readStats (VirtualGeometry.ts:591-632) for one output slot; synchronises with `stream`, and with a cut of the slot
+   that ran on another, blocking stream. */
 int vgc_read_stats(vgc_context *ctx, uint32_t slot, vgc_stats *stats, vgc_stream stream);
 /* Copies an output slot's draw list of `cut` into host memory: up to `capacity` entries (4 u32 each); *count
-   receives the number of drawn entries. Synchronises with `stream`. */
+   receives the number of drawn entries. Synchronises as vgc_read_stats does. */
 int vgc_read_draw_list(vgc_context *ctx, uint32_t slot, uint32_t cut, uint32_t *entries, uint32_t capacity,
                        uint32_t *count, vgc_stream stream);
 /* Capacity-controller state words of a state slot (8 u32, fixed point x 10000): read or overwrite. */

@@ -264,9 +264,33 @@ int ensure_outputs(vgc_context *ctx, uint32_t slots) {
   std::memset(ctx->h_stats, 0, (size_t)n * kStatWords * 4);
   CUDA_TRY(cudaMemset(ctx->d_counters.ptr, 0, (size_t)n * ctx->counter_words * 4));
   CUDA_TRY(cudaMemset(ctx->d_args.ptr, 0, (size_t)n * 2 * ctx->slot_capacity * 2 * 5 * 4));
+  ctx->slot_stream.resize(n, nullptr);
   ctx->out_slots = n;
   ctx->out_slot_capacity = ctx->slot_capacity;
   return VGC_OK;
+}
+
+// Output slots [first, first + count) are cut on `st`.
+static void cut_on(vgc_context *ctx, uint32_t first, uint32_t count, cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    st = kReplayed;
+  }
+  if (cs != cudaStreamCaptureStatusNone) st = kReplayed;
+  for (uint32_t i = first; i < first + count; i++)
+    if (ctx->slot_stream[i] != kReplayed) ctx->slot_stream[i] = st;
+}
+
+// Waits for slot `slot`'s cut before its mirrored counters are read; `st` has been waited for. A cut of another stream
+// than that and the context's own is waited for by a copy on the legacy stream, which follows every blocking stream's
+// work (11 us, which a reader that names the cut's stream does not pay).
+static cudaError_t wait_slot(vgc_context *ctx, uint32_t slot, cudaStream_t st) {
+  const cudaStream_t cut = ctx->slot_stream[slot];
+  if (cut != kReplayed && (cut == st || cut == ctx->stream)) return cudaSuccess;
+  uint32_t word;
+  return cudaMemcpy(&word, (const uint32_t *)ctx->d_counters.ptr + (size_t)slot * ctx->counter_words, 4,
+                    cudaMemcpyDeviceToHost);
 }
 
 size_t output_slot_bytes(const vgc_context *ctx) {
@@ -1398,6 +1422,7 @@ int vgc_cut(vgc_context *ctx, const vgc_view *views, uint32_t count, uint32_t fi
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   int rc = prepare(ctx, ctx->scratch, views, count, first_slot);
   if (rc) return rc;
+  cut_on(ctx, first_slot, count, st);
   if ((rc = enqueue(ctx, ctx->scratch, count, st, false))) return rc;
   CUDA_TRY(cudaEventRecord(ctx->scratch.done, st));
   ctx->scratch.pending = true;
@@ -1461,6 +1486,7 @@ int vgc_batch_run(vgc_batch *b, const vgc_view *views, uint32_t count, uint32_t 
     b->graph_chunk_shift = b->scratch.chunk_shift;
     b->graph_chunk_tuned = b->scratch.chunk_tuned;
   }
+  cut_on(ctx, first_slot, count, st);
   CUDA_TRY(cudaGraphLaunch(b->exec, st));
   CUDA_TRY(cudaEventRecord(b->scratch.done, st));
   b->scratch.pending = true;
@@ -1580,6 +1606,7 @@ int vgc_read_stats(vgc_context *ctx, uint32_t slot, vgc_stats *s, vgc_stream str
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   CUDA_TRY(cudaStreamSynchronize(st));
   if (st != ctx->stream) CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  CUDA_TRY(wait_slot(ctx, slot, st));
   const uint32_t *c = ctx->h_stats + (size_t)slot * kStatWords;  // mirrored by the cut's last kernel
   float dyn;
   std::memcpy(&dyn, c + VGC_COUNTER_HEADER, 4);
@@ -1593,6 +1620,7 @@ int vgc_read_draw_list(vgc_context *ctx, uint32_t slot, uint32_t cut, uint32_t *
   if (slot >= ctx->out_slots) return fail(VGC_NOT_FOUND, "output slot not allocated");
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   CUDA_TRY(cudaStreamSynchronize(st));
+  CUDA_TRY(wait_slot(ctx, slot, st));
   const uint32_t sel = ctx->h_stats[(size_t)slot * kStatWords + VGC_COUNTER_CUT0 + cut * 5 + VGC_CUT_SELECTED];
   const uint32_t n = std::min(sel, ctx->opts.max_meshlets);
   *count = n;
@@ -1835,6 +1863,7 @@ extern "C" int vgc_cut_noalloc(vgc_context *ctx, const vgc_view *view, uint32_t 
   uint4 *chunks = (uint4 *)(scratch + kNoAllocChunks);
   uint32_t *overflow = (uint32_t *)(scratch + kNoAllocOverflow);  // zero at load; every pass leaves it zero
   const uint32_t redo_grid = (uint32_t)ctx->sm_count * 2;
+  cut_on(ctx, slot, 1, st);
   // the constants go in by value (k_reset clears the control words)
   k_noalloc_store_view<<<1, 128, 0, st>>>(k, d_view);
   CUDA_TRY(cudaGetLastError());

@@ -51,6 +51,9 @@ constexpr uint32_t kSelectPieces = 4;   // pinned pieces a selectCut's results c
 constexpr uint32_t kSplitLaunches = 64;  // after one that redid a cut, launch sequences with the retry rounds' own kernels
 constexpr uint32_t kQueueMin = 262144;  // entries of the smallest meshlet work queue
 
+// slot_stream of a slot whose cut a stream captured: it runs wherever its graph is replayed, which no call here sees
+inline const cudaStream_t kReplayed = cudaStreamLegacy;
+
 inline uint32_t pad32(uint32_t x) { return (x + 31u) & ~31u; }
 
 }  // namespace vgch
@@ -141,6 +144,7 @@ struct vgc_context {
   uint32_t counter_words = 0;
   DevBuf d_counters, d_draw, d_args, d_dyn, d_hist;
   uint32_t *h_stats = nullptr;  // pinned: kStatWords per output slot, written by the slot's last k_finish
+  std::vector<cudaStream_t> slot_stream;  // per output slot: the stream of its last cut (null: none; kReplayed)
   // controller state slots
   DevBuf d_state;
   uint32_t state_slots = 0;

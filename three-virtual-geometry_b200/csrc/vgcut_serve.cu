@@ -176,6 +176,11 @@ int launch_batch(vgc_server *s, Lane &lane, const std::vector<uint32_t> &slots, 
                        slots.data());
   }
   if (rc) return rc;
+  for (uint32_t i = 0; i < n; i++) {  // a result is read after its completion was seen: its readers have nothing to wait for
+    vgc_context *owner = s->scenes[scene_ids[i]].ctx;
+    cudaStream_t &cut = owner->slot_stream[slots[i]];
+    if (cut != kReplayed) cut = owner->stream;
+  }
   CUDA_TRY(cudaEventRecord(lane.start, lane.stream));
   if ((rc = enqueue(ctx, lane.scratch, n, lane.stream, false))) return rc;
   CUDA_TRY(cudaEventRecord(lane.end, lane.stream));
