@@ -376,7 +376,9 @@ int vgc_read_draw_list(vgc_context *ctx, uint32_t slot, uint32_t cut, uint32_t *
 int vgc_state_access(vgc_context *ctx, uint32_t state_slot, uint32_t *words, int write, vgc_stream stream);
 
 /* Index expansion (GeometryPool.ts:998-1021): writes 3 indices per drawn triangle, (drawSlot << 7) | localVertex,
-   into `index_buffer` (device, capacity of the cut in indices) for output slot `slot` and cut `cut`. */
+   into `index_buffer` (device, capacity of the cut in indices) for output slot `slot` and cut `cut`. Runs after the
+   context's last vgc_cut and before its next, whatever their streams; order it with any other cut (a batch's, a
+   server's, vgc_cut_noalloc, one under capture) on one stream. Asynchronous on `stream`. */
 int vgc_expand(vgc_context *ctx, uint32_t slot, uint32_t cut, uint32_t *index_buffer, uint64_t capacity,
                vgc_stream stream);
 

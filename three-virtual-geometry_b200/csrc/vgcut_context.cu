@@ -270,14 +270,16 @@ int ensure_outputs(vgc_context *ctx, uint32_t slots) {
   return VGC_OK;
 }
 
+static bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+  cudaGetLastError();  // the legacy stream while another stream captures
+  return true;
+}
+
 // Output slots [first, first + count) are cut on `st`.
 static void cut_on(vgc_context *ctx, uint32_t first, uint32_t count, cudaStream_t st) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
-    cudaGetLastError();
-    st = kReplayed;
-  }
-  if (cs != cudaStreamCaptureStatusNone) st = kReplayed;
+  if (capturing(st)) st = kReplayed;
   for (uint32_t i = first; i < first + count; i++)
     if (ctx->slot_stream[i] != kReplayed) ctx->slot_stream[i] = st;
 }
@@ -1426,6 +1428,7 @@ int vgc_cut(vgc_context *ctx, const vgc_view *views, uint32_t count, uint32_t fi
   if ((rc = enqueue(ctx, ctx->scratch, count, st, false))) return rc;
   CUDA_TRY(cudaEventRecord(ctx->scratch.done, st));
   ctx->scratch.pending = true;
+  ctx->scratch.done_on = capturing(st) ? nullptr : st;
   return VGC_OK;
 }
 
@@ -1651,11 +1654,21 @@ int vgc_expand(vgc_context *ctx, uint32_t slot, uint32_t cut, uint32_t *index_bu
     if (ctx->mesh_host[m].used && ctx->mesh_host[m].triangle_count == 0)
       return fail(VGC_INVALID_ARG, "vgc_expand needs meshlet_triangles for every mesh (slot " + std::to_string(m) + ")");
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-  ExpandView k;  // by value: no scratch is written, so nothing waits for the cut before
+  // behind the last plain cut, whichever stream it ran on; the next one waits for this (prepare). In a capture the order
+  // is the graph's.
+  LaunchScratch &s = ctx->scratch;
+  const bool captured = capturing(st);
+  if (!captured && s.pending && s.done_on && s.done_on != st) CUDA_TRY(cudaStreamWaitEvent(st, s.done, 0));
+  ExpandView k;  // by value: no scratch is written
   k.max_drawn = ctx->opts.max_meshlets;
   k.counters = (const uint32_t *)ctx->d_counters.ptr + (size_t)slot * ctx->counter_words;
   k.draw_list = (const uint4 *)ctx->d_draw.ptr + (size_t)slot * 2 * ctx->opts.max_meshlets;
   CUDA_TRY(launch_expand(scene_of(ctx), k, cut, index_buffer, capacity, ctx->sm_count * 8, st));
+  if (captured) return VGC_OK;
+  if (!s.done) CUDA_TRY(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
+  CUDA_TRY(cudaEventRecord(s.done, st));
+  s.pending = true;
+  s.done_on = st;
   return VGC_OK;
 }
 

@@ -99,8 +99,9 @@ struct LaunchScratch {
   size_t plan_maps = 0;             // byte offset of the tensor maps the keys were made for
   cudaStream_t side = nullptr;      // the cell pass beside the HZB build (forked from and joined to the launch stream)
   cudaEvent_t fork = nullptr, join = nullptr;
-  cudaEvent_t done = nullptr;
+  cudaEvent_t done = nullptr;  // the last launch sequence, or the index expansion behind it
   bool pending = false;
+  cudaStream_t done_on = nullptr;  // the stream `done` was recorded on (null: in a capture)
 };
 
 struct vgc_context {
