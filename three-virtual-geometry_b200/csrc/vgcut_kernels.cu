@@ -33,9 +33,17 @@ namespace vgc {
 // resident while this one's last blocks still run. Every kernel of the sequence starts with this wait for the whole
 // kernel before it (and, since that one waited too, for all before), so nothing is read early; what is saved is the
 // launch latency between the sequence's dozen short kernels. A plain launch returns at once.
-__device__ __forceinline__ void wait_previous_kernel() {
+//
+// `written`: the kernel's pointers to what the kernel before it writes. That memory changes while this kernel is already
+// resident, so these parameters carry no __restrict__ (with const it lets the compiler read through the non-coherent path,
+// and place reads ahead of the wait), and the wait hands their values on afresh: no read through them can come before it.
+// What earlier kernels wrote is final when this one becomes resident, since the kernel between waited for them.
+template <class... P>
+__device__ __forceinline__ void wait_previous_kernel(P *&...written) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const auto fresh = [](auto *&p) { asm volatile("" : "+l"(p)::"memory"); };
+  (fresh(written), ...);
 }
 
 constexpr uint64_t kWaitLimitNs = 1000000000ull;  // after which a wait of a kernel gives up
@@ -244,11 +252,10 @@ __device__ __forceinline__ uint32_t *mesh_count(const ViewConst &V, uint32_t slo
 
 // ------------------------------------------------------------------------------------------------ k_cells
 template <bool MULTI>
-__global__ void __launch_bounds__(256) k_cells(Scene S0, const Scene *__restrict__ scenes,
-                                               const ViewConst *__restrict__ views, uint32_t nviews,
-                                               uint32_t total_units, uint2 *__restrict__ units,
-                                               uint32_t *__restrict__ unit_count) {
-  wait_previous_kernel();
+__global__ void __launch_bounds__(256) k_cells(Scene S0, const Scene *scenes, const ViewConst *views,
+                                               uint32_t nviews, uint32_t total_units, uint2 *__restrict__ units,
+                                               uint32_t *unit_count) {
+  wait_previous_kernel(scenes, views, unit_count);
   const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
   if ((u & ~31u) >= total_units) return;  // whole warp out of range
@@ -1096,15 +1103,16 @@ __device__ __forceinline__ void instance_unit(const Scene &S0, const Scene *__re
 template <bool HIST, bool MULTI>
 __global__ void __launch_bounds__(128, MULTI ? 6 : 8) k_instances(Scene S0, const Scene *__restrict__ scenes,
                                                    const ViewConst *__restrict__ views,
-                                                   const HzbDesc *__restrict__ hzbs0, const uint2 *__restrict__ units,
+                                                   const HzbDesc *__restrict__ hzbs0, const uint2 *units,
                                                    uint32_t *__restrict__ ctl, uint4 *__restrict__ queue,
                                                    uint32_t capacity, int round, PassLimits lim,
                                                    uint32_t *__restrict__ overflow) {
   __shared__ Survivor lists[4][kHalfUnit];
-  wait_previous_kernel();
-  if (round > 0 && ctl[round] == 0) return;  // no view redoes a cut in this round
-  const PassShape shape = pass_shape(ctl, lim);
-  const uint32_t work = ctl[0] * (shape.fine ? 4 : 2);
+  const uint32_t *words = ctl;  // what is read of them; the rest of the kernel adds to some (batch_cascades 1% faster so)
+  wait_previous_kernel(units, words);
+  if (round > 0 && words[round] == 0) return;  // no view redoes a cut in this round
+  const PassShape shape = pass_shape(words, lim);
+  const uint32_t work = words[0] * (shape.fine ? 4 : 2);
   WarpFeed feed;
   feed.start(ctl + kCtlNextUnit);
   for (uint32_t w = feed.i; w < work; w = feed.next()) {
@@ -1141,12 +1149,12 @@ template <bool HIST, bool MULTI>
 __global__ void __launch_bounds__(128, 4) k_instances_redo(Scene S0, const Scene *__restrict__ scenes,
                                                             const ViewConst *__restrict__ views,
                                                             const HzbDesc *__restrict__ hzbs0,
-                                                            const uint2 *__restrict__ units, uint32_t *__restrict__ ctl,
+                                                            const uint2 *__restrict__ units, uint32_t *ctl,
                                                             uint4 *__restrict__ queue, uint32_t capacity, int round,
                                                             PassLimits lim, uint32_t *__restrict__ overflow) {
   __shared__ WarpStage stage[4];
   __shared__ Survivor lists[4][kHalfUnit];
-  wait_previous_kernel();
+  wait_previous_kernel(ctl);
   if (round > 0 && ctl[round] == 0) return;
   if (ctl[kCtlOverflowed] == 0) return;
   const PassShape shape = pass_shape(ctl, lim);
@@ -1273,14 +1281,14 @@ template <bool HIST, bool MULTI>
 __global__ void __launch_bounds__(128, MULTI || HIST ? 6 : 8) k_chunks(Scene S0, const Scene *__restrict__ scenes,
                                                             const ViewConst *__restrict__ views,
                                                             const HzbDesc *__restrict__ hzbs0,
-                                                            uint4 *__restrict__ queue, uint32_t *__restrict__ ctl,
+                                                            uint4 *queue, uint32_t *ctl,
                                                             uint32_t capacity, int round) {
   __shared__ WarpStage stage[4];
   __shared__ LodQueue queues[4];
   __shared__ SpanFrame frames[4];
   __shared__ BudgetWork<HIST> budgets[4];
   BudgetWork<HIST> &bw = budgets[threadIdx.x >> 5];
-  wait_previous_kernel();
+  wait_previous_kernel(queue, ctl);
   if (round > 0 && ctl[round] == 0) return;
   const WorkQueue Q = work_queue(queue, capacity);
   const uint32_t n_chunks = min(uint32_t(*queue_counter(ctl) >> 32), Q.chunk_cap);
@@ -1304,8 +1312,8 @@ __global__ void __launch_bounds__(128, MULTI || HIST ? 6 : 8) k_chunks(Scene S0,
 // T(t_k) <= budget (255 when none) sets this frame's errorThreshold and bands. Also empties the chunk queue for the
 // frame's first selection round.
 __global__ void __launch_bounds__(128) k_budget(const ViewConst *__restrict__ views, uint32_t nviews,
-                                                uint32_t *__restrict__ ctl) {
-  wait_previous_kernel();
+                                                uint32_t *ctl) {
+  wait_previous_kernel(ctl);
   if (blockIdx.x == 0 && threadIdx.x == 0) retire_queue(ctl);
   const uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
@@ -1471,9 +1479,8 @@ __device__ __forceinline__ void finish_view(const ViewConst &V, uint32_t *ctl, i
 }
 
 __global__ void __launch_bounds__(128) k_finish(const ViewConst *__restrict__ views, uint32_t nviews,
-                                                uint32_t *__restrict__ ctl, int round,
-                                                uint32_t *__restrict__ host_ctl) {
-  wait_previous_kernel();
+                                                uint32_t *ctl, int round, uint32_t *__restrict__ host_ctl) {
+  wait_previous_kernel(ctl);
   if (round > 0 && ctl[round] == 0) return;  // every view has settled, and this round's passes did nothing
   if (blockIdx.x == 0 && threadIdx.x == 0) end_round(ctl, round, host_ctl);
   const uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1511,7 +1518,7 @@ template <bool MULTI>
 __global__ void __launch_bounds__(128, kRetryBlocks) k_retry(Scene S0, const Scene *__restrict__ scenes,
                                                   const ViewConst *__restrict__ views, uint32_t nviews,
                                                   const HzbDesc *__restrict__ hzbs0, const uint2 *__restrict__ units,
-                                                  uint32_t *__restrict__ ctl, uint4 *__restrict__ queue,
+                                                  uint32_t *ctl, uint4 *__restrict__ queue,
                                                   uint32_t capacity, PassLimits lim, uint32_t *__restrict__ overflow,
                                                   uint32_t *__restrict__ host_ctl, uint64_t limit_ns) {
   __shared__ WarpStage stage[4];
@@ -1520,7 +1527,7 @@ __global__ void __launch_bounds__(128, kRetryBlocks) k_retry(Scene S0, const Sce
   __shared__ Survivor lists[4][kHalfUnit];
   __shared__ BudgetWork<false> no_budget;
   __shared__ uint32_t current, claimed;  // the phase the block works in, its warps' first pieces there
-  wait_previous_kernel();
+  wait_previous_kernel(ctl);
   if (ctl[1] == 0) return;  // no view redoes a cut
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t *const phase = ctl + kCtlPhase;
@@ -1659,7 +1666,7 @@ __device__ __forceinline__ void hzb_store(const HzbDesc &H, float *__restrict__ 
 // partner, and the pair's lanes go on with different texels, so that no lane holds a copy until level 3. A level's
 // texel past the level's edge holds the max over the edge texels of the same rows (or columns), which the in-range
 // texel's footprint already contains, so the max over the 2 x 2 block equals the max over its clamped reads.
-__device__ __forceinline__ void hzb_tile64(const float *__restrict__ depth, const HzbDesc &H, float *__restrict__ out,
+__device__ __forceinline__ void hzb_tile64(const float *depth, const HzbDesc &H, float *__restrict__ out,
                                            bool copy_mip0, uint32_t ox, uint32_t oy, float (*s4)[4]) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t W = H.w[0], Hh = H.h[0];
@@ -1668,8 +1675,8 @@ __device__ __forceinline__ void hzb_tile64(const float *__restrict__ depth, cons
 #pragma unroll
   for (int r = 0; r < 16; r++) {
     const float *row = depth + (size_t)min(y0 + r, Hh - 1) * W;
-    v[r][0] = __ldg(row + min(x0, W - 1));
-    v[r][1] = __ldg(row + min(x1, W - 1));
+    v[r][0] = row[min(x0, W - 1)];  // coherent loads: the kernel before may have drawn the image
+    v[r][1] = row[min(x1, W - 1)];
   }
   if (copy_mip0) {
     float *o = out + H.off[0];
@@ -1732,17 +1739,17 @@ __device__ __forceinline__ void hzb_tile64(const float *__restrict__ depth, cons
   if (lane == 0) hzb_store(H, out, 6, ox >> 6, oy >> 6, m);
 }
 
-__global__ void __launch_bounds__(kHzbTileThreads) k_hzb_tiles(const float *__restrict__ depth, HzbDesc H,
-                                                               float *__restrict__ out, int copy_mip0) {
+__global__ void __launch_bounds__(kHzbTileThreads) k_hzb_tiles(const float *depth, HzbDesc H, float *__restrict__ out,
+                                                               int copy_mip0) {
   __shared__ float s4[4][4];
-  wait_previous_kernel();
+  wait_previous_kernel(depth);
   hzb_tile64(depth, H, out, copy_mip0 != 0, blockIdx.x * kHzbTile, blockIdx.y * kHzbTile, s4);
 }
 
 // The HZB builds of a batch: grid.z = view, views without a depth image skip.
-__global__ void __launch_bounds__(kHzbTileThreads) k_hzb_tiles_views(const ViewConst *__restrict__ views) {
+__global__ void __launch_bounds__(kHzbTileThreads) k_hzb_tiles_views(const ViewConst *views) {
   __shared__ float s4[4][4];
-  wait_previous_kernel();
+  wait_previous_kernel(views);
   const ViewConst &V = views[blockIdx.z];
   if (!V.build_hzb) return;
   const HzbDesc &H = *V.hzb_desc;
@@ -1762,7 +1769,7 @@ struct TailSmem {
   float even[kTailTexels], odd[kTailTexels / 2];  // a level of 4,096 texels has at most 2,048 in the next
 };
 
-__device__ __forceinline__ void hzb_tail(const HzbDesc &H, float *__restrict__ out, uint32_t first, TailSmem &S) {
+__device__ __forceinline__ void hzb_tail(const HzbDesc &H, float *out, uint32_t first, TailSmem &S) {
   const uint32_t levels = H.levels;
   if (threadIdx.x < kMaxHzbLevels) {
     S.off[threadIdx.x] = H.off[threadIdx.x];
@@ -1800,9 +1807,9 @@ __global__ void __launch_bounds__(1024) k_hzb_tail_views(const ViewConst *__rest
 }
 
 // Levels 7 and up (at most 15 x 9 texels for a 1080p mip 0).
-__global__ void __launch_bounds__(1024) k_hzb_tail(HzbDesc H, float *__restrict__ out) {
+__global__ void __launch_bounds__(1024) k_hzb_tail(HzbDesc H, float *out) {
   __shared__ TailSmem S;
-  wait_previous_kernel();
+  wait_previous_kernel(out);
   hzb_tail(H, out, kHzbTileLevels, S);
 }
 
@@ -1924,14 +1931,14 @@ __device__ __forceinline__ void strip_store(const StripDesc &D, uint32_t l, uint
 }
 
 __global__ void __launch_bounds__(kHzbStreamThreads, VGC_HZB_BLOCKS_PER_SM) k_hzb_stream(
-    const unsigned char *__restrict__ plan) {
+    const unsigned char *plan) {
   extern __shared__ __align__(16) unsigned char dyn_smem[];
   // kHzbStages strips from the first 128-byte boundary of the dynamic shared memory (a bulk-tensor destination)
   float *stage = reinterpret_cast<float *>(dyn_smem + ((128u - (smem_addr(dyn_smem) & 127u)) & 127u));
   __shared__ __align__(8) uint64_t full[kHzbStages], empty[kHzbStages];
   __shared__ uint4 meta[kHzbStages];  // job, ox, oy, tma of the strip in each stage
   __shared__ uint32_t abort;
-  wait_previous_kernel();
+  wait_previous_kernel(plan);
   const HzbPlanHead &P = *reinterpret_cast<const HzbPlanHead *>(plan);
   const HzbJob *jobs = reinterpret_cast<const HzbJob *>(plan + sizeof(HzbPlanHead));
   const uint32_t njobs = P.jobs;
@@ -2143,8 +2150,8 @@ __global__ void __launch_bounds__(128) k_select_cut(Scene S, uint32_t slot, uint
 // output pointers from the view constants, so a captured graph serves any output slots. The launch's inputs (view
 // constants, HZB plan, scene table) come from pinned host memory by this kernel's own reads: as copies before it they
 // cost 6 us more in a stream and 20 us in a graph (the gap between a copy node and the first kernel). blocks <= views.
-__global__ void __launch_bounds__(256) k_reset(const LaunchInputs in, ViewConst *__restrict__ views, uint32_t nviews,
-                                               uint32_t *__restrict__ ctl) {
+__global__ void __launch_bounds__(256) k_reset(const LaunchInputs in, ViewConst *views, uint32_t nviews,
+                                               uint32_t *ctl) {
   __shared__ __align__(16) uint32_t staged[sizeof(ViewConst) / 4];
   static_assert(sizeof(ViewConst) / 4 <= 256, "a block stages a view's constants with one word per thread");
   const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
@@ -2154,7 +2161,7 @@ __global__ void __launch_bounds__(256) k_reset(const LaunchInputs in, ViewConst 
   if (host_view) view_word = reinterpret_cast<const uint32_t *>(in.views + blockIdx.x)[threadIdx.x];
   uint4 plan_vec = make_uint4(0u, 0u, 0u, 0u);
   if (first < in.plan_vecs) plan_vec = in.plan_src[first];
-  wait_previous_kernel();
+  wait_previous_kernel(views, ctl);
   if (blockIdx.x == 0 && threadIdx.x < kLaunchCtlWords) ctl[threadIdx.x] = 0;
   if (first < in.plan_vecs) in.plan_dst[first] = plan_vec;
   for (uint32_t i = first + stride; i < in.plan_vecs; i += stride) in.plan_dst[i] = in.plan_src[i];
