@@ -52,3 +52,14 @@ def test_reads_follow_the_wait(name):
 def test_every_kernel_with_the_attribute_waits():
     for name in set(re.findall(r"launch_after\([^,]*,\s*(k_\w+)", SOURCE)):
         assert "wait_previous_kernel(" in _kernel(name)[1], name
+
+
+def test_retry_phase_is_acquired_by_the_thread_that_reads_it():
+    """The thread that saw the phase word change fences before the barrier that lets its block in (the word itself is
+    polled relaxed), and so does each thread that counts a phase's last pieces before it reads what they wrote."""
+    body = _kernel("k_retry")[1]
+    enter = body[body.index("const auto enter"):]
+    enter = enter[:enter.index("};")]
+    assert enter.index("fence_gpu()") < enter.index("atomicAdd") < enter.index("current = to")
+    last = body[body.index("+ held == n"):]
+    assert last.index("__threadfence()") < last.index("__ldcg")
