@@ -413,6 +413,10 @@ int vgc_debug_wait_probe(vgc_context *ctx, uint32_t limit_us, uint32_t *complete
 /* The same for the retry rounds' wait: a phase whose pieces are taken and never counted done, with a limit of
    `limit_us` microseconds; *faults = what the waiting view reports (VGC_FAULT_RETRY_WAIT). */
 int vgc_debug_retry_probe(vgc_context *ctx, uint32_t limit_us, uint32_t *faults);
+/* Leaves the context's last vgc_cut (noalloc: the last vgc_cut_noalloc) as a retry round that gave up would: its first
+   view's counters cleared, the visible units marked as still to be tested in place, then the wait of `limit_us` that
+   runs out. Its counters, faults among them, and later cuts can then be looked at. Synchronous. */
+int vgc_debug_retry_lost(vgc_context *ctx, int noalloc, uint32_t limit_us);
 
 #ifdef __cplusplus
 }

@@ -323,7 +323,8 @@ int ensure_state(vgc_context *ctx, uint32_t slot) {
 }
 
 // the unit list of `n` (view, cell) units and, after it, the overflow bits of its 4 n warp-units
-static size_t unit_bytes(size_t n) { return n * sizeof(uint2) + (n * 4 + 31) / 32 * sizeof(uint32_t); }
+static size_t overflow_bytes(size_t n) { return (n * 4 + 31) / 32 * sizeof(uint32_t); }
+static size_t unit_bytes(size_t n) { return n * sizeof(uint2) + overflow_bytes(n); }
 
 int ensure_scratch(vgc_context *ctx, LaunchScratch &s, uint32_t views, size_t units) {
   if (!s.owner) s.owner = ctx;  // growth below is counted where the scratch was first counted
@@ -362,7 +363,7 @@ int ensure_scratch(vgc_context *ctx, LaunchScratch &s, uint32_t views, size_t un
     size_t n = std::max<size_t>(units, 32);
     CUDA_TRY(cudaMalloc(&s.d_units, unit_bytes(n)));
     s.d_overflow = reinterpret_cast<uint32_t *>(s.d_units + n);
-    CUDA_TRY(cudaMemset(s.d_overflow, 0, unit_bytes(n) - n * sizeof(uint2)));
+    CUDA_TRY(cudaMemset(s.d_overflow, 0, overflow_bytes(n)));
     ctx->bytes += unit_bytes(n);
     s.unit_capacity = n;
   }
@@ -649,6 +650,21 @@ int view_constants(vgc_context *ctx, const vgc_view &in, uint32_t out_slot, uint
   return VGC_OK;
 }
 
+// Waits for the scratch's last launch sequence and takes in what it left in the control words.
+static int after_last(LaunchScratch &s) {
+  if (s.pending) CUDA_TRY(cudaEventSynchronize(s.done));
+  s.pending = false;
+  if (!s.h_ctl) return VGC_OK;
+  // its peak queue demand (spans take 3/4 of the entries, chunks 1/4), plus 25%
+  const uint64_t need = std::max<uint64_t>((uint64_t)s.h_ctl[6] * 4 / 3, (uint64_t)s.h_ctl[7] * 4) * 5 / 4;
+  if (need > s.chunk_capacity) s.queue_want = (uint32_t)std::min<uint64_t>((need + 65535) & ~65535ull, 1u << 28);
+  if (s.h_ctl[8]) s.split_left = kSplitLaunches + 1;
+  if (s.split_left) s.split_left--;
+  if (s.h_ctl[9]) CUDA_TRY(cudaMemset(s.d_overflow, 0, overflow_bytes(s.unit_capacity)));
+  s.h_ctl[8] = s.h_ctl[9] = 0;
+  return VGC_OK;
+}
+
 // Prepares scene, outputs and the views' constants in `s.h_views` (pinned).
 int prepare(vgc_context *ctx, LaunchScratch &s, const vgc_view *views, uint32_t count, uint32_t first_slot,
             const uint32_t *slots) {
@@ -661,15 +677,7 @@ int prepare(vgc_context *ctx, LaunchScratch &s, const vgc_view *views, uint32_t 
     for (uint32_t i = 0; i < count; i++) slot_end = std::max(slot_end, slots[i] + 1);
   }
   if ((rc = ensure_outputs(ctx, slot_end))) return rc;
-  if (s.pending) CUDA_TRY(cudaEventSynchronize(s.done));
-  s.pending = false;
-  if (s.h_ctl) {  // the last sequence's peak queue demand (spans take 3/4 of the entries, chunks 1/4), plus 25%
-    const uint64_t need = std::max<uint64_t>((uint64_t)s.h_ctl[6] * 4 / 3, (uint64_t)s.h_ctl[7] * 4) * 5 / 4;
-    if (need > s.chunk_capacity) s.queue_want = (uint32_t)std::min<uint64_t>((need + 65535) & ~65535ull, 1u << 28);
-    if (s.h_ctl[8]) s.split_left = kSplitLaunches + 1;
-    if (s.split_left) s.split_left--;
-    s.h_ctl[8] = 0;
-  }
+  if ((rc = after_last(s))) return rc;
   const uint32_t cells = pad32((uint32_t)ctx->cells.size());
   if ((rc = ensure_scratch(ctx, s, count, (size_t)count * cells))) return rc;
   s.multi = false;
@@ -745,15 +753,7 @@ int prepare_multi(vgc_context *const *ctxs, uint32_t nctx, LaunchScratch &s, con
     if (slot_end[k] && (rc = ensure_outputs(ctxs[k], slot_end[k]))) return rc;
   }
   for (uint32_t i = 0; i < count; i++) units += pad32((uint32_t)ctxs[scene[i]]->cells.size());
-  if (s.pending) CUDA_TRY(cudaEventSynchronize(s.done));
-  s.pending = false;
-  if (s.h_ctl) {  // the last sequence's peak queue demand, as in prepare
-    const uint64_t need = std::max<uint64_t>((uint64_t)s.h_ctl[6] * 4 / 3, (uint64_t)s.h_ctl[7] * 4) * 5 / 4;
-    if (need > s.chunk_capacity) s.queue_want = (uint32_t)std::min<uint64_t>((need + 65535) & ~65535ull, 1u << 28);
-    if (s.h_ctl[8]) s.split_left = kSplitLaunches + 1;
-    if (s.split_left) s.split_left--;
-    s.h_ctl[8] = 0;
-  }
+  if ((rc = after_last(s))) return rc;
   if ((rc = ensure_scratch(ctxs[0], s, count, units))) return rc;
   if (nctx > s.scene_capacity) {
     vgc_context *owner = s.owner ? s.owner : ctxs[0];
@@ -1341,8 +1341,8 @@ int vgc_debug_retry_probe(vgc_context *ctx, uint32_t limit_us, uint32_t *faults)
   cudaError_t e = cudaMemset(d, 0, bytes);
   if (e == cudaSuccess) e = cudaMemcpy(d, &k, sizeof k, cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
-    e = launch_retry_probe((ViewConst *)d, (uint32_t *)(d + ctl), (uint32_t *)(d + overflow), (uint64_t)limit_us * 1000u,
-                           ctx->stream);
+    e = launch_retry_probe((ViewConst *)d, (uint32_t *)(d + ctl), (uint32_t *)(d + overflow), nullptr,
+                           (uint64_t)limit_us * 1000u, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e == cudaSuccess) e = cudaMemcpy(faults, k.counters + VGC_COUNTER_ERROR, 4, cudaMemcpyDeviceToHost);
   cudaFree(d);
@@ -1825,7 +1825,11 @@ int noalloc_scratch(int device, unsigned char **out) {
 // Writes the view constants into the scratch array. They travel as a kernel argument, which the launch copies, so
 // no host buffer has to outlive the call and nothing is copied from host memory.
 static_assert(sizeof(ViewConst) % 4 == 0, "view constants are copied as 32-bit words");
-__global__ void k_noalloc_store_view(const ViewConst k, ViewConst *dst) {
+// It also clears the overflow bits when a wait of the call before gave up (every other call leaves them zero).
+__global__ void k_noalloc_store_view(const ViewConst k, ViewConst *dst, const uint32_t *ctl, uint32_t *overflow,
+                                     uint32_t overflow_words) {
+  if (ctl[kCtlGaveUp])
+    for (uint32_t i = threadIdx.x; i < overflow_words; i += blockDim.x) overflow[i] = 0;
   const uint32_t *src = reinterpret_cast<const uint32_t *>(&k);
   uint32_t *out = reinterpret_cast<uint32_t *>(dst);
   for (uint32_t i = threadIdx.x; i < sizeof(ViewConst) / 4; i += blockDim.x) out[i] = src[i];
@@ -1874,11 +1878,11 @@ extern "C" int vgc_cut_noalloc(vgc_context *ctx, const vgc_view *view, uint32_t 
   ViewConst *d_view = (ViewConst *)(scratch + kNoAllocView);
   uint2 *units = (uint2 *)(scratch + kNoAllocUnits);
   uint4 *chunks = (uint4 *)(scratch + kNoAllocChunks);
-  uint32_t *overflow = (uint32_t *)(scratch + kNoAllocOverflow);  // zero at load; every pass leaves it zero
+  uint32_t *overflow = (uint32_t *)(scratch + kNoAllocOverflow);  // zero at load; every pass that completes leaves it zero
   const uint32_t redo_grid = (uint32_t)ctx->sm_count * 2;
   cut_on(ctx, slot, 1, st);
   // the constants go in by value (k_reset clears the control words)
-  k_noalloc_store_view<<<1, 128, 0, st>>>(k, d_view);
+  k_noalloc_store_view<<<1, 128, 0, st>>>(k, d_view, ctl, overflow, kNoAllocMaxUnits * 4 / 32);
   CUDA_TRY(cudaGetLastError());
   const Scene S = scene_of(ctx);
   if (build_hzb) {
@@ -1903,5 +1907,32 @@ extern "C" int vgc_cut_noalloc(vgc_context *ctx, const vgc_view *view, uint32_t 
   CUDA_TRY(launch_finish(d_view, 1, ctl, 0, nullptr, st));
   CUDA_TRY(launch_retry(S, nullptr, d_view, 1, units, ctl, chunks, kNoAllocMaxChunks, overflow, nullptr,
                         (uint32_t)ctx->sm_count * kRetryBlocks, st));
+  return VGC_OK;
+}
+
+extern "C" int vgc_debug_retry_lost(vgc_context *ctx, int noalloc, uint32_t limit_us) {
+  if (!ctx || limit_us == 0 || limit_us > 2000000) return fail(VGC_INVALID_ARG, "vgc_debug_retry_lost: bad arguments");
+  cudaSetDevice(ctx->device);
+  LaunchScratch &s = ctx->scratch;
+  if (!noalloc && !s.d_views) return fail(VGC_INVALID_ARG, "vgc_debug_retry_lost: no cut before");
+  unsigned char *scratch = nullptr;
+  if (noalloc)
+    if (const int rc = noalloc_scratch(ctx->device, &scratch)) return rc;
+  CUDA_TRY(cudaDeviceSynchronize());
+  uint32_t *ctl = noalloc ? (uint32_t *)(scratch + kNoAllocCtl) : s.d_unit_count;
+  const ViewConst *view = noalloc ? (const ViewConst *)(scratch + kNoAllocView) : s.d_views;
+  uint32_t *overflow = noalloc ? (uint32_t *)(scratch + kNoAllocOverflow) : s.d_overflow;
+  ViewConst k;
+  uint32_t units = 0;
+  CUDA_TRY(cudaMemcpy(&k, view, sizeof k, cudaMemcpyDeviceToHost));
+  CUDA_TRY(cudaMemcpy(&units, ctl, 4, cudaMemcpyDeviceToHost));
+  const uint32_t *first = (const uint32_t *)ctx->d_counters.ptr;
+  if (k.counters < first || k.counters >= first + (size_t)ctx->out_slots * ctx->counter_words)
+    return fail(VGC_INVALID_ARG, "vgc_debug_retry_lost: the last cut was another context's, or its outputs have moved");
+  const size_t words = ((size_t)(noalloc ? kNoAllocMaxUnits : s.unit_capacity) * 4 + 31) / 32;
+  CUDA_TRY(cudaMemset(k.counters, 0, VGC_COUNTER_HEADER * 4));
+  CUDA_TRY(cudaMemset(overflow, 0xff, std::min<size_t>(units / 8, words) * 4));  // of the visible units alone
+  CUDA_TRY(launch_retry_probe(view, ctl, overflow, noalloc ? nullptr : s.h_ctl, (uint64_t)limit_us * 1000u, ctx->stream));
+  CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return VGC_OK;
 }

@@ -75,7 +75,8 @@ struct LaunchScratch {
   uint32_t chunk_capacity = 0;    // its entries
   size_t queue_uncharged = 0;     // bytes of it that the owner's HBM budget does not count
   uint32_t queue_want = 0;        // entries the last launch sequence asked for (grown to before the next one)
-  uint32_t *h_ctl = nullptr;      // pinned: control words 6 and 7 at the end of the last launch sequence; [8] it redid a cut
+  uint32_t *h_ctl = nullptr;      // pinned: control words 6 and 7 at the end of the last launch sequence; [8] it redid a cut,
+                                  //   [9] a wait of k_retry gave up in it
   uint32_t split_left = 0;        // launch sequences from now on whose retry rounds are kernels of their own (see enqueue)
   uint32_t grid_instances = 0;    // persistent grids of k_instances / k_chunks (0: the context's occupancy defaults)
   uint32_t grid_chunks = 0;

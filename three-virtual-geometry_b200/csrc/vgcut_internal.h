@@ -34,6 +34,7 @@ constexpr uint32_t kFullFadeBits = 255u << 16;
 constexpr uint32_t kLocalVertexBits = 7;   // ceil(log2(MAX_MESHLET_VERTICES = 128))
 constexpr uint32_t kMaxHzbLevels = 16;
 constexpr uint32_t kLaunchCtlWords = 64;  // control words of a launch sequence
+constexpr uint32_t kCtlGaveUp = 12;       // ... of which this one says that a wait of k_retry gave up
 constexpr uint32_t kRetryBlocks = 4;  // blocks of k_retry per SM
 constexpr uint32_t kStateWords = 8;        // S_SCALE 0..1, S_FILL 2..3, S_RETRY 4..5
 constexpr uint32_t kStatWords = 32;        // an output slot's mirror in pinned memory

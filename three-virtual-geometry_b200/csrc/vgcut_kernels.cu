@@ -1604,9 +1604,14 @@ __global__ void __launch_bounds__(128, kRetryBlocks) k_retry(Scene S0, const Sce
         __nanosleep(100);
         if ((polls & 31u) == 0 && global_ns() - t0 > limit_ns) {
           for (uint32_t v = 0; v < nviews; v++) {
-            const uint32_t fault = atomicOr(views[v].counters + VGC_COUNTER_ERROR, (uint32_t)VGC_FAULT_RETRY_WAIT);
-            if (views[v].host_stats) views[v].host_stats[VGC_COUNTER_ERROR] = fault | (uint32_t)VGC_FAULT_RETRY_WAIT;
+            atomicOr(views[v].counters + VGC_COUNTER_ERROR, (uint32_t)VGC_FAULT_RETRY_WAIT);
+            uint32_t *const host = views[v].host_stats;  // until now a view that has not settled has the cut before there
+            for (uint32_t i = 0; host && i < VGC_COUNTER_HEADER; i++) host[i] = __ldcg(views[v].counters + i);
+            if (host) host[VGC_COUNTER_HEADER] = __float_as_uint(views[v].dyn[0]);
           }
+          // overflow bits of the phases that did not run are still set: the next sequence clears them first
+          ctl[kCtlGaveUp] = 1;
+          if (host_ctl) host_ctl[9] = 1;
           now = 8;
           break;
         }
@@ -2412,8 +2417,8 @@ cudaError_t launch_hzb_views(const ViewConst *views, uint32_t nviews, uint32_t m
   return launch_after(false, k_hzb_tail_views, nviews, 1024, 0, st, views, kHzbTileLevels);
 }
 
-cudaError_t launch_retry_probe(const ViewConst *view, uint32_t *ctl, uint32_t *overflow, uint64_t limit_ns,
-                               cudaStream_t st) {
+cudaError_t launch_retry_probe(const ViewConst *view, uint32_t *ctl, uint32_t *overflow, uint32_t *host_ctl,
+                               uint64_t limit_ns, cudaStream_t st) {
   uint32_t words[kLaunchCtlWords] = {};
   words[1] = 1;               // a cut is to be redone
   words[kCtlPhase] = 3;       // round 1, finish
@@ -2422,7 +2427,7 @@ cudaError_t launch_retry_probe(const ViewConst *view, uint32_t *ctl, uint32_t *o
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return e;
   return launch_after(true, k_retry<false>, 8, 128, 0, st, Scene(), nullptr, view, 1u, nullptr, nullptr, ctl, nullptr, 0u,
-                      PassLimits(), overflow, nullptr, limit_ns);
+                      PassLimits(), overflow, host_ctl, limit_ns);
 }
 
 cudaError_t launch_wait_probe(uint64_t limit_ns, unsigned long long *out, cudaStream_t st) {

@@ -75,11 +75,11 @@ cudaError_t launch_hzb_views(const ViewConst *views, uint32_t nviews, uint32_t m
 // `grid` blocks (hzb_stream_blocks_per_sm() per SM), then the tail kernel for levels 5+ when `tail`.
 cudaError_t launch_hzb_stream(const unsigned char *plan, uint32_t grid, const ViewConst *views, uint32_t nviews,
                               bool tail, cudaStream_t st);
-// The bounded mbarrier wait of the strip stream on a barrier nothing completes (out[0]: completed, out[1]: ns waited).
 // k_retry of one view in the last phase of round 1, whose one piece is taken already: it waits for `limit_ns` and leaves a
-// fault in the view's counters. ctl (kLaunchCtlWords) and overflow are the probe's own.
-cudaError_t launch_retry_probe(const ViewConst *view, uint32_t *ctl, uint32_t *overflow, uint64_t limit_ns,
-                               cudaStream_t st);
+// fault in the view's counters. ctl (kLaunchCtlWords) is overwritten first.
+cudaError_t launch_retry_probe(const ViewConst *view, uint32_t *ctl, uint32_t *overflow, uint32_t *host_ctl,
+                               uint64_t limit_ns, cudaStream_t st);
+// The bounded mbarrier wait of the strip stream on a barrier nothing completes (out[0]: completed, out[1]: ns waited).
 cudaError_t launch_wait_probe(uint64_t limit_ns, unsigned long long *out, cudaStream_t st);
 // Blocks of k_hzb_stream resident per SM (sets its shared-memory limit on the first call for the current device).
 uint32_t hzb_stream_blocks_per_sm();
