@@ -1432,6 +1432,18 @@ int vgc_cut(vgc_context *ctx, const vgc_view *views, uint32_t count, uint32_t fi
   return VGC_OK;
 }
 
+static GraphKey graph_key(const vgc_context *ctx, const LaunchScratch &s, uint32_t count) {
+  const Scene S = scene_of(ctx);
+  const auto at = [](const void *p) { return (uint64_t)reinterpret_cast<uintptr_t>(p); };
+  return {at(S.meshes), at(S.levels), at(S.m_lod), at(S.m_parent), at(S.m_err), at(S.m_cull), at(S.m_info), at(S.m_tris),
+          at(S.lsamples), at(S.positions), at(S.m_verts), at(S.inst), at(S.inst_slot), at(S.cells), at(S.hzbs),
+          S.cell_count, S.instance_count, S.meshlet_count, S.slot_capacity, S.slots_used,
+          at(s.h_views), at(s.d_views), at(s.h_plan), at(s.d_plan), at(s.d_units), at(s.d_overflow), at(s.d_unit_count),
+          at(s.d_chunks), at(s.h_ctl), s.unit_capacity, s.chunk_capacity, s.units_total, count, s.hzb_w, s.hzb_h,
+          s.hzb_tail, s.any_budget, s.split_left != 0, s.grid_instances, s.grid_chunks, s.chunk_shift, s.chunk_tuned,
+          ctx->hzb_grid};
+}
+
 int vgc_batch_create(vgc_context *ctx, uint32_t max_views, vgc_batch **out) {
   if (!ctx || !out || max_views == 0) return fail(VGC_INVALID_ARG, "bad arguments");
   vgc_batch *b = new vgc_batch();
@@ -1453,13 +1465,8 @@ int vgc_batch_run(vgc_batch *b, const vgc_view *views, uint32_t count, uint32_t 
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   int rc = prepare(ctx, b->scratch, views, count, first_slot);
   if (rc) return rc;
-  const uint32_t cells = (uint32_t)ctx->cells.size();
-  if (!b->exec || b->graph_views != count || b->graph_cells != cells || b->graph_slots != ctx->slot_capacity ||
-      b->graph_hzb_w != b->scratch.hzb_w || b->graph_hzb_h != b->scratch.hzb_h || b->graph_hzb_tail != b->scratch.hzb_tail ||
-      b->graph_split != (b->scratch.split_left != 0) ||
-      b->graph_budget != b->scratch.any_budget || b->graph_queue != b->scratch.d_chunks ||
-      b->graph_grids[0] != b->scratch.grid_instances || b->graph_grids[1] != b->scratch.grid_chunks ||
-      b->graph_chunk_shift != b->scratch.chunk_shift || b->graph_chunk_tuned != b->scratch.chunk_tuned) {
+  const GraphKey key = graph_key(ctx, b->scratch, count);
+  if (!b->exec || b->graph_key != key) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     b->exec = nullptr;
@@ -1475,19 +1482,7 @@ int vgc_batch_run(vgc_batch *b, const vgc_view *views, uint32_t count, uint32_t 
     if (e != cudaSuccess) return fail(VGC_DEVICE_ERROR, std::string("graph capture: ") + cudaGetErrorString(e));
     b->graph = g;
     CUDA_TRY(cudaGraphInstantiate(&b->exec, b->graph, 0));
-    b->graph_views = count;
-    b->graph_cells = cells;
-    b->graph_slots = ctx->slot_capacity;
-    b->graph_hzb_w = b->scratch.hzb_w;
-    b->graph_hzb_h = b->scratch.hzb_h;
-    b->graph_hzb_tail = b->scratch.hzb_tail;
-    b->graph_split = b->scratch.split_left != 0;
-    b->graph_budget = b->scratch.any_budget;
-    b->graph_queue = b->scratch.d_chunks;
-    b->graph_grids[0] = b->scratch.grid_instances;
-    b->graph_grids[1] = b->scratch.grid_chunks;
-    b->graph_chunk_shift = b->scratch.chunk_shift;
-    b->graph_chunk_tuned = b->scratch.chunk_tuned;
+    b->graph_key = key;
   }
   cut_on(ctx, first_slot, count, st);
   CUDA_TRY(cudaGraphLaunch(b->exec, st));

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <array>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -163,6 +164,10 @@ struct vgc_context {
   uint32_t prof_count[VGC_KERNEL_KINDS] = {0};
 };
 
+// What a captured launch sequence holds by value besides its views' constants: the scene's and the scratch's arrays and
+// sizes and the launches' shapes. A graph is replayed while its key is the scratch's.
+using GraphKey = std::array<uint64_t, 43>;
+
 struct vgc_batch {
   vgc_context *ctx = nullptr;
   uint32_t max_views = 0;
@@ -170,17 +175,7 @@ struct vgc_batch {
   cudaStream_t capture_stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  uint32_t graph_views = 0;
-  uint32_t graph_cells = 0;
-  uint32_t graph_slots = 0;
-  uint32_t graph_hzb_w = 0, graph_hzb_h = 0;
-  bool graph_hzb_tail = false;
-  bool graph_split = false;
-  bool graph_budget = false;
-  const uint4 *graph_queue = nullptr;  // work queue the graph was captured with
-  uint32_t graph_grids[2] = {0, 0};    // persistent grids the graph was captured with
-  uint32_t graph_chunk_shift = 0;      // chunk size it was captured with
-  bool graph_chunk_tuned = false;
+  GraphKey graph_key{};
 };
 
 namespace vgch {
