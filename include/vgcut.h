@@ -417,6 +417,9 @@ int vgc_debug_retry_probe(vgc_context *ctx, uint32_t limit_us, uint32_t *faults)
    view's counters cleared, the visible units marked as still to be tested in place, then the wait of `limit_us` that
    runs out. Its counters, faults among them, and later cuts can then be looked at. Synchronous. */
 int vgc_debug_retry_lost(vgc_context *ctx, int noalloc, uint32_t limit_us);
+/* How often the batch has captured its launch sequence: with the retry rounds in one kernel, and as kernels of their
+   own. */
+int vgc_debug_batch_captures(const vgc_batch *batch, uint32_t captures[2]);
 
 #ifdef __cplusplus
 }

@@ -1350,6 +1350,12 @@ int vgc_debug_retry_probe(vgc_context *ctx, uint32_t limit_us, uint32_t *faults)
   return VGC_OK;
 }
 
+int vgc_debug_batch_captures(const vgc_batch *b, uint32_t captures[2]) {
+  if (!b || !captures) return fail(VGC_INVALID_ARG, "null argument");
+  for (int i = 0; i < 2; i++) captures[i] = b->forms[i].captures;
+  return VGC_OK;
+}
+
 int vgc_debug_cells_device(vgc_context *ctx, float *cells, uint32_t capacity, uint32_t *count) {
   if (!ctx || !count) return fail(VGC_INVALID_ARG, "null argument");
   int rc = sync_scene(ctx);
@@ -1440,7 +1446,7 @@ static GraphKey graph_key(const vgc_context *ctx, const LaunchScratch &s, uint32
           S.cell_count, S.instance_count, S.meshlet_count, S.slot_capacity, S.slots_used,
           at(s.h_views), at(s.d_views), at(s.h_plan), at(s.d_plan), at(s.d_units), at(s.d_overflow), at(s.d_unit_count),
           at(s.d_chunks), at(s.h_ctl), s.unit_capacity, s.chunk_capacity, s.units_total, count, s.hzb_w, s.hzb_h,
-          s.hzb_tail, s.any_budget, s.split_left != 0, s.grid_instances, s.grid_chunks, s.chunk_shift, s.chunk_tuned,
+          s.hzb_tail, s.any_budget, s.grid_instances, s.grid_chunks, s.chunk_shift, s.chunk_tuned,
           ctx->hzb_grid};
 }
 
@@ -1466,11 +1472,12 @@ int vgc_batch_run(vgc_batch *b, const vgc_view *views, uint32_t count, uint32_t 
   int rc = prepare(ctx, b->scratch, views, count, first_slot);
   if (rc) return rc;
   const GraphKey key = graph_key(ctx, b->scratch, count);
-  if (!b->exec || b->graph_key != key) {
-    if (b->exec) cudaGraphExecDestroy(b->exec);
-    if (b->graph) cudaGraphDestroy(b->graph);
-    b->exec = nullptr;
-    b->graph = nullptr;
+  vgc_batch::Form &f = b->form();
+  if (!f.exec || f.key != key) {
+    if (f.exec) cudaGraphExecDestroy(f.exec);
+    if (f.graph) cudaGraphDestroy(f.graph);
+    f.exec = nullptr;
+    f.graph = nullptr;
     CUDA_TRY(cudaStreamBeginCapture(b->capture_stream, cudaStreamCaptureModeThreadLocal));
     rc = enqueue(ctx, b->scratch, count, b->capture_stream, true);
     cudaGraph_t g = nullptr;
@@ -1480,12 +1487,13 @@ int vgc_batch_run(vgc_batch *b, const vgc_view *views, uint32_t count, uint32_t 
       return rc;
     }
     if (e != cudaSuccess) return fail(VGC_DEVICE_ERROR, std::string("graph capture: ") + cudaGetErrorString(e));
-    b->graph = g;
-    CUDA_TRY(cudaGraphInstantiate(&b->exec, b->graph, 0));
-    b->graph_key = key;
+    f.graph = g;
+    CUDA_TRY(cudaGraphInstantiate(&f.exec, f.graph, 0));
+    f.key = key;
+    f.captures++;
   }
   cut_on(ctx, first_slot, count, st);
-  CUDA_TRY(cudaGraphLaunch(b->exec, st));
+  CUDA_TRY(cudaGraphLaunch(f.exec, st));
   CUDA_TRY(cudaEventRecord(b->scratch.done, st));
   b->scratch.pending = true;
   return VGC_OK;
@@ -1525,7 +1533,7 @@ int vgc_batch_autotune(vgc_batch *b, const vgc_view *views, uint32_t count, uint
       std::vector<float> ms;
       for (uint32_t r = 0; r < reps; r++) {  // replays of the captured graph: device time only
         cudaEventRecord(e0, st);
-        cudaGraphLaunch(b->exec, st);
+        cudaGraphLaunch(b->form().exec, st);
         cudaEventRecord(e1, st);
         if (cudaEventSynchronize(e1) != cudaSuccess) {
           rc = fail(VGC_DEVICE_ERROR, "autotune replay failed");
@@ -1571,8 +1579,10 @@ int vgc_batch_destroy(vgc_batch *b) {
   if (!b) return VGC_OK;
   cudaSetDevice(b->ctx->device);
   if (b->scratch.pending) cudaEventSynchronize(b->scratch.done);
-  if (b->exec) cudaGraphExecDestroy(b->exec);
-  if (b->graph) cudaGraphDestroy(b->graph);
+  for (vgc_batch::Form &f : b->forms) {
+    if (f.exec) cudaGraphExecDestroy(f.exec);
+    if (f.graph) cudaGraphDestroy(f.graph);
+  }
   if (b->capture_stream) cudaStreamDestroy(b->capture_stream);
   if (b->scratch.d_views)
     b->ctx->bytes -= sizeof(ViewConst) * b->scratch.view_capacity + hzb_plan_bytes(b->scratch.view_capacity);

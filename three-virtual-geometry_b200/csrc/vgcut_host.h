@@ -166,16 +166,22 @@ struct vgc_context {
 
 // What a captured launch sequence holds by value besides its views' constants: the scene's and the scratch's arrays and
 // sizes and the launches' shapes. A graph is replayed while its key is the scratch's.
-using GraphKey = std::array<uint64_t, 43>;
+using GraphKey = std::array<uint64_t, 42>;
 
 struct vgc_batch {
   vgc_context *ctx = nullptr;
   uint32_t max_views = 0;
   LaunchScratch scratch;
   cudaStream_t capture_stream = nullptr;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  GraphKey graph_key{};
+  // one graph for each form of the retry rounds (LaunchScratch::split_left), which a batch may go back and forth between:
+  // capturing and instantiating one takes about 200 us
+  struct Form {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    GraphKey key{};
+    uint32_t captures = 0;
+  } forms[2];
+  Form &form() { return forms[scratch.split_left ? 1 : 0]; }
 };
 
 namespace vgch {

@@ -155,6 +155,7 @@ def lib() -> C.CDLL:
         "vgc_debug_cells_device": ([vp, P(C.c_float), C.c_uint32, P(C.c_uint32)], C.c_int),
         "vgc_debug_retry_probe": ([vp, C.c_uint32, P(C.c_uint32)], C.c_int),
         "vgc_debug_retry_lost": ([vp, C.c_int, C.c_uint32], C.c_int),
+        "vgc_debug_batch_captures": ([vp, C.c_uint32 * 2], C.c_int),
         "vgc_debug_wait_probe": ([vp, C.c_uint32, P(C.c_uint32), P(C.c_uint64)], C.c_int),
         "vgc_occluder_depth": ([vp, C.c_uint32, P(View), vp, C.c_uint32, C.c_uint32, vp], C.c_int),
         "vgc_occluder_depth_batch": ([vp, C.c_uint32, P(C.c_uint32), P(View), P(vp), C.c_uint32, C.c_uint32, vp],
