@@ -24,8 +24,8 @@ def test_forms_are_captured_once():
     cam = Camera.perspective_look_at((-6.0, 5.0, -6.0), (60.0, 0.0, 60.0), 60, 1920, 1080, 0.1, 5000.0)
 
     def views(t):
-        return [engine.make_view(cam, engine.ViewParams(error_threshold=t * k, fresh_state=True, frustum_culling=False))
-                for k in (1.0, 2.0, 3.0)]
+        return [engine.make_view(cam, engine.ViewParams(error_threshold=t * (1 + k), fresh_state=True, state_slot=k,
+                                                        frustum_culling=False)) for k in range(3)]
 
     def read():
         return [(vg.read_stats(k)["rounds"], vg.read_stats(k)["selected"], key_set(vg.draw_list(k, 0), (0, 1, 3)))

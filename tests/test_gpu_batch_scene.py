@@ -16,7 +16,8 @@ def test_graph_follows_moved_arrays():
     cam = Camera.perspective_look_at((-6.0, 5.0, -6.0), (40.0, 0.0, 40.0), 60, 1920, 1080, 0.1, 5000.0)
 
     def views():
-        return [engine.make_view(cam, engine.ViewParams(error_threshold=t, fresh_state=True)) for t in (0.5, 4.0)]
+        return [engine.make_view(cam, engine.ViewParams(error_threshold=t, fresh_state=True, state_slot=k))
+                for k, t in enumerate((0.5, 4.0))]
 
     def read():
         out = []
