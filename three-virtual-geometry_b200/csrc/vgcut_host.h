@@ -82,7 +82,7 @@ struct LaunchScratch {
   uint32_t grid_instances = 0;    // persistent grids of k_instances / k_chunks (0: the context's occupancy defaults)
   uint32_t grid_chunks = 0;
   uint32_t chunk_shift = kChunkShiftDefault;  // 2^chunk_shift meshlets per k_chunks work unit at most,
-  bool chunk_tuned = false;                   //   or exactly (autotuned or set by the caller)
+  bool chunk_tuned = false;                   //   or exactly (set_chunks)
   uint32_t view_capacity = 0;
   size_t unit_capacity = 0;
   size_t units_total = 0;         // (view, cell) units of the prepared launch (each view: its scene's cells, padded)

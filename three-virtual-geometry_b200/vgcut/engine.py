@@ -481,7 +481,8 @@ class VirtualGeometry:
     def set_tuning(self, count: int, instances_blocks_per_sm: int = 0, chunks_blocks_per_sm: int = 0,
                    chunk_meshlets: int = 512) -> None:
         """Applies a tuning to the batched launch of `count` views (vgc_batch_set_tuning): blocks per SM of the
-        instance and meshlet kernels (0: occupancy default) and meshlets per chunk (256, 512 or 1024)."""
+        instance and meshlet kernels (0: occupancy default) and meshlets per chunk (256, 1024, or 512: the default, up to
+        512, fewer where a launch has few visible units). The defaults give back the shape of an untuned batch."""
         b = self._batches.get(count)
         if b is None:
             b = C.c_void_p()
