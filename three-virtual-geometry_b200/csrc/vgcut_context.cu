@@ -1530,13 +1530,18 @@ int vgc_batch_autotune(vgc_batch *b, const vgc_view *views, uint32_t count, uint
   CUDA_TRY(cudaEventCreate(&e1));
   reps = std::max(1u, reps);
   vgc_tune_result top{0, 0, INFINITY, 0};
-  int rc = VGC_OK;
+  // whether the views' cuts are redone decides the form of the retry rounds, and every candidate is timed in that form
+  LaunchScratch &s = b->scratch;
+  int rc = vgc_batch_run(b, views, count, first_slot, stream);
+  if (!rc) rc = after_last(s);
+  const bool split = s.split_left != 0;
   for (uint32_t shift = kChunkShiftMin; shift <= kChunkShiftMax && !rc; shift++)
   for (uint32_t bi : steps(max_i)) {
     for (uint32_t bc : steps(max_c)) {
-      b->scratch.grid_instances = bi * sms;
-      b->scratch.grid_chunks = bc * sms;
-      set_chunks(b->scratch, shift);
+      s.grid_instances = bi * sms;
+      s.grid_chunks = bc * sms;
+      set_chunks(s, shift);
+      s.h_ctl[8] = split, s.split_left = 0;
       if ((rc = vgc_batch_run(b, views, count, first_slot, stream))) break;  // capture + warm-up
       std::vector<float> ms;
       for (uint32_t r = 0; r < reps; r++) {  // replays of the captured graph: device time only
@@ -1561,9 +1566,9 @@ int vgc_batch_autotune(vgc_batch *b, const vgc_view *views, uint32_t count, uint
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc) return rc;
-  b->scratch.grid_instances = top.instances_blocks_per_sm * sms;
-  b->scratch.grid_chunks = top.chunks_blocks_per_sm * sms;
-  set_chunks(b->scratch, (uint32_t)__builtin_ctz(top.chunk_meshlets));
+  s.grid_instances = top.instances_blocks_per_sm * sms;
+  s.grid_chunks = top.chunks_blocks_per_sm * sms;
+  set_chunks(s, (uint32_t)__builtin_ctz(top.chunk_meshlets));
   *best = top;
   return VGC_OK;
 }
