@@ -46,7 +46,10 @@ typedef struct vgc_options {
   uint32_t max_meshlets;         /* draw-list capacity per cut per view (reference default 1 << 20) */
   uint32_t output_slots;         /* views whose outputs can be resident at once (batch width), default 1 */
   int32_t device;                /* CUDA device ordinal */
-  uint64_t hbm_budget_bytes;     /* admission limit for this context's allocations; 0 = no limit */
+  uint64_t hbm_budget_bytes;     /* admission limit for this context's allocations; 0 = no limit. With a limit the
+                                    context does without what it else takes for speed beyond its needs: three quarters
+                                    of the raster queue, work queues of 256k entries for launches of few views (64k a
+                                    view then), and selectCut's kept workspace where another allocation needs the room */
 } vgc_options;
 
 /* The part of VirtualMeshData (buildVirtualMesh.ts:75-138) that the cut reads. */
@@ -332,8 +335,8 @@ int vgc_server_destroy(vgc_server *server);
    sampled at pixel centres. A triangle crossing the near plane (clip z = 0) is clipped in clip space into one or two
    triangles (crossing points interpolated from the corner in front, at depth 0), as a GPU's clipper does; wholly
    behind it, it is not drawn. Pass `depth` as this frame's vgc_view.depth to build the HZB from it in the cut's own
-   launch sequence. The first call allocates the context's triangle queues (about 54 MB, shared with
-   vgc_visibility; up to 131,072 near-plane-crossing triangles a call are clipped, more are left out); calls on one
+   launch sequence. The first call allocates the context's triangle queues (56 MB, or 182 MB without an HBM
+   budget and where the device has the room; shared with vgc_visibility; up to 131,072 near-plane-crossing triangles a call are clipped, more are left out); calls on one
    context whose GPU work overlaps (different streams) race on them: order them on one stream. Asynchronous on
    `stream`. */
 int vgc_occluder_depth(vgc_context *ctx, uint32_t src_slot, const vgc_view *view, float *depth, uint32_t width,

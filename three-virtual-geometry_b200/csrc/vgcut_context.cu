@@ -62,46 +62,35 @@ constexpr double kNoDrawDistance = 1e30;  // GeometryPool.ts:111
 
 namespace vgch {
 
-// Gives the kept selectCut workspace back (its calls are synchronous, so nothing uses it).
-static void free_select(vgc_context *ctx) {
-  if (ctx->d_select.ptr) {
-    cudaFree(ctx->d_select.ptr);
-    ctx->bytes -= ctx->d_select.bytes;
-    ctx->uncharged -= ctx->d_select.bytes;
-  }
-  ctx->d_select = DevBuf();
+static bool over_budget(const vgc_context *ctx, size_t more) {
+  return ctx->opts.hbm_budget_bytes && ctx->bytes + more > ctx->opts.hbm_budget_bytes;
 }
 
 // The kept workspace: a device buffer for `bytes` at least (at most kSelectKeep), and the pinned pieces its results
-// come back through. Not charged to the context's HBM budget, and given back when the device runs out of memory.
+// come back through; false when the HBM budget or the device has no room for it. Given back when another allocation needs
+// the room (dev_alloc; a selectCut is synchronous, so nothing uses it then).
 // Pinned memory costs 1.2 ms for the first 2 MB and 0.4 ms for each further MB, which a context's first call pays: so
 // results pass through kSelectPieces small pieces instead of a buffer of their size.
 constexpr size_t kSelectKeep = 32u << 20;
 constexpr size_t kSelectPiece = 256u << 10;
-static int select_workspace(vgc_context *ctx, size_t bytes) {
+static bool select_workspace(vgc_context *ctx, size_t bytes) {
   cudaError_t e = cudaSuccess;
   if (ctx->d_select.bytes < bytes) {
-    free_select(ctx);
+    dev_free(ctx, ctx->d_select);
     size_t want = size_t(1) << 20;
     while (want < bytes) want *= 2;
+    if (over_budget(ctx, want)) return false;
     e = cudaMalloc(&ctx->d_select.ptr, want);
-    if (e == cudaSuccess) {
-      ctx->d_select.bytes = want;
-      ctx->bytes += want;
-      ctx->uncharged += want;
-    } else {
-      ctx->d_select.ptr = nullptr;
-    }
+    if (e == cudaSuccess) ctx->d_select.bytes = want, ctx->bytes += want;
+    else ctx->d_select.ptr = nullptr;
   }
   if (e == cudaSuccess && !ctx->h_select) e = cudaMallocHost(&ctx->h_select, kSelectPieces * kSelectPiece);
   for (uint32_t i = 0; i < kSelectPieces && e == cudaSuccess; i++)
     if (!ctx->select_piece[i]) e = cudaEventCreateWithFlags(&ctx->select_piece[i], cudaEventDisableTiming);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    free_select(ctx);
-    return fail(VGC_DEVICE_ERROR, std::string("select_cut: ") + cudaGetErrorString(e));
-  }
-  return VGC_OK;
+  if (e == cudaSuccess) return true;
+  cudaGetLastError();
+  dev_free(ctx, ctx->d_select);
+  return false;
 }
 
 // `bytes` of a select call's results from `src` to lo and, from byte `half` on, hi, through the pinned pieces: while
@@ -128,18 +117,24 @@ static cudaError_t select_results(vgc_context *ctx, const uint8_t *src, size_t h
   return e;
 }
 
+// cudaMalloc, with the kept selectCut workspace's room if the device has no other.
+template <class T>
+static cudaError_t device_malloc(vgc_context *ctx, T **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation || !ctx->d_select.ptr) return e;
+  cudaGetLastError();
+  dev_free(ctx, ctx->d_select);
+  return cudaMalloc(p, bytes);
+}
+
 int dev_alloc(vgc_context *ctx, DevBuf &b, size_t bytes) {
   if (b.bytes >= bytes && b.ptr) return VGC_OK;
   size_t want = std::max<size_t>(bytes, 256);
-  if (ctx->opts.hbm_budget_bytes && ctx->bytes - ctx->uncharged - b.bytes + want > ctx->opts.hbm_budget_bytes)
+  if (over_budget(ctx, want - b.bytes)) dev_free(ctx, ctx->d_select);
+  if (over_budget(ctx, want - b.bytes))
     return fail(VGC_OVER_BUDGET, "allocation of " + std::to_string(want) + " bytes exceeds the context's HBM budget");
   void *p = nullptr;
-  cudaError_t e = cudaMalloc(&p, want);
-  if (e == cudaErrorMemoryAllocation && ctx->d_select.ptr) {
-    cudaGetLastError();
-    free_select(ctx);
-    e = cudaMalloc(&p, want);
-  }
+  const cudaError_t e = device_malloc(ctx, &p, want);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(VGC_OOM, "cudaMalloc(" + std::to_string(want) + "): " + cudaGetErrorString(e));
@@ -345,9 +340,9 @@ int ensure_scratch(vgc_context *ctx, LaunchScratch &s, uint32_t views, size_t un
     s.h_plan = s.d_plan = nullptr;
     s.view_capacity = 0;
     CUDA_TRY(cudaMallocHost(&s.h_views, sizeof(ViewConst) * views));
-    CUDA_TRY(cudaMalloc(&s.d_views, sizeof(ViewConst) * views));
+    CUDA_TRY(device_malloc(ctx, &s.d_views, sizeof(ViewConst) * views));
     CUDA_TRY(cudaMallocHost(&s.h_plan, hzb_plan_bytes(views)));
-    CUDA_TRY(cudaMalloc(&s.d_plan, hzb_plan_bytes(views)));
+    CUDA_TRY(device_malloc(ctx, &s.d_plan, hzb_plan_bytes(views)));
     ctx->bytes += sizeof(ViewConst) * views + hzb_plan_bytes(views);
     s.plan_keys.assign(views, LaunchScratch::PlanKey{});
     s.plan_maps = 0;
@@ -361,32 +356,28 @@ int ensure_scratch(vgc_context *ctx, LaunchScratch &s, uint32_t views, size_t un
     s.d_units = nullptr;
     s.d_overflow = nullptr;
     size_t n = std::max<size_t>(units, 32);
-    CUDA_TRY(cudaMalloc(&s.d_units, unit_bytes(n)));
+    CUDA_TRY(device_malloc(ctx, &s.d_units, unit_bytes(n)));
     s.d_overflow = reinterpret_cast<uint32_t *>(s.d_units + n);
     CUDA_TRY(cudaMemset(s.d_overflow, 0, overflow_bytes(n)));
     ctx->bytes += unit_bytes(n);
     s.unit_capacity = n;
   }
-  if (!s.d_unit_count) CUDA_TRY(cudaMalloc(&s.d_unit_count, kLaunchCtlWords * 4));
+  if (!s.d_unit_count) CUDA_TRY(device_malloc(ctx, &s.d_unit_count, kLaunchCtlWords * 4));
   // meshlet work queue: about one span per instance with a level range and cut, one chunk per 512 meshlets of a
-  // warp's items (fewer in a launch of few views: pass_shape). Sized for 64k entries per view, 256k at least; a warp that cannot reserve tests its items itself, so a full
-  // queue costs time, not correctness.
-  const uint32_t want_chunks = std::max<uint32_t>(std::max<uint32_t>(kQueueMin, views * 65536u), s.queue_want);
+  // warp's items (fewer in a launch of few views: pass_shape). Sized for 64k entries per view, and for the small chunks of
+  // a launch of few views 256k at least, which a context with an HBM budget does without; a warp that cannot reserve
+  // tests its items itself, so a full queue costs time, not correctness.
+  const uint32_t least = ctx->opts.hbm_budget_bytes ? 65536 : kQueueMin;
+  const uint32_t want_chunks = std::max<uint32_t>(std::max<uint32_t>(least, views * 65536u), s.queue_want);
   if (want_chunks > s.chunk_capacity) {
-    // what a launch of few views gets above 64k entries a view serves its small chunks and is not charged to the budget
-    const uint32_t charged = std::max<uint32_t>(std::max<uint32_t>(65536, views * 65536u), s.queue_want);
     if (s.d_chunks) {
       cudaFree(s.d_chunks);
       ctx->bytes -= (size_t)s.chunk_capacity * sizeof(uint4);
-      ctx->uncharged -= s.queue_uncharged;
     }
     s.d_chunks = nullptr;
-    s.queue_uncharged = 0;
     s.chunk_capacity = 0;
-    CUDA_TRY(cudaMalloc(&s.d_chunks, (size_t)want_chunks * sizeof(uint4)));
+    CUDA_TRY(device_malloc(ctx, &s.d_chunks, (size_t)want_chunks * sizeof(uint4)));
     ctx->bytes += (size_t)want_chunks * sizeof(uint4);
-    s.queue_uncharged = (size_t)(want_chunks - charged) * sizeof(uint4);
-    ctx->uncharged += s.queue_uncharged;
     s.chunk_capacity = want_chunks;
   }
   if (!s.done) CUDA_TRY(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
@@ -1075,13 +1066,12 @@ int vgc_context_destroy(vgc_context *ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   free_scratch(ctx->scratch);
   for (DevBuf *b : {&ctx->d_meshes, &ctx->d_levels, &ctx->d_m_lod, &ctx->d_m_parent, &ctx->d_m_err, &ctx->d_m_cull,
-                    &ctx->d_lsamples, &ctx->d_positions, &ctx->d_m_verts, &ctx->d_raster, &ctx->d_resort,
+                    &ctx->d_lsamples, &ctx->d_positions, &ctx->d_m_verts, &ctx->d_raster, &ctx->d_resort, &ctx->d_select,
                     &ctx->d_m_info, &ctx->d_m_tris, &ctx->d_inst, &ctx->d_inst_slot, &ctx->d_cells, &ctx->d_counters,
                     &ctx->d_draw, &ctx->d_args, &ctx->d_dyn, &ctx->d_hist, &ctx->d_state, &ctx->d_hzb_desc})
     dev_free(ctx, *b);
   for (auto &h : ctx->hzb) dev_free(ctx, h.data);
   if (ctx->h_stats) cudaFreeHost(ctx->h_stats);
-  free_select(ctx);
   if (ctx->h_select) cudaFreeHost(ctx->h_select);
   for (cudaEvent_t &ev : ctx->select_piece)
     if (ev) cudaEventDestroy(ev);
@@ -1599,8 +1589,6 @@ int vgc_batch_destroy(vgc_batch *b) {
   if (b->scratch.d_views)
     b->ctx->bytes -= sizeof(ViewConst) * b->scratch.view_capacity + hzb_plan_bytes(b->scratch.view_capacity);
   if (b->scratch.d_units) b->ctx->bytes -= unit_bytes(b->scratch.unit_capacity);
-  b->ctx->bytes -= b->scratch.queue_uncharged;
-  b->ctx->uncharged -= b->scratch.queue_uncharged;
   free_scratch(b->scratch);
   delete b;
   return VGC_OK;
@@ -1709,14 +1697,9 @@ int vgc_select_cut(vgc_context *ctx, uint32_t slot, uint32_t count, const double
   // cudaFree took most of such a call) and its pinned pieces.
   const size_t outn = (size_t)count * mcount, in_bytes = ((m.size() + p.size()) * 4 + 255) & ~size_t(255);
   const size_t total = in_bytes + outn * 2;
-  const bool kept = total <= kSelectKeep;
-  void *d = nullptr;
-  if (kept) {
-    if ((rc = select_workspace(ctx, total))) return rc;
-    d = ctx->d_select.ptr;
-  } else {
-    CUDA_TRY(cudaMalloc(&d, total));
-  }
+  const bool kept = total <= kSelectKeep && select_workspace(ctx, total);
+  void *d = ctx->d_select.ptr;
+  if (!kept) CUDA_TRY(cudaMalloc(&d, total));
   float *dm = (float *)d, *dp = dm + m.size();
   uint8_t *dlo = (uint8_t *)d + in_bytes, *dhi = dlo + outn;
   cudaStream_t st = ctx->stream;

@@ -50,7 +50,7 @@ struct HzbSlot {
 
 constexpr uint32_t kSelectPieces = 4;   // pinned pieces a selectCut's results come back through
 constexpr uint32_t kSplitLaunches = 64;  // after one that redid a cut, launch sequences with the retry rounds' own kernels
-constexpr uint32_t kQueueMin = 262144;  // entries of the smallest meshlet work queue
+constexpr uint32_t kQueueMin = 262144;  // entries of the smallest meshlet work queue of a context without an HBM budget
 
 // slot_stream of a slot whose cut a stream captured: it runs wherever its graph is replayed, which no call here sees
 inline const cudaStream_t kReplayed = cudaStreamLegacy;
@@ -74,7 +74,6 @@ struct LaunchScratch {
   uint32_t *d_unit_count = nullptr;  // control words (see launch_reset)
   uint4 *d_chunks = nullptr;      // meshlet work queue (spans and chunks)
   uint32_t chunk_capacity = 0;    // its entries
-  size_t queue_uncharged = 0;     // bytes of it that the owner's HBM budget does not count
   uint32_t queue_want = 0;        // entries the last launch sequence asked for (grown to before the next one)
   uint32_t *h_ctl = nullptr;      // pinned: control words 6 and 7 at the end of the last launch sequence; [8] it redid a cut,
                                   //   [9] a wait of k_retry gave up in it
@@ -115,7 +114,6 @@ struct vgc_context {
   uint32_t chunk_grid = 0;   // persistent grid of k_chunks
   uint32_t hzb_grid = 0;     // persistent grid of k_hzb_stream (0: the per-view tile kernel instead)
   uint64_t bytes = 0;
-  uint64_t uncharged = 0;  // of `bytes`: workspaces that the HBM budget does not count
   std::mutex mu;
   // host mirrors of the resident scene
   std::vector<MeshHost> mesh_host;

@@ -44,7 +44,7 @@ constexpr uint32_t kLaneRasterMax = 32;
 constexpr uint32_t kWarpRasterMax = 1024;   // ... by one warp of the second kernel; beyond, as tiles
 constexpr uint32_t kTileW = 32, kTileH = 16;
 // Queue capacities: medium triangles in sub-queues (record i of sub-queue q at i * kSubQueues + q), 160 MB of them, a
-// quarter of that where the device has no room for more. What the queue does not hold is drawn by the warp that set it
+// quarter of that in a context with an HBM budget and where the device has no room for more. What the queue does not hold is drawn by the warp that set it
 // up, long after the others have finished: 1080p visibility buffers of near geometry 2.40 -> 1.30 ms, 32 two-pass images
 // of 960x540 2.06 -> 1.45 ms a step, against a quarter of the records.
 constexpr uint32_t kQueuedMedium = 5u << 19, kQueuedMediumMin = 5u << 17;
@@ -887,12 +887,8 @@ static int raster_queues(vgc_context *ctx, RasterArgs &R) {
   static_assert(kCtlWords * 4 <= ctl_bytes, "control words");
   const size_t rest = ctl_bytes + large_bytes + tile_bytes + clip_bytes, record = kRecord * 16;
   if (!ctx->d_raster.ptr) {
-    // the records above the smaller queue's are not charged to the context's HBM budget
-    const size_t extra = (size_t)(kQueuedMedium - kQueuedMediumMin) * record;
-    ctx->uncharged += extra;
-    int rc = dev_alloc(ctx, ctx->d_raster, rest + kQueuedMedium * record);
-    if (rc) ctx->uncharged -= extra;
-    if (rc == VGC_OOM) rc = dev_alloc(ctx, ctx->d_raster, rest + kQueuedMediumMin * record);
+    int rc = ctx->opts.hbm_budget_bytes ? VGC_OVER_BUDGET : dev_alloc(ctx, ctx->d_raster, rest + kQueuedMedium * record);
+    if (rc == VGC_OVER_BUDGET || rc == VGC_OOM) rc = dev_alloc(ctx, ctx->d_raster, rest + kQueuedMediumMin * record);
     if (rc) return rc;
   }
   char *q = (char *)ctx->d_raster.ptr;
