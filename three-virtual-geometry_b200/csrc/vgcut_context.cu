@@ -63,7 +63,7 @@ constexpr double kNoDrawDistance = 1e30;  // GeometryPool.ts:111
 namespace vgch {
 
 static bool over_budget(const vgc_context *ctx, size_t more) {
-  return ctx->opts.hbm_budget_bytes && ctx->bytes + more > ctx->opts.hbm_budget_bytes;
+  return ctx->opts.hbm_budget_bytes && ctx->bytes + *ctx->scratch_bytes + more > ctx->opts.hbm_budget_bytes;
 }
 
 // The kept workspace: a device buffer for `bytes` at least (at most kSelectKeep), and the pinned pieces its results
@@ -321,19 +321,25 @@ int ensure_state(vgc_context *ctx, uint32_t slot) {
 static size_t overflow_bytes(size_t n) { return (n * 4 + 31) / 32 * sizeof(uint32_t); }
 static size_t unit_bytes(size_t n) { return n * sizeof(uint2) + overflow_bytes(n); }
 
+// Counts `more` bytes of a scratch (or fewer) against the context it belongs to.
+static void charge(LaunchScratch &s, int64_t more) {
+  *s.account += more;
+  s.charged += more;
+}
+
 int ensure_scratch(vgc_context *ctx, LaunchScratch &s, uint32_t views, size_t units) {
-  if (!s.owner) s.owner = ctx;  // growth below is counted where the scratch was first counted
+  if (!s.owner) s.owner = ctx, s.account = ctx->scratch_bytes;  // all of it is counted where it was first
   ctx = s.owner;
   if (views > s.view_capacity) {
     if (s.h_views) cudaFreeHost(s.h_views);
     if (s.d_views) {
       cudaFree(s.d_views);
-      ctx->bytes -= sizeof(ViewConst) * s.view_capacity;
+      charge(s, -(int64_t)(sizeof(ViewConst) * s.view_capacity));
     }
     if (s.h_plan) cudaFreeHost(s.h_plan);
     if (s.d_plan) {
       cudaFree(s.d_plan);
-      ctx->bytes -= hzb_plan_bytes(s.view_capacity);
+      charge(s, -(int64_t)hzb_plan_bytes(s.view_capacity));
     }
     s.h_views = nullptr;
     s.d_views = nullptr;
@@ -343,7 +349,7 @@ int ensure_scratch(vgc_context *ctx, LaunchScratch &s, uint32_t views, size_t un
     CUDA_TRY(device_malloc(ctx, &s.d_views, sizeof(ViewConst) * views));
     CUDA_TRY(cudaMallocHost(&s.h_plan, hzb_plan_bytes(views)));
     CUDA_TRY(device_malloc(ctx, &s.d_plan, hzb_plan_bytes(views)));
-    ctx->bytes += sizeof(ViewConst) * views + hzb_plan_bytes(views);
+    charge(s, sizeof(ViewConst) * views + hzb_plan_bytes(views));
     s.plan_keys.assign(views, LaunchScratch::PlanKey{});
     s.plan_maps = 0;
     s.view_capacity = views;
@@ -351,7 +357,7 @@ int ensure_scratch(vgc_context *ctx, LaunchScratch &s, uint32_t views, size_t un
   if (units > s.unit_capacity || !s.d_units) {
     if (s.d_units) {
       cudaFree(s.d_units);
-      ctx->bytes -= unit_bytes(s.unit_capacity);
+      charge(s, -(int64_t)unit_bytes(s.unit_capacity));
     }
     s.d_units = nullptr;
     s.d_overflow = nullptr;
@@ -359,7 +365,7 @@ int ensure_scratch(vgc_context *ctx, LaunchScratch &s, uint32_t views, size_t un
     CUDA_TRY(device_malloc(ctx, &s.d_units, unit_bytes(n)));
     s.d_overflow = reinterpret_cast<uint32_t *>(s.d_units + n);
     CUDA_TRY(cudaMemset(s.d_overflow, 0, overflow_bytes(n)));
-    ctx->bytes += unit_bytes(n);
+    charge(s, unit_bytes(n));
     s.unit_capacity = n;
   }
   if (!s.d_unit_count) CUDA_TRY(device_malloc(ctx, &s.d_unit_count, kLaunchCtlWords * 4));
@@ -372,12 +378,12 @@ int ensure_scratch(vgc_context *ctx, LaunchScratch &s, uint32_t views, size_t un
   if (want_chunks > s.chunk_capacity) {
     if (s.d_chunks) {
       cudaFree(s.d_chunks);
-      ctx->bytes -= (size_t)s.chunk_capacity * sizeof(uint4);
+      charge(s, -(int64_t)(s.chunk_capacity * sizeof(uint4)));
     }
     s.d_chunks = nullptr;
     s.chunk_capacity = 0;
     CUDA_TRY(device_malloc(ctx, &s.d_chunks, (size_t)want_chunks * sizeof(uint4)));
-    ctx->bytes += (size_t)want_chunks * sizeof(uint4);
+    charge(s, (size_t)want_chunks * sizeof(uint4));
     s.chunk_capacity = want_chunks;
   }
   if (!s.done) CUDA_TRY(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
@@ -407,6 +413,7 @@ void free_scratch(LaunchScratch &s) {
   if (s.fork) cudaEventDestroy(s.fork);
   if (s.join) cudaEventDestroy(s.join);
   if (s.side) cudaStreamDestroy(s.side);
+  if (s.account) *s.account -= s.charged;
   s = LaunchScratch();
 }
 
@@ -747,18 +754,17 @@ int prepare_multi(vgc_context *const *ctxs, uint32_t nctx, LaunchScratch &s, con
   if ((rc = after_last(s))) return rc;
   if ((rc = ensure_scratch(ctxs[0], s, count, units))) return rc;
   if (nctx > s.scene_capacity) {
-    vgc_context *owner = s.owner ? s.owner : ctxs[0];
     if (s.h_scenes) cudaFreeHost(s.h_scenes);
     if (s.d_scenes) {
       cudaFree(s.d_scenes);
-      owner->bytes -= sizeof(Scene) * s.scene_capacity;
+      charge(s, -(int64_t)(sizeof(Scene) * s.scene_capacity));
     }
     s.h_scenes = nullptr;
     s.d_scenes = nullptr;
     s.scene_capacity = 0;
     CUDA_TRY(cudaMallocHost(&s.h_scenes, sizeof(Scene) * nctx));
     CUDA_TRY(cudaMalloc(&s.d_scenes, sizeof(Scene) * nctx));
-    owner->bytes += sizeof(Scene) * nctx;
+    charge(s, sizeof(Scene) * nctx);
     s.scene_capacity = nctx;
   }
   for (uint32_t k = 0; k < nctx; k++) s.h_scenes[k] = scene_of(ctxs[k]);
@@ -1087,7 +1093,7 @@ int vgc_context_destroy(vgc_context *ctx) {
 
 int vgc_context_footprint(const vgc_context *ctx, uint64_t *bytes) {
   if (!ctx || !bytes) return fail(VGC_INVALID_ARG, "null argument");
-  *bytes = ctx->bytes;
+  *bytes = ctx->bytes + *ctx->scratch_bytes;
   return VGC_OK;
 }
 
@@ -1586,9 +1592,6 @@ int vgc_batch_destroy(vgc_batch *b) {
     if (f.graph) cudaGraphDestroy(f.graph);
   }
   if (b->capture_stream) cudaStreamDestroy(b->capture_stream);
-  if (b->scratch.d_views)
-    b->ctx->bytes -= sizeof(ViewConst) * b->scratch.view_capacity + hzb_plan_bytes(b->scratch.view_capacity);
-  if (b->scratch.d_units) b->ctx->bytes -= unit_bytes(b->scratch.unit_capacity);
   free_scratch(b->scratch);
   delete b;
   return VGC_OK;

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <array>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -63,7 +64,9 @@ using namespace vgch;
 
 // Launch scratch: view constants and the (view, cell) unit list of one launch sequence.
 struct LaunchScratch {
-  vgc_context *owner = nullptr;   // the context whose byte count holds this scratch's device buffers
+  vgc_context *owner = nullptr;   // the context the scratch's device buffers are counted against,
+  std::shared_ptr<uint64_t> account;  //   its scratch_bytes (a server's lanes may outlive the context), and how much
+  uint64_t charged = 0;               //   of that is this scratch's
   uint32_t hzb_w = 0, hzb_h = 0;  // largest depth image the views of this launch build an HZB from (0: none)
   bool hzb_tail = false;
   bool any_budget = false;        // a view of this launch searches its threshold for a triangleBudget
@@ -113,7 +116,8 @@ struct vgc_context {
   uint32_t select_grid = 0;  // persistent grid of k_instances
   uint32_t chunk_grid = 0;   // persistent grid of k_chunks
   uint32_t hzb_grid = 0;     // persistent grid of k_hzb_stream (0: the per-view tile kernel instead)
-  uint64_t bytes = 0;
+  uint64_t bytes = 0;  // device memory held, besides launch scratches
+  std::shared_ptr<uint64_t> scratch_bytes = std::make_shared<uint64_t>(0);
   std::mutex mu;
   // host mirrors of the resident scene
   std::vector<MeshHost> mesh_host;
