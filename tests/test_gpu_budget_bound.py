@@ -52,8 +52,9 @@ def test_budget_bounds_what_is_held():
     assert held[-1] > 100 << 20  # without a budget: the larger raster queue among it
     roomy, same = _session(1 << 40)
     assert same == want
-    # the needs: what a context with room holds at the end, without the 1 MB that selectCut keeps
-    needs = roomy[-1] - (1 << 20)
+    # the needs: what a context with room holds at the end, without the workspace that selectCut keeps
+    needs = roomy[-1] - (roomy[1] - roomy[0])
+    assert roomy[1] > roomy[0]
     assert needs < held[-1] - (100 << 20)
     for budget in (needs, needs + 1, needs + (1 << 20), needs + (40 << 20)):
         used, same = _session(budget)

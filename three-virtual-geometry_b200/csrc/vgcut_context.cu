@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -66,30 +67,48 @@ static bool over_budget(const vgc_context *ctx, size_t more) {
   return ctx->opts.hbm_budget_bytes && ctx->bytes + *ctx->scratch_bytes + more > ctx->opts.hbm_budget_bytes;
 }
 
-// The kept workspace: a device buffer for `bytes` at least (at most kSelectKeep), and the pinned pieces its results
-// come back through; false when the HBM budget or the device has no room for it. Given back when another allocation needs
-// the room (dev_alloc; a selectCut is synchronous, so nothing uses it then).
-// Pinned memory costs 1.2 ms for the first 2 MB and 0.4 ms for each further MB, which a context's first call pays: so
-// results pass through kSelectPieces small pieces instead of a buffer of their size.
+// The kept workspace: a device buffer for `bytes` at least (at most kSelectKeep), as cudaMalloc and cudaFree take most of a
+// call that allocates its own; false when the HBM budget or the device has no room for it. Given back when another
+// allocation needs the room (dev_alloc; a selectCut is synchronous, so nothing uses it then). The first has the call's
+// size, so that a context's first call, which may be its only one, pays for no more than it needs.
 constexpr size_t kSelectKeep = 32u << 20;
-constexpr size_t kSelectPiece = 256u << 10;
 static bool select_workspace(vgc_context *ctx, size_t bytes) {
-  cudaError_t e = cudaSuccess;
-  if (ctx->d_select.bytes < bytes) {
-    dev_free(ctx, ctx->d_select);
-    size_t want = size_t(1) << 20;
-    while (want < bytes) want *= 2;
-    if (over_budget(ctx, want)) return false;
-    e = cudaMalloc(&ctx->d_select.ptr, want);
-    if (e == cudaSuccess) ctx->d_select.bytes = want, ctx->bytes += want;
-    else ctx->d_select.ptr = nullptr;
+  if (ctx->d_select.bytes >= bytes) return true;
+  const size_t want = std::min(kSelectKeep, std::max(bytes, 2 * ctx->d_select.bytes));
+  dev_free(ctx, ctx->d_select);
+  if (over_budget(ctx, want)) return false;
+  if (cudaMalloc(&ctx->d_select.ptr, want) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->d_select.ptr = nullptr;
+    return false;
   }
-  if (e == cudaSuccess && !ctx->h_select) e = cudaMallocHost(&ctx->h_select, kSelectPieces * kSelectPiece);
+  ctx->d_select.bytes = want;
+  ctx->bytes += want;
+  return true;
+}
+
+// Page-locked pieces that a call's data comes and goes through; false when there are none. They save 8 to 15 us of a call
+// with up to 0.5 MB of results and nothing of one with more, and take 0.4 ms to set up (as ordinary memory registered; the
+// first page-locked memory of a process from the driver's allocator takes 0.8 to 2.6). So a context sets them up once it
+// has made kSelectMany calls without.
+constexpr size_t kSelectPiece = 256u << 10;
+constexpr uint32_t kSelectMany = 16;
+static bool select_pieces(vgc_context *ctx) {
+  if (ctx->h_select) return true;
+  if (++ctx->selects_without <= kSelectMany) return false;
+  ctx->selects_without = 0;  // should it fail, after as many more
+  void *p = std::aligned_alloc(4096, kSelectPieces * kSelectPiece);
+  cudaError_t e = p ? cudaHostRegister(p, kSelectPieces * kSelectPiece, cudaHostRegisterDefault) : cudaErrorMemoryAllocation;
+  const bool registered = e == cudaSuccess;
   for (uint32_t i = 0; i < kSelectPieces && e == cudaSuccess; i++)
     if (!ctx->select_piece[i]) e = cudaEventCreateWithFlags(&ctx->select_piece[i], cudaEventDisableTiming);
-  if (e == cudaSuccess) return true;
+  if (e == cudaSuccess) {
+    ctx->h_select = (unsigned char *)p;
+    return true;
+  }
   cudaGetLastError();
-  dev_free(ctx, ctx->d_select);
+  if (registered) cudaHostUnregister(p);
+  std::free(p);
   return false;
 }
 
@@ -1078,7 +1097,10 @@ int vgc_context_destroy(vgc_context *ctx) {
     dev_free(ctx, *b);
   for (auto &h : ctx->hzb) dev_free(ctx, h.data);
   if (ctx->h_stats) cudaFreeHost(ctx->h_stats);
-  if (ctx->h_select) cudaFreeHost(ctx->h_select);
+  if (ctx->h_select) {
+    cudaHostUnregister(ctx->h_select);
+    std::free(ctx->h_select);
+  }
   for (cudaEvent_t &ev : ctx->select_piece)
     if (ev) cudaEventDestroy(ev);
   for (auto &p : ctx->prof_pending) {
@@ -1689,37 +1711,31 @@ int vgc_select_cut(vgc_context *ctx, uint32_t slot, uint32_t count, const double
   int rc = sync_scene(ctx);
   if (rc) return rc;
   const uint32_t mcount = ctx->mesh_host[slot].meshlet_count;
-  std::vector<float> m((size_t)count * 16), p((size_t)count * 3);
-  for (size_t i = 0; i < m.size(); i++) m[i] = (float)vm16[i];
-  for (uint32_t i = 0; i < count; i++) {
-    p[i * 3] = (float)proj_scale[i];
-    p[i * 3 + 1] = (float)near_[i];
-    p[i * 3 + 2] = (float)scale[i];
+  const size_t mats = (size_t)count * 16;
+  std::vector<float> in(mats + (size_t)count * 3);  // the matrices, then the parameters
+  for (size_t i = 0; i < mats; i++) in[i] = (float)vm16[i];
+  for (size_t i = 0; i < count; i++) {
+    in[mats + i * 3] = (float)proj_scale[i];
+    in[mats + i * 3 + 1] = (float)near_[i];
+    in[mats + i * 3 + 2] = (float)scale[i];
   }
-  // Inputs, then lo, then hi in one device buffer; calls of ordinary size use the context's (kept, as cudaMalloc and
-  // cudaFree took most of such a call) and its pinned pieces.
-  const size_t outn = (size_t)count * mcount, in_bytes = ((m.size() + p.size()) * 4 + 255) & ~size_t(255);
-  const size_t total = in_bytes + outn * 2;
+  // inputs, then lo, then hi in one device buffer
+  const size_t outn = (size_t)count * mcount, in_bytes = (in.size() * 4 + 255) & ~size_t(255), total = in_bytes + outn * 2;
   const bool kept = total <= kSelectKeep && select_workspace(ctx, total);
+  const bool pieced = kept && select_pieces(ctx);
   void *d = ctx->d_select.ptr;
   if (!kept) CUDA_TRY(cudaMalloc(&d, total));
-  float *dm = (float *)d, *dp = dm + m.size();
+  const float *dm = (const float *)d;
   uint8_t *dlo = (uint8_t *)d + in_bytes, *dhi = dlo + outn;
   cudaStream_t st = ctx->stream;
-  cudaError_t e = cudaSuccess;
-  if (kept && in_bytes <= kSelectPieces * kSelectPiece) {
-    std::memcpy(ctx->h_select, m.data(), m.size() * 4);
-    std::memcpy(ctx->h_select + m.size() * 4, p.data(), p.size() * 4);
-    e = cudaMemcpyAsync(d, ctx->h_select, (m.size() + p.size()) * 4, cudaMemcpyHostToDevice, st);
-  } else {
-    e = cudaMemcpyAsync(dm, m.data(), m.size() * 4, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dp, p.data(), p.size() * 4, cudaMemcpyHostToDevice, st);
-  }
+  const void *src = in.data();
+  if (pieced && in.size() * 4 <= kSelectPieces * kSelectPiece) src = std::memcpy(ctx->h_select, in.data(), in.size() * 4);
+  cudaError_t e = cudaMemcpyAsync(d, src, in.size() * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess)
-    e = launch_select_cut(scene_of(ctx), slot, mcount, count, dm, dp, (float)threshold, (float)blend, dlo, dhi, st);
-  if (e == cudaSuccess && kept) e = select_results(ctx, dlo, outn, lo, hi, st);
-  if (e == cudaSuccess && !kept) e = cudaMemcpyAsync(lo, dlo, outn, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess && !kept) e = cudaMemcpyAsync(hi, dhi, outn, cudaMemcpyDeviceToHost, st);
+    e = launch_select_cut(scene_of(ctx), slot, mcount, count, dm, dm + mats, (float)threshold, (float)blend, dlo, dhi, st);
+  if (e == cudaSuccess && pieced) e = select_results(ctx, dlo, outn, lo, hi, st);
+  if (e == cudaSuccess && !pieced) e = cudaMemcpyAsync(lo, dlo, outn, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess && !pieced) e = cudaMemcpyAsync(hi, dhi, outn, cudaMemcpyDeviceToHost, st);
   const cudaError_t done = cudaStreamSynchronize(st);
   if (e == cudaSuccess) e = done;
   if (!kept) cudaFree(d);

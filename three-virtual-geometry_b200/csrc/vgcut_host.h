@@ -49,7 +49,7 @@ struct HzbSlot {
   bool valid = false;
 };
 
-constexpr uint32_t kSelectPieces = 4;   // pinned pieces a selectCut's results come back through
+constexpr uint32_t kSelectPieces = 4;   // page-locked pieces a selectCut's results come back through
 constexpr uint32_t kSplitLaunches = 64;  // after one that redid a cut, launch sequences with the retry rounds' own kernels
 constexpr uint32_t kQueueMin = 262144;  // entries of the smallest meshlet work queue of a context without an HBM budget
 
@@ -139,8 +139,9 @@ struct vgc_context {
   DevBuf d_meshes, d_levels, d_m_lod, d_m_parent, d_m_err, d_m_cull, d_m_info, d_m_tris, d_inst, d_inst_slot, d_cells;
   DevBuf d_lsamples, d_positions, d_m_verts;
   DevBuf d_raster;  // occluder depth pass: the tile pass's work lists
-  DevBuf d_select;  // selectCut workspace (kept while small), the pinned pieces of its results and their arrivals
+  DevBuf d_select;  // selectCut workspace (kept while small), the pieces its results come through and their arrivals
   unsigned char *h_select = nullptr;
+  uint32_t selects_without = 0;
   cudaEvent_t select_piece[kSelectPieces] = {};
   DevBuf d_resort;  // instance re-sort: centres, keys, permutation scratch (grows only)
   // output slots
