@@ -269,18 +269,27 @@ int ensure_outputs(vgc_context *ctx, uint32_t slots) {
   if ((rc = dev_alloc(ctx, ctx->d_args, (size_t)n * 2 * ctx->slot_capacity * 2 * 5 * 4))) return rc;
   if ((rc = dev_alloc(ctx, ctx->d_dyn, (size_t)n * 8 * 4))) return rc;
   if ((rc = dev_alloc(ctx, ctx->d_hist, (size_t)n * 2 * kBudgetBins * 8))) return rc;
-  if (n > ctx->out_slots) {
-    uint32_t *fresh = nullptr;
-    CUDA_TRY(cudaMallocHost(&fresh, (size_t)n * kStatWords * 4));
-    if (ctx->h_stats) cudaFreeHost(ctx->h_stats);
-    ctx->h_stats = fresh;
+  if (n > ctx->out_slots && ctx->h_stats) {
+    cudaFreeHost(ctx->h_stats);
+    ctx->h_stats = nullptr;
   }
-  std::memset(ctx->h_stats, 0, (size_t)n * kStatWords * 4);
+  if (ctx->h_stats) std::memset(ctx->h_stats, 0, (size_t)n * kStatWords * 4);
   CUDA_TRY(cudaMemset(ctx->d_counters.ptr, 0, (size_t)n * ctx->counter_words * 4));
   CUDA_TRY(cudaMemset(ctx->d_args.ptr, 0, (size_t)n * 2 * ctx->slot_capacity * 2 * 5 * 4));
   ctx->slot_stream.resize(n, nullptr);
+  ctx->slot_mirror.resize(n, kNoMirror);
+  if (!ctx->h_stats) std::fill(ctx->slot_mirror.begin(), ctx->slot_mirror.end(), kNoMirror);
   ctx->out_slots = n;
   ctx->out_slot_capacity = ctx->slot_capacity;
+  return VGC_OK;
+}
+
+// The counters' mirror, made for a context's first cut beside that cut's other page-locked memory: a context that only
+// builds HZBs or runs selectCuts does without (the first page-locked memory of a process takes 0.8 to 2.6 ms).
+static int ensure_mirror(vgc_context *ctx) {
+  if (ctx->h_stats) return VGC_OK;
+  CUDA_TRY(cudaMallocHost(&ctx->h_stats, (size_t)ctx->out_slots * kStatWords * 4));
+  std::memset(ctx->h_stats, 0, (size_t)ctx->out_slots * kStatWords * 4);
   return VGC_OK;
 }
 
@@ -294,19 +303,29 @@ static bool capturing(cudaStream_t st) {
 // Output slots [first, first + count) are cut on `st`.
 static void cut_on(vgc_context *ctx, uint32_t first, uint32_t count, cudaStream_t st) {
   if (capturing(st)) st = kReplayed;
-  for (uint32_t i = first; i < first + count; i++)
+  for (uint32_t i = first; i < first + count; i++) {
+    if (st == kReplayed && !ctx->h_stats) ctx->slot_mirror[i] = kNeverMirror;
+    if (ctx->slot_mirror[i] != kNeverMirror) ctx->slot_mirror[i] = ctx->h_stats ? kMirror : kNoMirror;
     if (ctx->slot_stream[i] != kReplayed) ctx->slot_stream[i] = st;
+  }
 }
 
-// Waits for slot `slot`'s cut before its mirrored counters are read; `st` has been waited for. A cut of another stream
-// than that and the context's own is waited for by a copy on the legacy stream, which follows every blocking stream's
-// work (11 us, which a reader that names the cut's stream does not pay).
-static cudaError_t wait_slot(vgc_context *ctx, uint32_t slot, cudaStream_t st) {
+// Slot `slot`'s counter header and threshold (kStatWords) for a reader that has waited for `st`: the mirror's, after a cut
+// of another stream than that and the context's own was waited for by a copy on the legacy stream, which follows every
+// blocking stream's work (11 us, which a reader that names the cut's stream does not pay); or the device's, where the
+// last cut had no mirror.
+static cudaError_t slot_words(vgc_context *ctx, uint32_t slot, cudaStream_t st, uint32_t *words) {
   const cudaStream_t cut = ctx->slot_stream[slot];
-  if (cut != kReplayed && (cut == st || cut == ctx->stream)) return cudaSuccess;
-  uint32_t word;
-  return cudaMemcpy(&word, (const uint32_t *)ctx->d_counters.ptr + (size_t)slot * ctx->counter_words, 4,
-                    cudaMemcpyDeviceToHost);
+  const bool mirror = ctx->slot_mirror[slot] == kMirror;
+  if (!mirror || cut == kReplayed || (cut != st && cut != ctx->stream)) {
+    const cudaError_t e = cudaMemcpy(words, (const uint32_t *)ctx->d_counters.ptr + (size_t)slot * ctx->counter_words,
+                                     VGC_COUNTER_HEADER * 4, cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return e;
+  }
+  if (!mirror)
+    return cudaMemcpy(words + VGC_COUNTER_HEADER, (const float *)ctx->d_dyn.ptr + (size_t)slot * 8, 4, cudaMemcpyDeviceToHost);
+  std::memcpy(words, ctx->h_stats + (size_t)slot * kStatWords, kStatWords * 4);
+  return cudaSuccess;
 }
 
 size_t output_slot_bytes(const vgc_context *ctx) {
@@ -662,7 +681,7 @@ int view_constants(vgc_context *ctx, const vgc_view &in, uint32_t out_slot, uint
   k.draw_list = (uint4 *)ctx->d_draw.ptr + (size_t)out_slot * 2 * ctx->opts.max_meshlets;
   k.draw_args = (uint32_t *)ctx->d_args.ptr + (size_t)out_slot * 2 * ctx->slot_capacity * 2 * 5;
   k.dyn = (float *)ctx->d_dyn.ptr + (size_t)out_slot * 8;
-  k.host_stats = ctx->h_stats + (size_t)out_slot * kStatWords;
+  k.host_stats = ctx->h_stats ? ctx->h_stats + (size_t)out_slot * kStatWords : nullptr;  // null: vgc_cut_noalloc alone
   k.hist = (unsigned long long *)ctx->d_hist.ptr + (size_t)out_slot * 2 * kBudgetBins;
   return VGC_OK;
 }
@@ -693,7 +712,7 @@ int prepare(vgc_context *ctx, LaunchScratch &s, const vgc_view *views, uint32_t 
     slot_end = 0;
     for (uint32_t i = 0; i < count; i++) slot_end = std::max(slot_end, slots[i] + 1);
   }
-  if ((rc = ensure_outputs(ctx, slot_end))) return rc;
+  if ((rc = ensure_outputs(ctx, slot_end)) || (rc = ensure_mirror(ctx))) return rc;
   if ((rc = after_last(s))) return rc;
   const uint32_t cells = pad32((uint32_t)ctx->cells.size());
   if ((rc = ensure_scratch(ctx, s, count, (size_t)count * cells))) return rc;
@@ -767,7 +786,7 @@ int prepare_multi(vgc_context *const *ctxs, uint32_t nctx, LaunchScratch &s, con
   size_t units = 0;
   for (uint32_t k = 0; k < nctx; k++) {
     if ((rc = sync_scene(ctxs[k]))) return rc;
-    if (slot_end[k] && (rc = ensure_outputs(ctxs[k], slot_end[k]))) return rc;
+    if (slot_end[k] && ((rc = ensure_outputs(ctxs[k], slot_end[k])) || (rc = ensure_mirror(ctxs[k])))) return rc;
   }
   for (uint32_t i = 0; i < count; i++) units += pad32((uint32_t)ctxs[scene[i]]->cells.size());
   if ((rc = after_last(s))) return rc;
@@ -1639,8 +1658,8 @@ int vgc_read_stats(vgc_context *ctx, uint32_t slot, vgc_stats *s, vgc_stream str
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   CUDA_TRY(cudaStreamSynchronize(st));
   if (st != ctx->stream) CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  CUDA_TRY(wait_slot(ctx, slot, st));
-  const uint32_t *c = ctx->h_stats + (size_t)slot * kStatWords;  // mirrored by the cut's last kernel
+  uint32_t c[kStatWords];
+  CUDA_TRY(slot_words(ctx, slot, st, c));
   float dyn;
   std::memcpy(&dyn, c + VGC_COUNTER_HEADER, 4);
   decode_stats(ctx, c, dyn, s);
@@ -1653,9 +1672,9 @@ int vgc_read_draw_list(vgc_context *ctx, uint32_t slot, uint32_t cut, uint32_t *
   if (slot >= ctx->out_slots) return fail(VGC_NOT_FOUND, "output slot not allocated");
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   CUDA_TRY(cudaStreamSynchronize(st));
-  CUDA_TRY(wait_slot(ctx, slot, st));
-  const uint32_t sel = ctx->h_stats[(size_t)slot * kStatWords + VGC_COUNTER_CUT0 + cut * 5 + VGC_CUT_SELECTED];
-  const uint32_t n = std::min(sel, ctx->opts.max_meshlets);
+  uint32_t c[kStatWords];
+  CUDA_TRY(slot_words(ctx, slot, st, c));
+  const uint32_t n = std::min(c[VGC_COUNTER_CUT0 + cut * 5 + VGC_CUT_SELECTED], ctx->opts.max_meshlets);
   *count = n;
   const uint32_t copy = std::min(n, capacity);
   if (copy) {

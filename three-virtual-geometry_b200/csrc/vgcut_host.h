@@ -53,6 +53,9 @@ constexpr uint32_t kSelectPieces = 4;   // page-locked pieces a selectCut's resu
 constexpr uint32_t kSplitLaunches = 64;  // after one that redid a cut, launch sequences with the retry rounds' own kernels
 constexpr uint32_t kQueueMin = 262144;  // entries of the smallest meshlet work queue of a context without an HBM budget
 
+// slot_mirror: in the mirror; on the device, as the slot's last cut had none (or there was none); always there, as a graph
+// holds a cut of the slot that has none
+enum : uint8_t { kMirror, kNoMirror, kNeverMirror };
 // slot_stream of a slot whose cut a stream captured: it runs wherever its graph is replayed, which no call here sees
 inline const cudaStream_t kReplayed = cudaStreamLegacy;
 
@@ -149,7 +152,8 @@ struct vgc_context {
   uint32_t out_slot_capacity = 0;  // slot_capacity the output buffers were sized for
   uint32_t counter_words = 0;
   DevBuf d_counters, d_draw, d_args, d_dyn, d_hist;
-  uint32_t *h_stats = nullptr;  // pinned: kStatWords per output slot, written by the slot's last k_finish
+  uint32_t *h_stats = nullptr;  // pinned: kStatWords per output slot, written by the slot's last k_finish (null: no cut yet)
+  std::vector<uint8_t> slot_mirror;       // per output slot: where its counters are read (kMirror, ...)
   std::vector<cudaStream_t> slot_stream;  // per output slot: the stream of its last cut (null: none; kReplayed)
   // controller state slots
   DevBuf d_state;

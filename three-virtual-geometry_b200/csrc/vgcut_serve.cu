@@ -180,6 +180,8 @@ int launch_batch(vgc_server *s, Lane &lane, const std::vector<uint32_t> &slots, 
     vgc_context *owner = s->scenes[scene_ids[i]].ctx;
     cudaStream_t &cut = owner->slot_stream[slots[i]];
     if (cut != kReplayed) cut = owner->stream;
+    uint8_t &mirror = owner->slot_mirror[slots[i]];
+    if (mirror != kNeverMirror) mirror = kMirror;
   }
   CUDA_TRY(cudaEventRecord(lane.start, lane.stream));
   if ((rc = enqueue(ctx, lane.scratch, n, lane.stream, false))) return rc;
