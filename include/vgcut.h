@@ -335,8 +335,9 @@ int vgc_server_destroy(vgc_server *server);
    sampled at pixel centres. A triangle crossing the near plane (clip z = 0) is clipped in clip space into one or two
    triangles (crossing points interpolated from the corner in front, at depth 0), as a GPU's clipper does; wholly
    behind it, it is not drawn. Pass `depth` as this frame's vgc_view.depth to build the HZB from it in the cut's own
-   launch sequence. The first call allocates the context's triangle queues (56 MB, or 182 MB without an HBM
-   budget and where the device has the room; shared with vgc_visibility; up to 131,072 near-plane-crossing triangles a call are clipped, more are left out); calls on one
+   launch sequence. The first call allocates the context's triangle queues (57 MB; 183 MB for images of more than
+   524,288 pixels in all, which also add 168 MB to a smaller call's queues, without an HBM budget and where the device has
+   the room; shared with vgc_visibility; up to 131,072 near-plane-crossing triangles a call are clipped, more are left out); calls on one
    context whose GPU work overlaps (different streams) race on them: order them on one stream. Asynchronous on
    `stream`. */
 int vgc_occluder_depth(vgc_context *ctx, uint32_t src_slot, const vgc_view *view, float *depth, uint32_t width,

@@ -34,8 +34,8 @@ def _session(budget):
         vm[:, 14] = -5.0
         for _ in range(3):
             step(*(a.tobytes() for a in vg.select_cut(mesh.slot, vm, 900.0, 0.1, np.ones(9), 1.0, 2.0)))
-        depth = torch.empty((64, 64), dtype=torch.float32, device="cuda")
-        vg.occluder_depth(0, cam, depth.data_ptr(), 64, 64)
+        depth = torch.empty((1024, 1024), dtype=torch.float32, device="cuda")
+        vg.occluder_depth(0, cam, depth.data_ptr(), 1024, 1024)
         torch.cuda.synchronize()
         step(depth.cpu().numpy().tobytes())
         vg.create_mesh(scenes.icosphere_mesh(24, seed=2), grid_matrices(5000, 2.0, 6))

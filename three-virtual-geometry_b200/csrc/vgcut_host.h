@@ -142,6 +142,7 @@ struct vgc_context {
   DevBuf d_meshes, d_levels, d_m_lod, d_m_parent, d_m_err, d_m_cull, d_m_info, d_m_tris, d_inst, d_inst_slot, d_cells;
   DevBuf d_lsamples, d_positions, d_m_verts;
   DevBuf d_raster;  // occluder depth pass: the tile pass's work lists
+  DevBuf d_raster_medium;  // ... and the larger medium queue, when d_raster was made for small images
   DevBuf d_select;  // selectCut workspace (kept while small), the pieces its results come through and their arrivals
   unsigned char *h_select = nullptr;
   uint32_t selects_without = 0;

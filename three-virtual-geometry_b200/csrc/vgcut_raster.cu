@@ -43,11 +43,12 @@ namespace {
 constexpr uint32_t kLaneRasterMax = 32;
 constexpr uint32_t kWarpRasterMax = 1024;   // ... by one warp of the second kernel; beyond, as tiles
 constexpr uint32_t kTileW = 32, kTileH = 16;
-// Queue capacities: medium triangles in sub-queues (record i of sub-queue q at i * kSubQueues + q), 160 MB of them, a
-// quarter of that in a context with an HBM budget and where the device has no room for more. What the queue does not hold is drawn by the warp that set it
+// Queue capacities: medium triangles in sub-queues (record i of sub-queue q at i * kSubQueues + q), 160 MB of them; a
+// quarter of that for images of up to kManyPixels in all (as many records a pixel as a 1080p image then has), in a context
+// with an HBM budget and where the device has no room for more. What the queue does not hold is drawn by the warp that set it
 // up, long after the others have finished: 1080p visibility buffers of near geometry 2.40 -> 1.30 ms, 32 two-pass images
 // of 960x540 2.06 -> 1.45 ms a step, against a quarter of the records.
-constexpr uint32_t kQueuedMedium = 5u << 19, kQueuedMediumMin = 5u << 17;
+constexpr uint32_t kQueuedMedium = 5u << 19, kQueuedMediumMin = 5u << 17, kManyPixels = 1u << 19;
 constexpr uint32_t kSubQueues = 256;
 constexpr uint32_t kClipCtl = 4 + kSubQueues;   // occluder pass: triangles crossing the near plane, queued
 constexpr uint32_t kCtlWords = kClipCtl + 1;
@@ -879,25 +880,34 @@ __global__ void __launch_bounds__(128, 7) k_visibility(const __grid_constant__ S
 
 }  // namespace
 
-// The queues of the second kernel (allocated once per context; the passes of one context share them, so calls on
-// different streams must not overlap).
-static int raster_queues(vgc_context *ctx, RasterArgs &R) {
+// The queues of the second kernel for images of `pixels` in all (the passes of one context share them, so calls on
+// different streams must not overlap). What a call has used is kept until the context ends, since a captured graph may
+// hold it: a first call of larger images takes everything at once, one of smaller images the smaller medium queue, to
+// which a larger one is added when larger images come.
+static int raster_queues(vgc_context *ctx, RasterArgs &R, size_t pixels, cudaStream_t st) {
   const size_t large_bytes = (size_t)kQueuedLarge * kRecord * 16, tile_bytes = (size_t)kTileUnits * 8;
   const size_t ctl_bytes = 2048, clip_bytes = (size_t)kClipQueue * 8;
   static_assert(kCtlWords * 4 <= ctl_bytes, "control words");
   const size_t rest = ctl_bytes + large_bytes + tile_bytes + clip_bytes, record = kRecord * 16;
+  const bool many = pixels > kManyPixels && !ctx->opts.hbm_budget_bytes;
   if (!ctx->d_raster.ptr) {
-    int rc = ctx->opts.hbm_budget_bytes ? VGC_OVER_BUDGET : dev_alloc(ctx, ctx->d_raster, rest + kQueuedMedium * record);
-    if (rc == VGC_OVER_BUDGET || rc == VGC_OOM) rc = dev_alloc(ctx, ctx->d_raster, rest + kQueuedMediumMin * record);
+    int rc = many ? dev_alloc(ctx, ctx->d_raster, rest + kQueuedMedium * record) : VGC_OOM;
+    if (rc == VGC_OOM) rc = dev_alloc(ctx, ctx->d_raster, rest + kQueuedMediumMin * record);
     if (rc) return rc;
+  } else if (many && ctx->d_raster.bytes < rest + kQueuedMedium * record && !ctx->d_raster_medium.ptr) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;  // a capture allows no allocation
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
+        dev_alloc(ctx, ctx->d_raster_medium, kQueuedMedium * record))
+      cudaGetLastError();
   }
   char *q = (char *)ctx->d_raster.ptr;
   R.ctl = (uint32_t *)q;
   R.large = (float4 *)(q + ctl_bytes);
   R.tiles = (uint2 *)(q + ctl_bytes + large_bytes);
   R.clip = (uint2 *)(q + ctl_bytes + large_bytes + tile_bytes);
-  R.medium = (float4 *)(q + rest);
-  R.medium_each = (uint32_t)((ctx->d_raster.bytes - rest) / record) / kSubQueues;
+  const bool added = many && ctx->d_raster_medium.ptr;
+  R.medium = (float4 *)(added ? (char *)ctx->d_raster_medium.ptr : q + rest);
+  R.medium_each = (uint32_t)((added ? ctx->d_raster_medium.bytes : ctx->d_raster.bytes - rest) / record) / kSubQueues;
   return VGC_OK;
 }
 
@@ -924,8 +934,8 @@ static int occluder_depth_images(vgc_context *ctx, uint32_t count, const uint32_
   }
   R.width = width;
   R.height = height;
-  if ((rc = raster_queues(ctx, R))) return rc;
   const size_t pixels = (size_t)width * height;
+  if ((rc = raster_queues(ctx, R, pixels * count, st))) return rc;
   k_occluder_clear<<<(unsigned)std::min<size_t>((pixels * count + 255) / 256, (size_t)ctx->sm_count * 16), 256, 0,
                      st>>>(R, count, pixels);
   CUDA_TRY(cudaGetLastError());
@@ -1022,8 +1032,8 @@ extern "C" int vgc_visibility(vgc_context *ctx, uint32_t slot, uint32_t cut, con
   R.height = height;
   R.vis = reinterpret_cast<unsigned long long *>(vis);
   R.frame = frame;
-  if ((rc = raster_queues(ctx, R))) return rc;
   const size_t pixels = (size_t)width * height;
+  if ((rc = raster_queues(ctx, R, pixels, st))) return rc;
   k_target_clear<unsigned long long>
       <<<(unsigned)std::min<size_t>((pixels + 255) / 256, (size_t)ctx->sm_count * 16), 256, 0, st>>>(
           R.vis, pixels, (unsigned long long)VGC_VIS_EMPTY, R.ctl);
