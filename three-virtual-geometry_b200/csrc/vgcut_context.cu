@@ -516,8 +516,6 @@ HzbDesc hzb_layout(uint32_t width, uint32_t height, size_t *total_floats) {
   return desc;
 }
 
-// Allocates / lays out HZB slot `hzb` for a width x height mip 0 and publishes its descriptor; returns whether the
-// device descriptor array changed (the caller uploads it).
 // cuTensorMapEncodeTiled of the driver, found once through the runtime (the library does not link libcuda).
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
@@ -586,6 +584,8 @@ void build_hzb_plan(vgc_context *ctx, LaunchScratch &s, const vgc_view *views, u
   P.maps = (uint32_t)maps;
 }
 
+// Allocates / lays out HZB slot `hzb` for a width x height mip 0 and publishes its descriptor; *changed: the device's
+// descriptor array differs (the caller uploads it).
 int hzb_prepare(vgc_context *ctx, int32_t hzb, uint32_t width, uint32_t height, bool *changed) {
   if (width == 0 || height == 0 || width > 32768 || height > 32768) return fail(VGC_INVALID_ARG, "HZB size out of range");
   size_t total = 0;
@@ -771,8 +771,6 @@ cudaError_t timed(vgc_context *ctx, bool capture, int kind, cudaStream_t st, F &
   return e;
 }
 
-// The launch sequence of one frame: reset, cells, then select + finish for the first round, and the two retry rounds
-// (GeometryPool.ts:1081-1092 without the dispatch-argument kernels, which persistent launches do not need).
 int prepare_multi(vgc_context *const *ctxs, uint32_t nctx, LaunchScratch &s, const vgc_view *views,
                   const uint32_t *scene, uint32_t count, const uint32_t *slots) {
   if (!ctxs || nctx == 0 || !views || !scene || !slots || count == 0) return fail(VGC_INVALID_ARG, "no views");
@@ -823,6 +821,8 @@ int prepare_multi(vgc_context *const *ctxs, uint32_t nctx, LaunchScratch &s, con
   return VGC_OK;
 }
 
+// The launch sequence of one frame: reset, cells, then select + finish for the first round, and the two retry rounds
+// (GeometryPool.ts:1081-1092 without the dispatch-argument kernels, which persistent launches do not need).
 int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st, bool capture) {
   const Scene S = scene_of(ctx);
   const Scene *scenes = s.multi ? s.d_scenes : nullptr;
@@ -888,8 +888,8 @@ int enqueue(vgc_context *ctx, LaunchScratch &s, uint32_t count, cudaStream_t st,
   }
   // The retry rounds are one kernel that returns at once when no cut overflowed (k_retry, which has the figures), until a
   // sequence of this scratch redoes one: then, for kSplitLaunches sequences after the last that did, they are kernels of
-  // their own, with all of the chip's warps in each. 320 views of which an eighth
-  // overflow: 4.00 ms, 4.71 with the one kernel throughout.
+  // their own, with all of the chip's warps in each. 320 views of which an eighth overflow: 4.00 ms, 4.71 with the one
+  // kernel throughout.
   const bool split = s.split_left != 0;
   for (int round = 0; round < (split ? 3 : 1); round++) {
     if (round > 0 && kChunkShiftRetry) lim.chunk_max = kChunkShiftRetry, lim.chunk_min = std::min(lim.chunk_min, kChunkShiftRetry);

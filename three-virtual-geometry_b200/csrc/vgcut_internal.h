@@ -115,8 +115,8 @@ struct alignas(16) HzbDesc {
 static_assert(offsetof(HzbDesc, size) == 12, "HzbDesc::head reads the first 16 bytes");
 
 // The HZB builds of one launch sequence as one stream of 128 x 32 mip-0 strips (k_hzb_stream): a header, one job per
-// view that brings a depth image, then one tensor map per job. Written on the host into pinned memory and copied
-// with the view constants.
+// view that brings a depth image, then one tensor map per job. Written on the host into pinned memory, which
+// k_reset reads with the view constants.
 struct HzbPlanHead {
   uint32_t jobs, tiles;  // jobs; strips of all jobs
   uint32_t maps;         // byte offset of the tensor maps (kTensorMapBytes each, in job order)

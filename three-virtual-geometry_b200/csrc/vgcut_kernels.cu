@@ -302,8 +302,9 @@ __global__ void __launch_bounds__(256) k_cells(Scene S0, const Scene *scenes, co
 // ------------------------------------------------------------------------------------------------ k_instances
 constexpr int kWarpStage = 96;   // staged draw entries per warp (a step adds <= 32; one cut at a time)
 // The meshlet work queue between k_instances and k_chunks, in one buffer of `capacity` uint4: spans (one item's
-// meshlets inside one window of 2^chunk_shift meshlets of its warp's items laid end to end; 512 unless the batch's
-// autotuner picked 256 or 1024) and chunks (the <= 32 spans of one window: one (view, cell, cut)). ctl[4..5] is the 64-bit reservation counter: spans low, chunks high.
+// meshlets inside one window of 2^chunk_shift meshlets of its warp's items laid end to end: 32 to 512 by the visible units,
+// or what the batch was tuned to, pass_shape) and chunks (the <= 32 spans of one window: one (view, cell, cut)). ctl[4..5]
+// is the 64-bit reservation counter: spans low, chunks high.
 struct WorkQueue {
   uint4 *spans, *chunks;
   uint32_t span_cap, chunk_cap;
@@ -1769,8 +1770,8 @@ __global__ void __launch_bounds__(kHzbTileThreads) k_hzb_tiles_views(const ViewC
 
 // Levels `first` and up of one HZB by one block (the tile or strip kernel wrote the level below). The kernel is a chain
 // of short dependent steps, and a level read back from memory puts an L2 round trip into each: so a level of up to
-// 4,096 texels is also kept in shared memory for the next one (all of a 4K image's from level 5; the larger levels of
-// wider images go through memory). Launched behind the tile kernel's last blocks it adds 2 us to a build, which it
+// 4,096 texels is also kept in shared memory for the next one (a 4K image's from level 6; larger ones, such as its 120 x 68
+// of level 5, go through memory). Launched behind the tile kernel's last blocks it adds 2 us to a build, which it
 // added 5.5 us to.
 constexpr uint32_t kTailTexels = 4096;
 struct TailSmem {
@@ -1905,8 +1906,8 @@ __global__ void k_wait_probe(uint64_t limit_ns, unsigned long long *out) {
   }
 }
 
-// The tensor map was written to global memory by a copy before this launch: order that write before its use by
-// the tensor-map proxy.
+// The tensor map was written to global memory by k_reset, with the other proxy: order that write before its use by the
+// tensor-map proxy.
 __device__ __forceinline__ void tensormap_acquire(const void *map) {
   asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
 }

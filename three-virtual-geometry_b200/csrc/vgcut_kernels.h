@@ -20,7 +20,10 @@ struct LaunchInputs {
   const uint32_t *scenes_src = nullptr;
   uint32_t *scenes_dst = nullptr;
 };
-// ctl: per-batch control words: [0] visible units, [1..2] a view redoes a cut in round 1..2, [3] chunks queued
+// ctl: the sequence's control words (kLaunchCtlWords, cleared here): [0] visible units, [1..2] a view redoes a cut in round
+// 1..2, [4..5] the work queue's 64-bit counter (spans low, chunks high), [6..7] the most spans / chunks any pass asked for,
+// [8] the next chunk, [9] the next instance unit, [10] a unit's items did not fit the queue, [11] the next overflow word,
+// [12] a wait of k_retry gave up, [16] k_retry's phase and from [17] the phases' counters of its two rounds
 cudaError_t launch_reset(const LaunchInputs &in, ViewConst *views, uint32_t nviews, uint32_t *ctl, cudaStream_t st,
                          bool plain = false);
 // plain: launched without programmatic serialization (launch_after).

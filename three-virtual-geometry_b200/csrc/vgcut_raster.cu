@@ -655,7 +655,6 @@ struct VisArgs {
   uint32_t meshlets, instances, meshlet_vertices, vertices;
 };
 
-// Screen-space vertex of index `idx` (w = 0: unusable), and its entry's draw slot and blend range.
 // The clip-space position of index `idx` of the expanded buffer (ok: the index and its data are in range).
 __device__ __forceinline__ float4 pulled_clip(const Scene &S, const VisArgs &A, uint32_t idx, bool &ok) {
   const uint32_t ds = idx >> kLocalVertexBits, lv = idx & ((1u << kLocalVertexBits) - 1u);
