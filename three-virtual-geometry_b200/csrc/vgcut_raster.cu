@@ -755,7 +755,8 @@ __device__ __noinline__ int pulled_triangle(const Scene &S, const VisArgs &A, ui
 // from there: about 70 pulls for the 80 triangles of a meshlet, where a pull per index took 240. Bound by instruction
 // issue (pulls 35%, pixels 20%, the rest indices and set-up); the ring's draw stands at one place of the loop, so that its
 // registers and the set-up's share the 72 that let 28 warps live on an SM (80 and 64 measured 760 and 735 us, the
-// indices of the next step fetched ahead 765). 1080p, 290k meshlets of 24M triangles: 1433 -> 737 us.
+// indices of the next step fetched ahead 765). 1080p, 290k meshlets of 24M triangles: 1433 -> 737 us, with a quarter of the
+// medium queue; with all of it another such view takes 540, and the queue kernel 147.
 constexpr uint32_t kVisRunMin = 64, kVisRunMax = 512;
 __global__ void __launch_bounds__(128, 7) k_visibility(const __grid_constant__ Scene S,
                                                        const __grid_constant__ VisArgs A,
