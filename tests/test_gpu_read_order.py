@@ -78,3 +78,39 @@ def test_slot_that_was_never_cut():
     assert vg.read_stats(1)["selected"] == [0, 0] and len(vg.draw_list(1, 0)) == 0
     assert np.array_equal(vg.draw_list(0, 1), np.zeros((0, 4), np.uint32))
     vg.dispose()
+
+
+@pytest.mark.parametrize("first", ["stats", "list"])
+def test_cut_on_the_contexts_stream_with_another_one_named(first):
+    import torch
+    n = 48
+    vg = engine.VirtualGeometry(max_meshlets=1 << 16, output_slots=n)
+    vg.create_mesh(scenes.icosphere_mesh(24, seed=2), grid_matrices(4000, 2.0, 5))
+    cam = Camera.perspective_look_at((-6.0, 5.0, -6.0), (60.0, 0.0, 60.0), 60, 1920, 1080, 0.1, 5000.0)
+
+    def views(threshold):
+        return [engine.make_view(cam, engine.ViewParams(error_threshold=threshold, fresh_state=True, state_slot=k))
+                for k in range(n)]
+
+    other = torch.cuda.Stream()
+
+    def read(slot):
+        s, count = engine.Stats(), C.c_uint32()
+        calls = [lambda: engine.check(engine.lib().vgc_read_stats(vg.handle, slot, C.byref(s), other.cuda_stream)),
+                 lambda: engine.check(engine.lib().vgc_read_draw_list(vg.handle, slot, 0, None, 0, C.byref(count),
+                                                                      other.cuda_stream))]
+        for call in calls if first == "stats" else calls[::-1]:
+            call()
+        return s.selected[0], count.value
+
+    want = []
+    for t in (8.0, 0.5):
+        vg.cut(views(t))
+        torch.cuda.synchronize()
+        want.append(read(n - 1))
+    assert want[0][0] == want[0][1] != want[1][0] == want[1][1]
+    for _ in range(5):
+        for k, t in enumerate((8.0, 0.5)):
+            vg.cut(views(t))  # 48 views: the read comes long before they are cut
+            assert read(n - 1) == want[k]
+    vg.dispose()

@@ -310,16 +310,19 @@ static void cut_on(vgc_context *ctx, uint32_t first, uint32_t count, cudaStream_
   }
 }
 
-// Slot `slot`'s counter header and threshold (kStatWords) for a reader that has waited for `st`: the mirror's, after a cut
-// of another stream than that and the context's own was waited for by a copy on the legacy stream, which follows every
+// Slot `slot`'s counter header and threshold (kStatWords) for a reader that names `st`: waits for that and the context's own
+// stream. Then the mirror's, after a cut of another stream was waited for by a copy on the legacy stream, which follows every
 // blocking stream's work (11 us, which a reader that names the cut's stream does not pay); or the device's, where the
 // last cut had no mirror.
 static cudaError_t slot_words(vgc_context *ctx, uint32_t slot, cudaStream_t st, uint32_t *words) {
+  cudaError_t e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && st != ctx->stream) e = cudaStreamSynchronize(ctx->stream);
+  if (e != cudaSuccess) return e;
   const cudaStream_t cut = ctx->slot_stream[slot];
   const bool mirror = ctx->slot_mirror[slot] == kMirror;
   if (!mirror || cut == kReplayed || (cut != st && cut != ctx->stream)) {
-    const cudaError_t e = cudaMemcpy(words, (const uint32_t *)ctx->d_counters.ptr + (size_t)slot * ctx->counter_words,
-                                     VGC_COUNTER_HEADER * 4, cudaMemcpyDeviceToHost);
+    e = cudaMemcpy(words, (const uint32_t *)ctx->d_counters.ptr + (size_t)slot * ctx->counter_words, VGC_COUNTER_HEADER * 4,
+                   cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return e;
   }
   if (!mirror)
@@ -1655,11 +1658,8 @@ int vgc_get_output(const vgc_context *ctx, uint32_t slot, vgc_output *out) {
 int vgc_read_stats(vgc_context *ctx, uint32_t slot, vgc_stats *s, vgc_stream stream) {
   if (!ctx || !s) return fail(VGC_INVALID_ARG, "null argument");
   if (slot >= ctx->out_slots) return fail(VGC_NOT_FOUND, "output slot not allocated");
-  cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-  CUDA_TRY(cudaStreamSynchronize(st));
-  if (st != ctx->stream) CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   uint32_t c[kStatWords];
-  CUDA_TRY(slot_words(ctx, slot, st, c));
+  CUDA_TRY(slot_words(ctx, slot, stream ? (cudaStream_t)stream : ctx->stream, c));
   float dyn;
   std::memcpy(&dyn, c + VGC_COUNTER_HEADER, 4);
   decode_stats(ctx, c, dyn, s);
@@ -1670,10 +1670,8 @@ int vgc_read_draw_list(vgc_context *ctx, uint32_t slot, uint32_t cut, uint32_t *
                        uint32_t *count, vgc_stream stream) {
   if (!ctx || !count || cut > 1 || (capacity && !entries)) return fail(VGC_INVALID_ARG, "bad arguments");
   if (slot >= ctx->out_slots) return fail(VGC_NOT_FOUND, "output slot not allocated");
-  cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-  CUDA_TRY(cudaStreamSynchronize(st));
   uint32_t c[kStatWords];
-  CUDA_TRY(slot_words(ctx, slot, st, c));
+  CUDA_TRY(slot_words(ctx, slot, stream ? (cudaStream_t)stream : ctx->stream, c));
   const uint32_t n = std::min(c[VGC_COUNTER_CUT0 + cut * 5 + VGC_CUT_SELECTED], ctx->opts.max_meshlets);
   *count = n;
   const uint32_t copy = std::min(n, capacity);
